@@ -1,0 +1,94 @@
+// Device helpers of the kernels that stream rows through a ring of shared-memory stages filled by
+// asynchronous bulk copies (the wave plan, gn_wave.cu, and the resident plan, gn_resident.cu).
+#pragma once
+#include "gn_common.cuh"
+#include "gn_math.cuh"
+
+namespace gnb200 {
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+// A consumer warp hands a stage back to the producer only after it has USED the vectors it read from
+// the stage.  The shared-memory loads are merely issued when the warp moves on; signalling the stage
+// as free right after them let the producer's next TMA copy into the stage (fast when the rows come from
+// L2) now and then overtake a load that was still queued, and a warp computed one stage's rows from
+// pieces of a later stage.  So the arrival follows the arithmetic in program order - instructions
+// issue in order and the arithmetic cannot issue before its operands have arrived - and pin_regs keeps
+// the compiler from moving that arithmetic behind the arrival (the output stores of pass B are
+// volatile asm statements and stay in front of it by themselves).
+template <int N>
+__device__ __forceinline__ void pin_regs(float (&a)[N]) {
+#pragma unroll
+  for (int e = 0; e < N; ++e) asm volatile("" : "+f"(a[e]));
+}
+__device__ __forceinline__ void release_stage(uint64_t* empty_bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(empty_bar);
+}
+__device__ __forceinline__ float warp_sum_all(float v) {
+#pragma unroll
+  for (int b = 16; b >= 1; b >>= 1) v += __shfl_xor_sync(0xffffffffu, v, b);
+  return v;
+}
+// streaming 16-byte store: the line is marked evict-first, so results do not push the rows that
+// pass B still has to read out of L2
+__device__ __forceinline__ void stg128_stream(void* p, const uint4 v) {
+  asm volatile("st.global.cs.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
+  unsigned int v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+#define kNaN __int_as_float(0x7fc00000)
+
+// mbarrier waits of the streaming kernels.  `gave_up` is the CTA's shared flag: the first wait that runs
+// out sets it (and poisons the results, see the callers); from then on no wait of this CTA spends
+// its limit again, so a broken run ends after about one limit instead of one limit per stage.
+// producer (a single thread):
+__device__ __forceinline__ void producer_wait(uint64_t* bar, unsigned parity, volatile int* gave_up, const WaitLimit& lim) {
+  if (mbar_try_wait(bar, parity)) return;
+  if (*gave_up != 0) return;
+  if (!mbar_wait_bounded(bar, parity, lim)) *gave_up = 1;
+}
+// consumers (whole warps): if the phase is not complete yet, lane 0 alone polls - 256 polling threads
+// would take issue slots from the CTAs that share the SM - and afterwards every lane observes the
+// completed phase with one more try_wait of its own, which is what makes the TMA's writes visible
+// to it.
+__device__ __forceinline__ void consumer_wait(uint64_t* bar, unsigned parity, volatile int* gave_up, const WaitLimit& lim) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return;
+  if ((threadIdx.x & 31) == 0 && *gave_up == 0) {
+    if (!mbar_wait_bounded(bar, parity, lim)) *gave_up = 1;
+  }
+  __syncwarp();
+  (void)mbar_try_wait(bar, parity);
+}
+
+// dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half
+// precision, dx = ag * dyh + c1 * x + c2.
+template <typename T, int ACT>
+__device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw, const float (&a)[8],
+                                               const float (&b)[8], const float (&ag)[8], const float (&c1)[8],
+                                               const float (&c2)[8]) {
+  static_assert(sizeof(T) == 2, "16-bit tensors only");
+  float fx[8], fd[8], o[8];
+  unpack16<T, 8>(xw, fx);
+  unpack16<T, 8>(dw, fd);
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    float g0 = 1.f, g1 = 1.f;
+    if constexpr (ACT != kActIdentity) {
+      const float yh0 = fmaf(fx[2 * p], a[2 * p], b[2 * p]);
+      const float yh1 = fmaf(fx[2 * p + 1], a[2 * p + 1], b[2 * p + 1]);
+      const float2 gf = __half22float2(act_grad_h2<ACT>(f32x2_to_h2_sat(yh0, yh1)));
+      g0 = gf.x;
+      g1 = gf.y;
+    }
+    o[2 * p] = fmaf(ag[2 * p], fd[2 * p] * g0, fmaf(c1[2 * p], fx[2 * p], c2[2 * p]));
+    o[2 * p + 1] = fmaf(ag[2 * p + 1], fd[2 * p + 1] * g1, fmaf(c1[2 * p + 1], fx[2 * p + 1], c2[2 * p + 1]));
+  }
+  return pack16<T, 8>(o);
+}
+
+}  // namespace gnb200

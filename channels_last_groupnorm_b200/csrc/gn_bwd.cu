@@ -891,6 +891,11 @@ cudaError_t launch_param_exchange(const BwdCall& c, int C, cudaStream_t stream, 
 }
 
 cudaError_t launch_backward(const BwdCall& c, const Plan& p, cudaStream_t stream) {
+  if (p.resident) {
+    const cudaError_t err = launch_backward_resident(c, p.rgeom, stream);
+    if (err == cudaSuccess) return launch_param_exchange(c, p.rgeom.g.C, stream, false, true, c.peer && c.peer->collect);
+    if (err != cudaErrorCooperativeLaunchTooLarge) return err;
+  }
   if (p.wave) {
     // the wave kernel finishes dgamma / dbeta itself; the exchange over the ranks follows it
     const cudaError_t err = launch_backward_wave(c, p, stream);

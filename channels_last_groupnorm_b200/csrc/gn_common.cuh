@@ -685,6 +685,23 @@ struct WaveGeom {
   unsigned long long* trace;  // optional timeline buffer (tuning aid), else null
 };
 
+// Geometry of the resident plan (gn_resident.cu): one CTA per SM; every sample's rows are cut into `cps`
+// contiguous row ranges, and a CTA streams its range - whole rows, hence one contiguous run of memory - in
+// tiles of BR rows through a ring of `stages` shared-memory stages.
+constexpr int kResidentThreads = 512;
+constexpr int kResidentRows = 2;  // rows per thread and tile
+struct ResidentGeom {
+  Geom g;              // CW = C, ncb = 1, slots = G; rows_per_cta, chunks = cps
+  int cps;             // CTAs per sample
+  int BR;              // rows per tile (kResidentRows * TY)
+  int tile_bytes;      // BR * C * sizeof(T), one tensor
+  int stages;
+  int threads;
+  long long grid;      // N * cps
+  size_t smem_bytes;
+  size_t ws_bytes;     // scratch the kernel itself needs
+};
+
 // Groups touched by column block starting at channel c0 (width CW, clipped to C):
 // first group and how many.
 __device__ __forceinline__ void cb_groups(const Geom& g, int c0, int& g_lo, int& n_slots) {

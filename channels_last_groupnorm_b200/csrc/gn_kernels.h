@@ -21,6 +21,10 @@ struct Plan {
   bool chain;         // kernels after the first are launched as programmatic dependents of their predecessor
   Geom geom;
   WaveGeom wgeom;
+  // Backward: the resident kernel (gn_resident.cu) takes the place of the multi-kernel or wave plan described by the
+  // fields above, which stay filled in: they are what runs where the grid cannot be resident at once.
+  bool resident;
+  ResidentGeom rgeom;
 };
 
 struct FwdCall {
@@ -86,6 +90,13 @@ void debug_set_trace(void* ptr, size_t bytes);
 size_t wave_workspace_bytes(const WaveGeom& g, int direction);
 cudaError_t launch_forward_wave(const FwdCall& c, const Plan& p, cudaStream_t stream);
 cudaError_t launch_backward_wave(const BwdCall& c, const Plan& p, cudaStream_t stream);
+// resident plan (gn_resident.cu).  cudaErrorCooperativeLaunchTooLarge: nothing was launched, the device (or the
+// share of it that this process has) cannot hold the grid
+cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream);
+size_t resident_workspace_bytes(const ResidentGeom& r);
+size_t resident_fixed_smem(const ResidentGeom& r);  // shared memory besides the stages
+// cudaSuccess if `grid` CTAs of this kernel can be resident at once on the current device
+cudaError_t check_resident(const void* func, int threads, size_t smem, long long grid);
 // dgamma / dbeta from `rows` rows of per-channel (S1, S2) pairs (gn_bwd.cu)
 // `chained`: as a programmatic dependent of the kernel before it in the stream
 cudaError_t launch_param_grads(const BwdCall& c, const float* sums, int rows, int C, cudaStream_t stream,

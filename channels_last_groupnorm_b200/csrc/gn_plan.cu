@@ -430,9 +430,74 @@ bool plan_wave(const Shape& sh, Plan* out) {
   return true;
 }
 
+// Resident plan (gn_resident.cu), backward, in place of the multi-kernel or wave plan in *plan.  A sample's rows are
+// cut into cps = 148 / N contiguous ranges, one CTA per SM; at least 85 % of the SMs must get one.  Tiles hold two rows
+// per thread (16 KB each of x and dy); what is left of the SM's shared memory holds as many of them as fit.
+// The line: measured on B200, us, resident / the plan it replaces (w wave, m multi-kernel):
+//   fp16  512@256^2 64.2 / 68.7 w    256@512^2 118 / 129 w    128@1024^2 226 / 242 m    2 x 256@512x256 117 / 125 w
+//   bf16  3 x 512@200x300 158 / 167 w    20 x 96@320x90, 3 groups 107 / 145 w
+//   bf16, one group per sample  8 x 1024@64^2 72 / 140 m    1 x 512@64^2 16.5 / 100 m (one CTA of that plan's finalize
+//         kernel adds up all channels of a group)    fp32  8 x 512@64^2 79 / 115 m
+//   fp32  256@512^2, 32 groups 258 / 249 w: with fp32 arithmetic both passes are bound by instruction issue, where
+//         sixteen warps per SM do worse - so fp32 takes it only for wide groups.
+// GNB200_RESIDENT_CTAS / _STAGES (tests, experiments) bound the CTAs per sample and the stages.
+bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
+  const int ve = sh.ve, s = sh.s;
+  if (sh.direction != 1 || ve == 1 || sh.N > kSmCount) return false;
+  if (sh.G > 128) return false;  // every CTA merges cps * G partials
+  if (!forced && s == 4 && sh.D < 128) return false;
+  const int CV = sh.C / ve;
+  if (CV > kResidentThreads) return false;
+  ResidentGeom r = {};
+  int cps = kSmCount / sh.N;
+  const int max_ctas = env_int("GNB200_RESIDENT_CTAS", 0);
+  if (max_ctas > 0 && cps > max_ctas) cps = max_ctas;
+  if (cps > sh.R) cps = sh.R;
+  if (!forced && sh.N * cps < kSmCount * 85 / 100) return false;
+  const int rows = (sh.R + cps - 1) / cps;
+  cps = (sh.R + rows - 1) / rows;
+  Geom g = {};
+  g.N = sh.N, g.R = sh.R, g.C = sh.C, g.G = sh.G, g.D = sh.D;
+  g.CW = sh.C, g.CV = CV, g.TY = kResidentThreads / CV;
+  g.ncb = 1, g.rows_per_cta = rows, g.chunks = cps, g.slots = sh.G, g.k = 1;
+  g.persist = 1, g.skip_push_rank = -1;
+  g.red_floats = g.TY * sh.C;  // reductions over the row lanes; later the warps' sums of a merge
+  if (g.red_floats < 2 * (kResidentThreads / 32) * sh.G) g.red_floats = 2 * (kResidentThreads / 32) * sh.G;
+  g.div_D = make_fast_div(sh.D);
+  g.div_CV = make_fast_div(CV);
+  g.div_CW = make_fast_div(sh.C);
+  g.div_ncb = make_fast_div(1);
+  g.div_chunks = make_fast_div(cps);
+  r.g = g;
+  r.cps = cps;
+  r.BR = kResidentRows * g.TY;
+  r.tile_bytes = r.BR * sh.C * s;
+  r.threads = round_up(CV * g.TY, 32);
+  r.grid = (long long)sh.N * cps;
+  const size_t fixed = resident_fixed_smem(r), stage = (size_t)2 * r.tile_bytes;
+  const size_t room = kSmemMaxOptin - 1024;
+  if (fixed + 2 * stage > room) return false;
+  r.stages = (int)((room - fixed) / stage);
+  const int max_stages = env_int("GNB200_RESIDENT_STAGES", 16);
+  if (r.stages > max_stages) r.stages = max_stages < 2 ? 2 : max_stages;
+  if (r.stages > 16) r.stages = 16;
+  r.smem_bytes = fixed + (size_t)r.stages * stage;
+  r.ws_bytes = resident_workspace_bytes(r);
+  // The scratch limits of callers stay what they are: a call never asks for less than the plan that this one
+  // replaces, nor - beyond the 4 MiB that every backward call may rely on - for more.
+  const size_t static_limit = 4u << 20;
+  if (!forced && r.ws_bytes > plan->ws_bytes && r.ws_bytes > static_limit) return false;
+  if (r.ws_bytes > plan->ws_bytes) plan->ws_bytes = r.ws_bytes;
+  plan->resident = true;
+  plan->launches = 1;
+  plan->rgeom = r;
+  return true;
+}
+
 }  // namespace
 
 static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan);
+static bool plan_streaming(const Shape& sh, bool twopass_only, bool wave_only, Plan* plan);
 
 bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan) {
   if (!make_plan_inner(N, R, C, G, dtype, direction, aligned16, plan)) return false;
@@ -457,12 +522,19 @@ static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
   const int vfull = 16 / sh.s;
   sh.ve = (aligned16 && C % vfull == 0) ? vfull : 1;
   sh.direction = direction;
-  // GNB200_FORCE_PATH = twopass: the multi-kernel plan; wave: the wave plan where the shape allows it
+  // GNB200_FORCE_PATH = twopass: the multi-kernel plan; wave, resident: these plans where the shape allows it
   const char* force = getenv("GNB200_FORCE_PATH");
   const bool twopass_only = force && !strcmp(force, "twopass");
-  const bool skip_fused = twopass_only || (force && !strcmp(force, "wave"));
-  if (!skip_fused && plan_fused(sh, plan)) return true;
-  if (force && !strcmp(force, "wave")) {
+  const bool wave_only = force && !strcmp(force, "wave"), resident_only = force && !strcmp(force, "resident");
+  if (!twopass_only && !wave_only && !resident_only && plan_fused(sh, plan)) return true;
+  if (!plan_streaming(sh, twopass_only, wave_only, plan)) return false;
+  if (!twopass_only && !wave_only) plan_resident(sh, resident_only, plan);
+  return true;
+}
+
+// Slabs that do not fit a cluster: the wave plan or the multi-kernel plan
+static bool plan_streaming(const Shape& sh, bool twopass_only, bool wave_only, Plan* plan) {
+  if (wave_only) {
     if (plan_wave(sh, plan)) return true;
   } else if (!twopass_only && sh.direction == 1) {
     // Measured on B200 (1024-px VAE-decoder shapes, fp16 SiLU): the wave plan beats the multi-kernel plan

@@ -1,0 +1,463 @@
+// "Resident" launch plan for slabs that do not fit a thread-block cluster: backward GroupNorm (+activation) for
+// NHWC tensors as ONE persistent cooperative kernel, one CTA per SM, sm_100a.
+//
+// The sums of dyh and dyh * xh need every row of a sample before the first dx can be written, so these shapes take
+// two passes over x and dy.  What bounds them is HBM: how much of the second pass is read from there again, and what
+// lies between the passes.  Here a CTA owns one contiguous range of a sample's rows for both passes:
+//
+//   pass 1   the range streams through a ring of shared-memory stages (untiled cp.async.bulk copies: whole rows are
+//            one contiguous run, so no thread computes an address and no tensor map is needed); the last `stages`
+//            tiles are not overwritten: 148 x 192 KB, 28 MB, stay on chip
+//   barrier  partial sums to scratch, one arrival per CTA, bounded wait; every CTA merges what it needs
+//   pass 2   the resident tiles first - no read at all - and, as their stages become free, the tiles before them
+//            in reverse order, so that what was read last (and L2 still holds) is read first; dx leaves with
+//            streaming (evict-first) stores
+//
+// dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.  The same kernel for the
+// forward direction gained less over the three chained kernels than it lost on small slabs (fp16, us: 67 MB 39.2 / 39.8,
+// 134 MB 73.6 / 74.8, 4 MB 16.5 / 8.8) and was left out: its arithmetic is short and there is half as much to keep.
+// Measured against the plan it replaces: see the rule in gn_plan.cu.
+//
+// Every sum is formed in an order fixed by the launch geometry: bit-identical reruns.
+// The passes restate what src/gnnhwc/csrc/gn_kernel.cu:533-872 of the reference computes.
+#include "gn_async.cuh"
+#include "gn_kernels.h"
+#include "gn_math.cuh"
+
+namespace gnb200 {
+
+namespace {
+
+constexpr int kMaxStages = 16;
+constexpr int kMergeLoads = 5;   // channel-sum rows a lane has in flight in the dgamma / dbeta sums
+constexpr int kMergeRows = 10;   // partial rows a warp has in flight in a merge (148 CTAs / 16 warps)
+
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
+
+// Shared memory: [stages * (x tile, dy tile)][full][empty][flags][reduction scratch]
+struct Smem {
+  uint32_t stage0;
+  uint64_t* full;
+  uint64_t* empty;
+  int* flags;  // [0] a wait gave up
+  float* red;
+};
+__device__ __forceinline__ Smem carve(const ResidentGeom& r, unsigned char* base) {
+  Smem s;
+  s.stage0 = smem_addr(base);
+  unsigned char* p = base + (size_t)r.stages * 2 * r.tile_bytes;  // tile_bytes is a multiple of 16
+  s.full = reinterpret_cast<uint64_t*>(p);
+  s.empty = s.full + kMaxStages;
+  s.flags = reinterpret_cast<int*>(s.empty + kMaxStages);
+  s.red = reinterpret_cast<float*>(s.flags + 4);
+  return s;
+}
+constexpr size_t kControlBytes = 2 * kMaxStages * 8 + 16;
+
+// The stage sequence of both passes, as thread 0 (which issues the copies) and all threads walk it.  Tile t
+// lives in stage t % stages in both passes; the parity of a barrier's current phase is one bit per stage.
+template <typename T>
+struct Stream {
+  const T* src[2];  // x, dy: first element of the CTA's row range
+  int tiles, nrows, BR, stages;
+  uint32_t row_bytes, tile_bytes;
+  unsigned full_ph, empty_ph;
+  Smem sm;
+
+  __device__ __forceinline__ void issue(int t, int stage) {  // thread 0
+    const uint32_t bytes = (uint32_t)min(BR, nrows - t * BR) * row_bytes;
+    mbar_arrive_expect_tx(&sm.full[stage], 2 * bytes);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      bulk_load(sm.stage0 + (uint32_t)(stage * 2 + i) * tile_bytes,
+                reinterpret_cast<const char*>(src[i]) + (size_t)t * tile_bytes, bytes, &sm.full[stage]);
+  }
+  // thread 0: waits until every warp has handed the stage back, then refills it.  Without the hand-back
+  // (its wait gave up) nothing is copied over a stage that may still be read.
+  __device__ __forceinline__ void refill(int t, int stage, const WaitLimit& lim) {
+    producer_wait(&sm.empty[stage], (empty_ph >> stage) & 1u, &sm.flags[0], lim);
+    empty_ph ^= 1u << stage;
+    if (*(volatile int*)&sm.flags[0] == 0) issue(t, stage);
+  }
+  __device__ __forceinline__ void wait_full(int stage, const WaitLimit& lim) {
+    consumer_wait(&sm.full[stage], (full_ph >> stage) & 1u, &sm.flags[0], lim);
+    full_ph ^= 1u << stage;
+  }
+};
+
+template <typename T>
+__device__ __forceinline__ void stream_start(Stream<T>& st, const ResidentGeom& r, const Smem& sm, int nrows) {
+  st.sm = sm;
+  st.nrows = nrows;
+  st.BR = r.BR;
+  st.stages = r.stages;
+  st.tiles = (nrows + r.BR - 1) / r.BR;
+  st.row_bytes = (uint32_t)(r.g.C * (int)sizeof(T));
+  st.tile_bytes = (uint32_t)r.tile_bytes;
+  st.full_ph = st.empty_ph = 0;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < r.stages; ++s) {
+      mbar_init(&sm.full[s], 1);
+      mbar_init(&sm.empty[s], blockDim.x >> 5);
+    }
+    sm.flags[0] = 0;
+    fence_mbar_init_cluster();
+    for (int t = 0; t < min(r.stages, st.tiles); ++t) st.issue(t, t);
+  }
+  __syncthreads();
+}
+
+// Grid barrier: every CTA has written its partial sums.  `count` starts at 0 (cleared in stream order
+// before the launch).  A wait that gives up sets flags[0]; the caller then writes NaN.
+__device__ __forceinline__ void grid_barrier(unsigned int* count, int* flags, const WaitLimit& lim) {
+  __syncwarp();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(count, 1u);
+    const long long t0 = clock64();
+    unsigned int polls = 0;
+    while (ld_acquire_u32(count) < gridDim.x) {
+      if (++polls > lim.polls && clock64() - t0 > lim.clocks) {
+        wait_gave_up(lim);
+        flags[0] = 1;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+}
+
+// Sums over `rows` partial rows of G pairs each: warp w takes the rows w, w + nwarps, ..., lane l the groups l, l + 32, ...;
+// acc[w * G + s], acc[(nwarps + w) * G + s] receive the warp's two sums of group s, formed in row order.  All CTAs of
+// a sample read the same rows at the same moment, so what counts is the number of L2 requests: with one warp per
+// group and a lane per row (32 requests of 8 or 16 bytes per load) a merge of 32 groups x 148 rows took 8.1 us.
+__device__ __forceinline__ void merge_rows(const float2* p, int rows, int G, int warp, int nwarps, int lane, float* acc) {
+  for (int s = lane; s < G; s += 32) {
+    float a1 = 0.f, a2 = 0.f;
+    for (int i0 = warp; i0 < rows; i0 += nwarps * kMergeRows) {
+      float2 v[kMergeRows];
+#pragma unroll
+      for (int q = 0; q < kMergeRows; ++q) {
+        const int i = i0 + nwarps * q;
+        v[q] = i < rows ? __ldcg(p + (size_t)i * G + s) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < kMergeRows; ++q) a1 += v[q].x, a2 += v[q].y;
+    }
+    acc[warp * G + s] = a1;
+    acc[(nwarps + warp) * G + s] = a2;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// scratch: tpart[cta * C + c] = (S1, S2) of channel c over the CTA's rows,
+//          gpart[cta * G + s] = gamma-weighted sums of group s over the CTA's rows.
+// ------------------------------------------------------------------------------------------------
+template <typename T, int ACT, bool UNI>
+__global__ void __launch_bounds__(kResidentThreads, 1)
+    gn_bwd_resident_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
+                           const T* __restrict__ beta, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
+                           T* __restrict__ dx, float2* tpart, float2* gpart, unsigned int* count,
+                           float* __restrict__ dparam_f32, T* __restrict__ dgamma, T* __restrict__ dbeta,
+                           const ResidentGeom r) {
+  constexpr int VE = 16 / sizeof(T);
+  constexpr int KR = kResidentRows;
+  constexpr bool kRaw = sizeof(T) == 2;  // 16-bit tensors: packed arithmetic, S2 against the raw x
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const Geom& g = r.g;
+  const Smem sm = carve(r, smem_raw);
+  float* red = sm.red;              // TY * C
+  float* chan = red + g.red_floats;  // S1[C], S2[C]
+  float* coef = chan + 2 * g.C;      // A[G], B[G]
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
+  const int n = g.div_chunks.div((int)blockIdx.x), j = (int)blockIdx.x - n * r.cps;
+  const int r0 = j * g.rows_per_cta;
+  const int nrows = min(g.rows_per_cta, g.R - r0);
+  const int ty = g.div_CV.div(tid), tx = tid - ty * g.CV;
+  const bool streaming = ty < g.TY;
+  const size_t row0 = (size_t)n * g.R + r0;
+
+  Stream<T> st;
+  st.src[0] = x + row0 * g.C;
+  st.src[1] = dy + row0 * g.C;
+  stream_start(st, r, sm, nrows);
+  const int T_ = st.tiles, S = st.stages;
+  const uint32_t my_off = sm.stage0 + (streaming ? (uint32_t)(ty * g.CV + tx) * 16u : 0u);
+  const uint32_t step = (uint32_t)(g.TY * g.CV) * 16u;
+  const int my_row = streaming ? ty : 0x40000000;
+
+  BwdLane<T, VE> L;
+  float a[VE], b[VE];
+#pragma unroll
+  for (int e = 0; e < VE; ++e) L.r[e] = L.nmr[e] = L.ga[e] = L.be[e] = 0.f;
+  if (streaming)
+    lane_setup<T, VE, UNI>(gamma, beta, mean_in + (size_t)n * g.G, rstd_in + (size_t)n * g.G, tx * VE, g.div_D, L);
+#pragma unroll
+  for (int e = 0; e < VE; ++e) {
+    a[e] = L.r[e] * L.ga[e];
+    b[e] = fmaf(L.nmr[e], L.ga[e], L.be[e]);
+  }
+
+  // ---- pass 1: S1, S2 over the thread's rows
+  float s1[VE], s2[VE];
+#pragma unroll
+  for (int e = 0; e < VE; ++e) s1[e] = 0.f, s2[e] = 0.f;
+  int stage = 0, prev = 0;
+  for (int t = 0; t < T_; ++t) {
+    st.wait_full(stage, g.wait);
+    const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
+    const int here = nrows - t * st.BR;
+    uint4 xw[KR], dw[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      xw[u] = lds128(base + u * step);
+      dw[u] = lds128(base + st.tile_bytes + u * step);
+    }
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      if (my_row + u * g.TY < here) {
+        if constexpr (kRaw) {
+          bwd_row_sums_packed<T, ACT>(xw[u], dw[u], a, b, s1, s2);
+        } else {
+          float fx[VE], fd[VE];
+          unpack16<T, VE>(xw[u], fx);
+          unpack16<T, VE>(dw[u], fd);
+          bwd_row_sums<T, VE, ACT>(fx, fd, L, s1, s2);
+        }
+      }
+    }
+    pin_regs(s1);
+    pin_regs(s2);
+    if (t + S < T_) release_stage(&sm.empty[stage], lane);
+    if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
+    prev = stage;
+    if (++stage == S) stage = 0;
+  }
+  if constexpr (kRaw) {  // S2 = sum dyh * xh = rstd * (sum dyh * x - mean * sum dyh)
+#pragma unroll
+    for (int e = 0; e < VE; ++e) s2[e] = fmaf(L.r[e], s2[e], L.nmr[e] * s1[e]);
+  }
+  // channel sums over the row lanes, S1 and S2 one after the other through the same scratch
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    __syncwarp();
+    __syncthreads();
+    if (streaming) {
+#pragma unroll
+      for (int e = 0; e < VE; e += 4) {
+        const float4 v = which == 0 ? make_float4(s1[e], s1[e + 1], s1[e + 2], s1[e + 3])
+                                    : make_float4(s2[e], s2[e + 1], s2[e + 2], s2[e + 3]);
+        *reinterpret_cast<float4*>(red + (size_t)ty * g.C + tx * VE + e) = v;
+      }
+    }
+    __syncthreads();
+    for (int c = tid; c < g.C; c += blockDim.x) {
+      float acc = 0.f;
+#pragma unroll 4
+      for (int q = 0; q < g.TY; ++q) acc += red[(size_t)q * g.C + c];
+      chan[which * g.C + c] = acc;
+    }
+  }
+  __syncthreads();
+  for (int c = tid; c < g.C; c += blockDim.x) tpart[(size_t)blockIdx.x * g.C + c] = make_float2(chan[c], chan[g.C + c]);
+  for (int s = warp; s < g.G; s += nwarps) {  // gamma-weighted group sums of the CTA's rows
+    float w1 = 0.f, w2 = 0.f;
+    for (int c = s * g.D + lane; c < (s + 1) * g.D; c += 32) {
+      const float ga = load_param<T>(gamma, c);
+      w1 = fmaf(ga, chan[c], w1);
+      w2 = fmaf(ga, chan[g.C + c], w2);
+    }
+    w1 = warp_sum_all(w1);
+    w2 = warp_sum_all(w2);
+    if (lane == 0) gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2);
+  }
+  grid_barrier(count, sm.flags, g.wait);
+
+  // ---- A, B of the sample's groups
+  const bool ok = *(volatile int*)&sm.flags[0] == 0;
+  const float inv_m = ok ? 1.0f / ((float)g.D * (float)g.R) : kNaN;
+  {
+    float* acc = red;  // [2][nwarps][G]
+    merge_rows(gpart + (size_t)n * r.cps * g.G, r.cps, g.G, warp, nwarps, lane, acc);
+    __syncthreads();
+    for (int s = tid; s < g.G; s += blockDim.x) {
+      float w1 = 0.f, w2 = 0.f;
+      for (int w = 0; w < nwarps; ++w) {
+        w1 += acc[w * g.G + s];
+        w2 += acc[(nwarps + w) * g.G + s];
+      }
+      coef[s] = w1 * inv_m;
+      coef[g.G + s] = w2 * inv_m;
+    }
+  }
+  __syncthreads();
+
+  // ---- pass 2: dx = ag dyh - r (A + xh B), with xh = r x + nmr:  c1 x + c2 (16-bit) or c1 xh + c2 (fp32)
+  float c1[VE], c2[VE];
+#pragma unroll
+  for (int e = 0; e < VE; ++e) c1[e] = c2[e] = 0.f;
+  if (streaming) {
+#pragma unroll
+    for (int e = 0; e < VE; ++e) {
+      const int s = g.div_D.div(tx * VE + (UNI ? 0 : e));
+      const float nb = -L.r[e] * coef[g.G + s], na = -L.r[e] * coef[s];
+      c1[e] = kRaw ? nb * L.r[e] : nb;
+      c2[e] = kRaw ? fmaf(nb, L.nmr[e], na) : na;
+    }
+  }
+  T* out = dx + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
+  const size_t ostep = (size_t)g.TY * g.C;
+  stage = prev;
+  for (int t = T_ - 1; t >= 0; --t) {
+    if (t < T_ - S) st.wait_full(stage, g.wait);
+    const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
+    const int here = nrows - t * st.BR;
+    T* o = out + (size_t)t * st.BR * g.C;
+    uint4 xw[KR], dw[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      xw[u] = lds128(base + u * step);
+      dw[u] = lds128(base + st.tile_bytes + u * step);
+    }
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      if (my_row + u * g.TY < here) {
+        if constexpr (kRaw) {
+          stg128_stream(o + (size_t)u * ostep, bwd_dx_packed<T, ACT>(xw[u], dw[u], a, b, a, c1, c2));
+        } else {
+          float fx[VE], fd[VE], xh[VE], yh[VE], gr[VE];
+          unpack16<T, VE>(xw[u], fx);
+          unpack16<T, VE>(dw[u], fd);
+#pragma unroll
+          for (int e = 0; e < VE; ++e) {
+            xh[e] = fmaf(fx[e], L.r[e], L.nmr[e]);
+            yh[e] = fmaf(xh[e], L.ga[e], L.be[e]);
+          }
+          act_grad_vec<T, VE, ACT>(yh, gr);
+#pragma unroll
+          for (int e = 0; e < VE; ++e) fx[e] = fmaf(a[e], fd[e] * gr[e], fmaf(c1[e], xh[e], c2[e]));
+          stg128_stream(o + (size_t)u * ostep, pack16<T, VE>(fx));
+        }
+      }
+    }
+    if (t >= S) release_stage(&sm.empty[stage], lane);
+    if (tid == 0 && t + 1 < T_ && t + 1 >= S) st.refill(t + 1 - S, prev, g.wait);
+    prev = stage;
+    stage = stage == 0 ? S - 1 : stage - 1;
+  }
+
+  // ---- dgamma / dbeta: the grid's warps share the channels; all channel sums are visible since the barrier
+  const int rows = g.N * r.cps;
+  const bool bad = *(volatile int*)&sm.flags[0] != 0;
+  for (int c = (int)blockIdx.x + (int)gridDim.x * warp; c < g.C; c += (int)gridDim.x * nwarps) {
+    float t1 = 0.f, t2 = 0.f;
+    for (int i0 = lane; i0 < rows + lane; i0 += 32 * kMergeLoads) {
+      float2 v[kMergeLoads];
+#pragma unroll
+      for (int q = 0; q < kMergeLoads; ++q) {
+        const int i = i0 + 32 * q;
+        v[q] = i < rows ? __ldcg(tpart + (size_t)i * g.C + c) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < kMergeLoads; ++q) t1 += v[q].x, t2 += v[q].y;
+    }
+    t1 = warp_sum_all(t1);
+    t2 = warp_sum_all(t2);
+    if (lane == 0) {
+      if (bad) t1 = t2 = kNaN;
+      dparam_f32[c] = t2;
+      dparam_f32[g.C + c] = t1;
+      if (dgamma) dgamma[c] = store_param<T>(t2);
+      if (dbeta) dbeta[c] = store_param<T>(t1);
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// host side
+// ------------------------------------------------------------------------------------------------
+struct Scratch {
+  size_t gpart, count, total;  // channel sums first
+};
+Scratch scratch_of(const ResidentGeom& r) {
+  Scratch s;
+  s.gpart = (size_t)r.grid * r.g.C * sizeof(float2);
+  s.count = s.gpart + (size_t)r.grid * r.g.G * sizeof(float2);
+  s.total = (s.count + 4 + 15) & ~(size_t)15;
+  return s;
+}
+
+template <typename Kern, typename... Args>
+cudaError_t launch(Kern kern, const ResidentGeom& r, unsigned int* count, cudaStream_t stream, Args... args) {
+  cudaError_t err = ensure_kernel_attributes((const void*)kern, r.smem_bytes, false);
+  if (err != cudaSuccess) return err;
+  err = check_resident((const void*)kern, r.threads, r.smem_bytes, r.grid);
+  if (err != cudaSuccess) return err;
+  err = cudaMemsetAsync(count, 0, sizeof(unsigned int), stream);
+  if (err != cudaSuccess) return err;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)r.grid, 1, 1);
+  cfg.blockDim = dim3((unsigned)r.threads, 1, 1);
+  cfg.dynamicSmemBytes = r.smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <typename T, int ACT, bool UNI>
+cudaError_t launch_u(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+  const Scratch s = scratch_of(r);
+  char* ws = static_cast<char*>(c.workspace);
+  unsigned int* count = reinterpret_cast<unsigned int*>(ws + s.count);
+  return launch(gn_bwd_resident_kernel<T, ACT, UNI>, r, count, stream, (const T*)c.dy, (const T*)c.x, (const T*)c.gamma,
+                (const T*)c.beta, c.mean, c.rstd, (T*)c.dx, reinterpret_cast<float2*>(ws),
+                reinterpret_cast<float2*>(ws + s.gpart), count, c.dparam_f32, (T*)c.dgamma, (T*)c.dbeta, r);
+}
+template <typename T, int ACT>
+cudaError_t launch_t(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+  constexpr int VE = 16 / sizeof(T);
+  return r.g.D % VE == 0 ? launch_u<T, ACT, true>(c, r, stream) : launch_u<T, ACT, false>(c, r, stream);
+}
+template <typename T>
+cudaError_t launch_act(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+  switch (c.act) {
+    case kActIdentity: return launch_t<T, kActIdentity>(c, r, stream);
+    case kActRelu: return launch_t<T, kActRelu>(c, r, stream);
+    case kActSilu: return launch_t<T, kActSilu>(c, r, stream);
+    case kActGelu: return launch_t<T, kActGelu>(c, r, stream);
+    default: return launch_t<T, kActGeluTanh>(c, r, stream);
+  }
+}
+
+}  // namespace
+
+size_t resident_workspace_bytes(const ResidentGeom& r) { return scratch_of(r).total; }
+
+size_t resident_fixed_smem(const ResidentGeom& r) {
+  const Geom& g = r.g;
+  return kControlBytes + ((size_t)g.red_floats + 2 * (size_t)g.C + 2 * (size_t)g.G) * 4 + 16;
+}
+
+cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& geom, cudaStream_t stream) {
+  ResidentGeom r = geom;
+  const cudaError_t err = wait_limit_for_device(&r.g.wait);
+  if (err != cudaSuccess) return err;
+  switch (c.dtype) {
+    case 0: return launch_act<float>(c, r, stream);
+    case 1: return launch_act<__half>(c, r, stream);
+    default: return launch_act<__nv_bfloat16>(c, r, stream);
+  }
+}
+
+}  // namespace gnb200

@@ -25,6 +25,7 @@
 #include <map>
 #include <mutex>
 
+#include "gn_async.cuh"
 #include "gn_kernels.h"
 #include "gn_math.cuh"
 
@@ -43,26 +44,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap
       "l"(tm), "r"(c), "r"(row), "r"(smem_addr(bar))
       : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-// A consumer warp hands a stage back to the producer only after it has USED the vectors it read from
-// the stage.  The shared-memory loads are merely issued when the warp moves on; signalling the stage
-// as free right after them let the producer's next TMA copy into the stage (fast when the rows come from
-// L2) now and then overtake a load that was still queued, and a warp computed one stage's rows from
-// pieces of a later stage.  So the arrival follows the arithmetic in program order - instructions
-// issue in order and the arithmetic cannot issue before its operands have arrived - and pin_regs keeps
-// the compiler from moving that arithmetic behind the arrival (the output stores of pass B are
-// volatile asm statements and stay in front of it by themselves).
-template <int N>
-__device__ __forceinline__ void pin_regs(float (&a)[N]) {
-#pragma unroll
-  for (int e = 0; e < N; ++e) asm volatile("" : "+f"(a[e]));
-}
-__device__ __forceinline__ void release_stage(uint64_t* empty_bar, int lane) {
-  __syncwarp();
-  if (lane == 0) mbar_arrive(empty_bar);
-}
 // Block barrier of the consumer warps only (the producer warp never joins it).  The call sites
 // follow code in which single lanes of a warp act alone (lane 0 stores a partial, thread 0 counts a
 // delivery), so the warp is brought together first and the barrier is the form that counts threads
@@ -71,21 +52,6 @@ __device__ __forceinline__ void release_stage(uint64_t* empty_bar, int lane) {
 __device__ __forceinline__ void consumer_sync(int consumers) {
   __syncwarp();
   asm volatile("barrier.sync 1, %0;" ::"r"(consumers) : "memory");
-}
-__device__ __forceinline__ float warp_sum_all(float v) {
-#pragma unroll
-  for (int b = 16; b >= 1; b >>= 1) v += __shfl_xor_sync(0xffffffffu, v, b);
-  return v;
-}
-// streaming 16-byte store: the line is marked evict-first, so results do not push the rows that
-// pass B still has to read out of L2
-__device__ __forceinline__ void stg128_stream(void* p, const uint4 v) {
-  asm volatile("st.global.cs.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 // counter + 1 with release and acquire semantics in one round trip: the writes this CTA made before
 // its block barrier are released, and if the returned value tells that every other CTA has
@@ -129,8 +95,6 @@ __device__ __forceinline__ bool wait_pair(const unsigned long long* word, const 
   return true;
 }
 
-#define kNaN __int_as_float(0x7fc00000)
-
 // Optional timeline for tuning (WaveGeom::trace, set with gnb200_debug_set_trace): thread 0 of every CTA
 // stores the global nanosecond timer at a few points of every step: trace[(cta * steps + step) * 4 + k].
 __device__ __forceinline__ void trace_mark(const WaveGeom& g, int step, int k) {
@@ -139,28 +103,6 @@ __device__ __forceinline__ void trace_mark(const WaveGeom& g, int step, int k) {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     g.trace[((size_t)blockIdx.x * (2 * g.waves) + step) * 4 + k] = t;  // (a team uses the first 2 * its waves steps)
   }
-}
-
-// mbarrier waits of the wave kernels.  `gave_up` is the CTA's shared flag: the first wait that runs
-// out sets it (and poisons the results, see the callers); from then on no wait of this CTA spends
-// its limit again, so a broken run ends after about one limit instead of one limit per stage.
-// producer (a single thread):
-__device__ __forceinline__ void producer_wait(uint64_t* bar, unsigned parity, volatile int* gave_up, const WaitLimit& lim) {
-  if (mbar_try_wait(bar, parity)) return;
-  if (*gave_up != 0) return;
-  if (!mbar_wait_bounded(bar, parity, lim)) *gave_up = 1;
-}
-// consumers (whole warps): if the phase is not complete yet, lane 0 alone polls - 256 polling threads
-// would take issue slots from the CTAs that share the SM - and afterwards every lane observes the
-// completed phase with one more try_wait of its own, which is what makes the TMA's writes visible
-// to it.
-__device__ __forceinline__ void consumer_wait(uint64_t* bar, unsigned parity, volatile int* gave_up, const WaitLimit& lim) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return;
-  if ((threadIdx.x & 31) == 0 && *gave_up == 0) {
-    if (!mbar_wait_bounded(bar, parity, lim)) *gave_up = 1;
-  }
-  __syncwarp();
-  (void)mbar_try_wait(bar, parity);
 }
 
 // One unit of work: the rows [r0, r1) of one (sample, column block) slab.
@@ -522,32 +464,6 @@ __global__ void __launch_bounds__(kWaveThreads, 3)
 // Only the small group sums are on the path between the passes; the channel sums are added up - for
 // dgamma / dbeta - by all CTAs together when they have finished their last unit.
 // ------------------------------------------------------------------------------------------------
-// dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half
-// precision, dx = ag * dyh + c1 * x + c2.
-template <typename T, int ACT>
-__device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw, const float (&a)[8],
-                                               const float (&b)[8], const float (&ag)[8], const float (&c1)[8],
-                                               const float (&c2)[8]) {
-  static_assert(sizeof(T) == 2, "16-bit tensors only");
-  float fx[8], fd[8], o[8];
-  unpack16<T, 8>(xw, fx);
-  unpack16<T, 8>(dw, fd);
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    float g0 = 1.f, g1 = 1.f;
-    if constexpr (ACT != kActIdentity) {
-      const float yh0 = fmaf(fx[2 * p], a[2 * p], b[2 * p]);
-      const float yh1 = fmaf(fx[2 * p + 1], a[2 * p + 1], b[2 * p + 1]);
-      const float2 gf = __half22float2(act_grad_h2<ACT>(f32x2_to_h2_sat(yh0, yh1)));
-      g0 = gf.x;
-      g1 = gf.y;
-    }
-    o[2 * p] = fmaf(ag[2 * p], fd[2 * p] * g0, fmaf(c1[2 * p], fx[2 * p], c2[2 * p]));
-    o[2 * p + 1] = fmaf(ag[2 * p + 1], fd[2 * p + 1] * g1, fmaf(c1[2 * p + 1], fx[2 * p + 1], c2[2 * p + 1]));
-  }
-  return pack16<T, 8>(o);
-}
-
 template <typename T, int ACT, bool UNI, int KR>
 __global__ void __launch_bounds__(kWaveThreads, 2)
     gn_bwd_wave_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_dy,
@@ -817,6 +733,37 @@ __global__ void __launch_bounds__(kWaveThreads, 2)
 
 }  // namespace
 
+// the cooperative grid of the plan must be resident at once
+cudaError_t check_resident(const void* func, int threads, size_t smem, long long grid) {
+  struct Key {
+    int dev;
+    const void* func;
+    size_t smem;
+    bool operator<(const Key& o) const {
+      if (dev != o.dev) return dev < o.dev;
+      if (func != o.func) return func < o.func;
+      return smem < o.smem;
+    }
+  };
+  static std::mutex mu;
+  static std::map<Key, long long> cache;
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  std::lock_guard<std::mutex> lock(mu);
+  const Key key = {dev, func, smem};
+  auto it = cache.find(key);
+  if (it == cache.end()) {
+    int per_sm = 0, sms = 0;
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, smem);
+    if (err != cudaSuccess) return err;
+    err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (err != cudaSuccess) return err;
+    it = cache.emplace(key, (long long)per_sm * sms).first;
+  }
+  return grid <= it->second ? cudaSuccess : cudaErrorCooperativeLaunchTooLarge;
+}
+
 namespace {
 
 // ------------------------------------------------------------------------------------------------
@@ -867,37 +814,6 @@ cudaError_t make_tensor_map(CUtensorMap* tm, const void* base, int dtype, const 
   const CUresult rc = enc(tm, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_NONE, promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
-// the cooperative grid of the plan must be resident at once
-cudaError_t check_resident(const void* func, int threads, size_t smem, long long grid) {
-  struct Key {
-    int dev;
-    const void* func;
-    size_t smem;
-    bool operator<(const Key& o) const {
-      if (dev != o.dev) return dev < o.dev;
-      if (func != o.func) return func < o.func;
-      return smem < o.smem;
-    }
-  };
-  static std::mutex mu;
-  static std::map<Key, long long> cache;
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return err;
-  std::lock_guard<std::mutex> lock(mu);
-  const Key key = {dev, func, smem};
-  auto it = cache.find(key);
-  if (it == cache.end()) {
-    int per_sm = 0, sms = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, threads, smem);
-    if (err != cudaSuccess) return err;
-    err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (err != cudaSuccess) return err;
-    it = cache.emplace(key, (long long)per_sm * sms).first;
-  }
-  return grid <= it->second ? cudaSuccess : cudaErrorCooperativeLaunchTooLarge;
 }
 
 template <typename Kern, typename... Args>

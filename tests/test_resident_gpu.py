@@ -1,0 +1,57 @@
+"""GPU parity tests of the resident plan (csrc/gn_resident.cu): both backward passes in one cooperative kernel, one CTA
+per SM, the last tiles of a CTA's row range kept in shared memory between the passes.
+
+GNB200_RESIDENT_CTAS / _STAGES bound the grid and the ring, so that tile remainders, stage reuse in both
+passes and ranges of one short tile are reached at sizes the CPU oracle finishes in seconds.
+Tolerances as everywhere: 1e-5 (fp32), 1e-2 (fp16 / bf16), max-abs error relative to max(1, max|oracle|).
+"""
+import pytest
+import torch
+
+from oracle import gn_oracle as O
+
+from .test_parity_gpu import DT, check_against, run_cabi
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # (N, C, spatial, G, dtype, act, CTAs per sample, stages)
+    (1, 256, (96, 96), 32, "float16", "silu", 0, 16),        # every SM, one or two tiles each, all resident
+    (2, 256, (96, 97), 32, "bfloat16", "gelu", 5, 2),         # many tiles through two stages, ragged last tile
+    (3, 128, (40, 57), 32, "float32", "gelu_tanh", 3, 3),     # fp32: xh form
+    (2, 320, (33, 47), 32, "float16", "silu", 4, 3),          # D = 10: vectors straddle groups; 32 idle threads
+    (1, 40, (131, 17), 8, "float32", "relu", 2, 2),           # D = 5, 10 vectors per row
+    (1, 64, (57, 31), 64, "float32", "identity", 7, 2),       # D = 1
+    (1, 2048, (9, 11), 32, "bfloat16", "silu", 3, 2),         # two row lanes
+    (1, 4096, (5, 7), 1, "float16", "gelu_tanh", 2, 2),       # one row lane: the widest row
+    (1, 8, (301, 3), 1, "float16", "identity", 2, 2),         # one vector per row
+    (148, 64, (8, 8), 8, "float16", "silu", 0, 16),           # one CTA per sample
+    (1, 128, (1, 5), 4, "float32", "silu", 0, 16),            # fewer rows than CTAs
+]
+
+
+@pytest.fixture(scope="module")
+def nt():
+    assert torch.cuda.is_available(), "GPU tests need a CUDA device"
+    from channels_last_groupnorm_b200 import _native
+
+    return _native
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "%dx%dx%s-g%d-%s-%s-%d-%d" % (c[0], c[1], "x".join(map(str, c[2])), *c[3:]))
+def test_resident_plan_against_oracle(nt, case, monkeypatch):
+    N, C, sp, G, dt, act, ctas, stages = case
+    monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
+    monkeypatch.setenv("GNB200_RESIDENT_CTAS", str(ctas))
+    monkeypatch.setenv("GNB200_RESIDENT_STAGES", str(stages))
+    assert " resident=1 " in nt.describe_plan(N, sp[0] * sp[1], C, G, DT[dt], 1)
+    x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=23, x_dist="uniform3")
+    out = run_cabi(nt, x, ga, be, dy, G, 1e-5, act)
+    want = O.oracle_c(x, ga, be, dy, G, 1e-5, act, threads=4)
+    check_against(out, want, DT[dt])
+    assert O.rel_err(out["dparam"][0], want["dgamma"]) <= O.TOLERANCE[DT[dt]]
+    assert O.rel_err(out["dparam"][1], want["dbeta"]) <= O.TOLERANCE[DT[dt]]
+    again = run_cabi(nt, x, ga, be, dy, G, 1e-5, act)  # fixed summation order: bit-identical reruns
+    for k in ("dx", "dparam"):
+        assert torch.equal(out[k], again[k]), k
+    assert nt.wait_timeouts() == 0
