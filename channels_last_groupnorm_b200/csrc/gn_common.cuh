@@ -660,6 +660,7 @@ struct Geom {
   WaitLimit wait;  // limits and give-up record of the bounded waits (set by the launcher)
   int skip_push_rank;  // -1; the exchange self-test names a cluster rank that withholds its pushes
   int persist;     // fused forward: the grid holds the resident clusters only, each looping over items
+  int back;        // multi-kernel forward: the output pass walks its tiles backwards
 };
 
 // Geometry of the wave plan (gn_wave.cu): a persistent cooperative kernel that takes the tensor

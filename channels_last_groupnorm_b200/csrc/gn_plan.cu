@@ -307,6 +307,8 @@ bool plan_two_pass(const Shape& sh, Plan* out) {
   }
   p.geom = Geom{sh.N, sh.R, sh.C, sh.G, sh.D, cw, CV, TY, ncb, (int)rows, (int)chunks, slots, 1};
   p.geom.persist = 0;
+  // L2 is 126 MB; at 134 MB walking back still pays, at 184 MB it is even, at 268 MB it costs 1 % (stream_apply)
+  p.geom.back = (double)sh.N * sh.R * sh.C * s <= 192.0 * 1024 * 1024 ? 1 : 0;
   fill_divisors(&p.geom, ve, sh.direction, threads, false);
   *out = p;
   return true;
