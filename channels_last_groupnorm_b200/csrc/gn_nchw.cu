@@ -14,6 +14,7 @@
 // Vectors are 16 bytes when R is a multiple of the vector width and the pointers are aligned (every
 // channel row then starts on a 16-byte boundary), single elements otherwise.  Sums are fp32, formed in
 // an order fixed by the launch geometry: no atomics, bit-identical reruns.
+#include "gn_async.cuh"
 #include "gn_kernels.h"
 #include "gn_math.cuh"
 
@@ -34,6 +35,7 @@ struct NchwGeom {
   long long piece_vecs;  // backward: vectors per warp piece
   int ppr;               // backward: pieces per channel row
   FastDiv div_R;         // element offset inside a slab -> channel (R < 2^31)
+  int evict;             // results leave with streaming stores
 };
 
 template <typename T, int VE>
@@ -45,10 +47,18 @@ __device__ __forceinline__ void load_vec(const T* p, float (&f)[VE]) {
     for (int e = 0; e < VE; ++e) f[e] = load_param<T>(p, e);
   }
 }
+// 16 bytes of a result.  A tensor that L2 can hold besides the inputs is left to the kernel that reads it next
+// (and streaming it measured 2 % slower); a larger one must not push out the inputs that are still to be read again.
+__device__ __forceinline__ void store16(void* p, const uint4 v, int evict) {
+  if (evict)
+    stg128_stream(p, v);
+  else
+    stg128(p, v);
+}
 template <typename T, int VE>
-__device__ __forceinline__ void store_vec(T* p, const float (&f)[VE]) {
+__device__ __forceinline__ void store_vec(T* p, const float (&f)[VE], int evict) {
   if constexpr (sizeof(T) * VE == 16) {
-    stg128(p, pack16<T, VE>(f));
+    store16(p, pack16<T, VE>(f), evict);
   } else {
 #pragma unroll
     for (int e = 0; e < VE; ++e) p[e] = store_param<T>(f[e]);
@@ -68,22 +78,38 @@ __global__ void __launch_bounds__(kThreads)
   const long long v0 = (long long)chunk * g.chunk_vecs;
   const long long v1 = min(g.slab_vecs, v0 + g.chunk_vecs);
   const T* base = x + slab * g.slab_vecs * VE;
-  // per-thread Welford over the lanes of its vectors (one count for all lanes)
+  // per-thread moments over the lanes of its vectors (one count for all lanes)
   float mean[VE], m2[VE], cnt = 0.f;
 #pragma unroll
   for (int e = 0; e < VE; ++e) mean[e] = 0.f, m2[e] = 0.f;
   long long v = v0 + threadIdx.x;
-  for (; v + (kUnroll - 1) * kThreads < v1; v += kUnroll * kThreads) {
-    float f[kUnroll][VE];
+  if constexpr (sizeof(T) == 2 && VE == 8) {
+    // 16-bit vectors: shifted sums about the thread's first element (gn_math.cuh), no division per vector, and the
+    // vectors stay packed while in flight
+    const int own = v < v1 ? (int)((v1 - v + kThreads - 1) / kThreads) : 0;
+    float K[1] = {own > 0 ? load_param<T>(base + v * VE, 0) : 0.f};
+    for (; v + (kUnroll - 1) * kThreads < v1; v += kUnroll * kThreads) {
+      uint4 w[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) load_vec<T, VE>(base + (v + u * kThreads) * VE, f[u]);
+      for (int u = 0; u < kUnroll; ++u) w[u] = ldg128(base + (v + u * kThreads) * VE);
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) welford_step<VE>(f[u], mean, m2, cnt);
-  }
-  for (; v < v1; v += kThreads) {
-    float f[VE];
-    load_vec<T, VE>(base + v * VE, f);
-    welford_step<VE>(f, mean, m2, cnt);
+      for (int u = 0; u < kUnroll; ++u) shifted_step<T, VE, 1>(w[u], K, mean, m2);
+    }
+    for (; v < v1; v += kThreads) shifted_step<T, VE, 1>(ldg128(base + v * VE), K, mean, m2);
+    shifted_finish<VE, 1>(K, own, mean, m2, cnt);
+  } else {
+    for (; v + (kUnroll - 1) * kThreads < v1; v += kUnroll * kThreads) {
+      float f[kUnroll][VE];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) load_vec<T, VE>(base + (v + u * kThreads) * VE, f[u]);
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) welford_step<VE>(f[u], mean, m2, cnt);
+    }
+    for (; v < v1; v += kThreads) {
+      float f[VE];
+      load_vec<T, VE>(base + v * VE, f);
+      welford_step<VE>(f, mean, m2, cnt);
+    }
   }
   // lanes -> thread, then threads -> CTA: mean first, squared deviations about it second
   float tsum = 0.f;
@@ -126,7 +152,9 @@ __device__ __forceinline__ void merge_partials(const float4* __restrict__ p, int
 }
 
 // ------------------------------------------------------------------------------------------------
-// forward 2: statistics of the slab, then y = act(x * a_c + b_c) over the chunk
+// forward 2: statistics of the slab, then y = act(x * a_c + b_c) over the chunk.  The chunks are visited in the
+// reverse order of the statistics kernel and walked from their end, and y leaves with streaming stores: what that
+// kernel read last is read first, while L2 still holds it.
 // ------------------------------------------------------------------------------------------------
 template <typename T, int VE, int ACT>
 __global__ void __launch_bounds__(kThreads)
@@ -135,8 +163,9 @@ __global__ void __launch_bounds__(kThreads)
                          float* __restrict__ rstd_out, float eps, const NchwGeom g) {
   constexpr bool FAST = sizeof(T) == 2;
   __shared__ float s_stat[2];
-  const long long slab = blockIdx.x / g.chunks;
-  const int chunk = (int)(blockIdx.x - slab * g.chunks);
+  const unsigned id = gridDim.x - 1 - blockIdx.x;
+  const long long slab = id / g.chunks;
+  const int chunk = (int)(id - slab * g.chunks);
   grid_dep_wait();  // the statistics kernel's partials
   if (threadIdx.x < 32) {
     float mu, rs;
@@ -166,21 +195,21 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
     for (int e = 0; e < VE; ++e) o[e] = fmaf(f[e], a, b);
     if constexpr (sizeof(T) * VE == 16) {
-      stg128(ys + v * VE, act_pack16<T, VE, ACT>(o));
+      store16(ys + v * VE, act_pack16<T, VE, ACT>(o), g.evict);
     } else {
 #pragma unroll
       for (int e = 0; e < VE; ++e) ys[v * VE + e] = store_param<T>(act_fwd<ACT, FAST>(o[e]));
     }
   };
-  long long v = v0 + threadIdx.x;
-  for (; v + (kUnroll - 1) * kThreads < v1; v += kUnroll * kThreads) {
+  long long v = v1 - 1 - threadIdx.x;
+  for (; v - (kUnroll - 1) * kThreads >= v0; v -= kUnroll * kThreads) {
     float f[kUnroll][VE];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) load_vec<T, VE>(xs + (v + u * kThreads) * VE, f[u]);
+    for (int u = 0; u < kUnroll; ++u) load_vec<T, VE>(xs + (v - u * kThreads) * VE, f[u]);
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) one(v + u * kThreads, f[u]);
+    for (int u = 0; u < kUnroll; ++u) one(v - u * kThreads, f[u]);
   }
-  for (; v < v1; v += kThreads) {
+  for (; v >= v0; v -= kThreads) {
     float f[VE];
     load_vec<T, VE>(xs + v * VE, f);
     one(v, f);
@@ -252,8 +281,8 @@ __global__ void __launch_bounds__(kThreads)
   if (lane == 0) tp[piece] = make_float2(s1, s2);
 }
 
-// backward 2: one CTA per (n, g): channel sums over the pieces (ascending) -> sums[n * C + c], and
-// the gamma-weighted group sums -> coef[(n * G + g) * 2] = A, B
+// backward 2: one CTA per (n, g): channel sums over the pieces (a lane per piece, then the butterfly)
+// -> sums[n * C + c], and the gamma-weighted group sums -> coef[(n * G + g) * 2] = A, B
 template <typename T>
 __global__ void __launch_bounds__(128)
     gn_nchw_finalize_kernel(const float2* __restrict__ tp, const T* __restrict__ gamma, float2* __restrict__ sums,
@@ -262,19 +291,33 @@ __global__ void __launch_bounds__(128)
   grid_dep_launch_dependents();
   grid_dep_wait();  // the reduce kernel's sums
   const int n = blockIdx.x / g.G, grp = blockIdx.x - n * g.G;
-  float w1 = 0.f, w2 = 0.f;
-  for (int cl = threadIdx.x; cl < g.D; cl += 128) {
-    const int c = grp * g.D + cl;
-    const float2* p = tp + ((size_t)n * g.C + c) * g.ppr;
+  // W lanes per channel, W the smallest power of two that covers the pieces (at most a warp)
+  int sh = 0;
+  while ((1 << sh) < g.ppr && sh < 5) ++sh;
+  const int W = 1 << sh, lx = threadIdx.x & (W - 1), per_cta = 128 >> sh;
+  float w1 = 0.f, w2 = 0.f;  // gamma-weighted sums, held by the first lane of every W
+  for (int c0 = 0; c0 < g.D; c0 += per_cta) {
+    const int cl = c0 + ((int)threadIdx.x >> sh), c = grp * g.D + cl;
     float t1 = 0.f, t2 = 0.f;
-    for (int j = 0; j < g.ppr; ++j) {
-      t1 += p[j].x;
-      t2 += p[j].y;
+    if (cl < g.D) {
+      const float2* p = tp + ((size_t)n * g.C + c) * g.ppr;
+#pragma unroll 4
+      for (int j = lx; j < g.ppr; j += W) {
+        const float2 v = p[j];
+        t1 += v.x;
+        t2 += v.y;
+      }
     }
-    sums[(size_t)n * g.C + c] = make_float2(t1, t2);
-    const float ga = load_param<T>(gamma, c);
-    w1 = fmaf(ga, t1, w1);
-    w2 = fmaf(ga, t2, w2);
+    for (int b = W >> 1; b >= 1; b >>= 1) {
+      t1 += __shfl_xor_sync(0xffffffffu, t1, b);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, b);
+    }
+    if (cl < g.D && lx == 0) {
+      sums[(size_t)n * g.C + c] = make_float2(t1, t2);
+      const float ga = load_param<T>(gamma, c);
+      w1 = fmaf(ga, t1, w1);
+      w2 = fmaf(ga, t2, w2);
+    }
   }
   w1 = block_sum(w1, scratch);
   w2 = block_sum(w2, scratch);
@@ -285,15 +328,16 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// backward 4: dx = rstd * (gamma_c * dyh - A - xh * B), one warp per piece as in the reduce kernel
+// backward 4: dx = rstd * (gamma_c * dyh - A - xh * B), one warp per piece as in the reduce kernel, the pieces in
+// reverse order and from their ends (see forward 2)
 template <typename T, int VE, int ACT>
 __global__ void __launch_bounds__(kThreads)
     gn_nchw_dx_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                       const T* __restrict__ beta, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                       const float* __restrict__ coef, T* __restrict__ dx, long long pieces, const NchwGeom g) {
   const int lane = threadIdx.x & 31;
-  const long long piece = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  if (piece >= pieces) return;
+  const long long piece = pieces - 1 - ((long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5));
+  if (piece < 0) return;
   const long long row = piece / g.ppr;
   const int j = (int)(piece - row * g.ppr);
   const int n = (int)(row / g.C), c = (int)(row - (long long)n * g.C);
@@ -320,20 +364,20 @@ __global__ void __launch_bounds__(kThreads)
     act_grad_vec<T, VE, ACT>(yh, gr);
 #pragma unroll
     for (int e = 0; e < VE; ++e) o[e] = fmaf(ag, fd[e] * gr[e], fmaf(nb, xh[e], na));
-    store_vec<T, VE>(os + v * VE, o);
+    store_vec<T, VE>(os + v * VE, o, g.evict);
   };
-  long long v = v0 + lane;
-  for (; v + (kUnroll - 1) * 32 < v1; v += kUnroll * 32) {
+  long long v = v1 - 1 - lane;
+  for (; v - (kUnroll - 1) * 32 >= v0; v -= kUnroll * 32) {
     float fx[kUnroll][VE], fd[kUnroll][VE];
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
-      load_vec<T, VE>(xs + (v + u * 32) * VE, fx[u]);
-      load_vec<T, VE>(ds + (v + u * 32) * VE, fd[u]);
+      load_vec<T, VE>(xs + (v - u * 32) * VE, fx[u]);
+      load_vec<T, VE>(ds + (v - u * 32) * VE, fd[u]);
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) one(v + u * 32, fx[u], fd[u]);
+    for (int u = 0; u < kUnroll; ++u) one(v - u * 32, fx[u], fd[u]);
   }
-  for (; v < v1; v += 32) {
+  for (; v >= v0; v -= 32) {
     float fx[VE], fd[VE];
     load_vec<T, VE>(xs + v * VE, fx);
     load_vec<T, VE>(ds + v * VE, fd);
@@ -363,18 +407,23 @@ NchwGeom make_geom(long long N, long long R, long long C, long long G, int ve) {
   g.slab_vecs = (long long)g.D * R / ve;
   g.row_vecs = R / ve;
   g.div_R = fast_div(R);
-  // forward: about four CTAs per SM, at least 2048 vectors (32 KB) per chunk
+  g.evict = (double)N * C * R * (16 / ve) > 32.0 * 1024 * 1024;  // (single elements are stored plainly)
+  // forward: sixteen chunks per SM, at least 2048 vectors (32 KB) each.  Several waves of CTAs even out the SMs and
+  // let the reverse order of the output pass work across CTAs too: with four chunks per SM (all in flight at once)
+  // 43.6 us at 512@256^2 fp16, 90 us at 2 x 256@256^2 fp32, 114 us at 3 x 128@300x301 bf16; with sixteen 39.0, 77.6, 78.6.
   const long long slabs = N * G;
-  long long chunks = (4LL * kSmCount + slabs - 1) / slabs;
+  long long chunks = (16LL * kSmCount + slabs - 1) / slabs;
   const long long max_chunks = (g.slab_vecs + 2047) / 2048;
   if (chunks > max_chunks) chunks = max_chunks;
   if (chunks < 1) chunks = 1;
   if (chunks > 1024) chunks = 1024;
   g.chunk_vecs = (g.slab_vecs + chunks - 1) / chunks;
   g.chunks = (int)((g.slab_vecs + g.chunk_vecs - 1) / g.chunk_vecs);
-  // backward: one warp per piece of a channel row; about 16 warps per SM, 128 .. 2048 vectors per piece
+  // backward: one warp per piece of a channel row; about 96 warps per SM, 128 .. 2048 vectors per piece, for the same
+  // reason: 512@256^2 fp16 101 us with 16, 78 with 64, 74.7 with 96, 74.9 with 128 (320 CTAs of the first kind lie
+  // three on some SMs and two on the others); 2 x 256@256^2 fp32 119 / 131 / 117.6 / 118.7
   const long long rows = N * C;
-  long long ppr = (16LL * kSmCount + rows - 1) / rows;
+  long long ppr = (96LL * kSmCount + rows - 1) / rows;
   const long long max_ppr = (g.row_vecs + 127) / 128;
   if (ppr > max_ppr) ppr = max_ppr;
   if (ppr < 1) ppr = 1;
