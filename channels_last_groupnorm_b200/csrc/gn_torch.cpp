@@ -15,10 +15,13 @@
 // carry explicit schemas with a CUDA implementation (the reference registers catch-all functions, which
 // cannot be traced).
 #include <ATen/Tensor.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
 #include <vector>
@@ -106,7 +109,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> gnb200_fwd_op(const at::Tensor& X
   }
   const size_t ws_bytes = layout == kNHWC ? gnb200_fwd_workspace_bytes(N, R, C, G, dtype)
                                           : gnb200_fwd_nchw_workspace_bytes(N, R, C, G, dtype);
-  at::Tensor ws = at::empty({(int64_t)ws_bytes}, X.options().dtype(at::kByte));
+  at::Tensor ws;  // most forward plans need no scratch
+  if (ws_bytes) ws = at::empty({(int64_t)ws_bytes}, X.options().dtype(at::kByte));
   auto fn = layout == kNHWC ? &gnb200_fwd : &gnb200_fwd_nchw;
   check_status(fn(X.const_data_ptr(), weight.const_data_ptr(), bias.const_data_ptr(), N, R, C, G, eps, (int)act, dtype,
                   Y.mutable_data_ptr(), means.mutable_data_ptr<float>(), rstds.mutable_data_ptr<float>(),
@@ -135,8 +139,10 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> bwd_impl(const at::Te
   check_stats(rstds, X, dtype, N, G, "rstds");
   c10::cuda::CUDAGuard guard(X.device());
   at::Tensor dX = empty_like_layout(X, layout);
-  at::Tensor dparam = at::empty({2, C}, X.options().dtype(stats_dtype(dtype)));
-  at::Tensor dweight, dbias;
+  // the packed fp32 sums: a result of their own, or - typed gradients - the tail of the scratch allocation
+  const bool packed_in_scratch = want_typed && dtype != kF64 && X.numel() != 0;
+  at::Tensor dparam, dweight, dbias;
+  if (!packed_in_scratch) dparam = at::empty({2, C}, X.options().dtype(stats_dtype(dtype)));
   if (want_typed && dtype != kF64) {
     dweight = at::empty({C}, X.options());
     dbias = at::empty({C}, X.options());
@@ -174,23 +180,25 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> bwd_impl(const at::Te
   }
   const size_t ws_bytes = layout == kNHWC ? gnb200_bwd_workspace_bytes(N, R, C, G, dtype)
                                           : gnb200_bwd_nchw_workspace_bytes(N, R, C, G, dtype);
-  at::Tensor ws = at::empty({(int64_t)ws_bytes}, X.options().dtype(at::kByte));
+  const size_t ws_end = (ws_bytes + 15) & ~(size_t)15;
+  at::Tensor ws = at::empty({(int64_t)(ws_end + (packed_in_scratch ? 2 * C * sizeof(float) : 0))}, X.options().dtype(at::kByte));
+  float* dp32 = packed_in_scratch ? reinterpret_cast<float*>(ws.mutable_data_ptr<uint8_t>() + ws_end) : dparam.mutable_data_ptr<float>();
   void* dw = want_typed ? dweight.mutable_data_ptr() : nullptr;
   void* db = want_typed ? dbias.mutable_data_ptr() : nullptr;
   if (world > 1 && layout == kNHWC) {
     check_status(gnb200_bwd_peer(dy.const_data_ptr(), X.const_data_ptr(), weight.const_data_ptr(), bias.const_data_ptr(),
                                  means.const_data_ptr<float>(), rstds.const_data_ptr<float>(), N, R, C, G, (int)act, dtype,
-                                 dX.mutable_data_ptr(), dparam.mutable_data_ptr<float>(), dw, db,
+                                 dX.mutable_data_ptr(), dp32, dw, db,
                                  ws_bytes ? ws.mutable_data_ptr() : nullptr, ws_bytes, peers.data(), (int)rank, world, stream));
     return {dX, dparam, dweight, dbias};
   }
   auto fn = layout == kNHWC ? &gnb200_bwd : &gnb200_bwd_nchw;
   check_status(fn(dy.const_data_ptr(), X.const_data_ptr(), weight.const_data_ptr(), bias.const_data_ptr(),
                   means.const_data_ptr<float>(), rstds.const_data_ptr<float>(), N, R, C, G, (int)act, dtype,
-                  dX.mutable_data_ptr(), dparam.mutable_data_ptr<float>(), dw, db,
+                  dX.mutable_data_ptr(), dp32, dw, db,
                   ws_bytes ? ws.mutable_data_ptr() : nullptr, ws_bytes, stream));
   if (world > 1)  // channels-first: the exchange follows the backward as a kernel of its own
-    check_status(gnb200_allreduce_param_grads(dparam.mutable_data_ptr<float>(), dw, db, C, dtype, peers.data(), (int)rank,
+    check_status(gnb200_allreduce_param_grads(dp32, dw, db, C, dtype, peers.data(), (int)rank,
                                               world, stream));
   return {dX, dparam, dweight, dbias};
 }
@@ -224,6 +232,94 @@ std::tuple<at::Tensor, at::Tensor> gnb200_bwd_f32_peer_op(const at::Tensor& dy, 
   return {std::get<0>(r), std::get<1>(r)};
 }
 
+// ------------------------------------------------------------------------------------------------
+// group_norm_act: flatten -> fwd -> restore with its autograd node, as one call.  What GN_NHWC_Func
+// (gn_nhwc.py) does in Python, view for view and op for op (the inner ops go through the dispatcher, so dispatch
+// modes see them), without the interpreter: on small maps a training step is bound by that (the Python node
+// alone, with its backward waiting for the interpreter lock in the engine's thread, took most of 150 us).
+// ------------------------------------------------------------------------------------------------
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+// the reference's layout rule (custom_gn.py:68): unit channel stride means channels-last
+bool is_channels_last(const at::Tensor& t) { return t.stride(1) == 1 || t.size(1) == 1; }
+
+at::Tensor flatten(const at::Tensor& t, bool channels_last) {
+  const int64_t n = t.size(0), c = t.size(1), nd = t.dim();
+  if (!channels_last) return t.contiguous().reshape({n, c, -1});
+  at::DimVector dims = {0};
+  for (int64_t d = 2; d < nd; ++d) dims.push_back(d);
+  dims.push_back(1);
+  return t.permute(dims).contiguous().reshape({n, -1, c}).permute({0, 2, 1});
+}
+
+at::Tensor restore(const at::Tensor& flat, at::IntArrayRef shape, bool channels_last) {
+  if (!channels_last) return flat.reshape(shape);
+  at::DimVector sizes = {shape[0]}, dims = {0, (int64_t)shape.size() - 1};
+  for (size_t d = 2; d < shape.size(); ++d) sizes.push_back(shape[d]), dims.push_back((int64_t)d - 1);
+  sizes.push_back(shape[1]);
+  return flat.permute({0, 2, 1}).reshape(sizes).permute(dims);
+}
+
+at::Tensor as_dtype(const at::Tensor& t, at::ScalarType dtype) { return t.scalar_type() == dtype ? t : t.to(dtype); }
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> call_fwd(const at::Tensor& X, const at::Tensor& w, const at::Tensor& b, int64_t G,
+                                                        double eps, int64_t act) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("gnb200::fwd", "").typed<decltype(gnb200_fwd_op)>();
+  at::AutoDispatchBelowADInplaceOrView guard;
+  return op.call(X, w, b, G, eps, act);
+}
+
+struct GnFunction : torch::autograd::Function<GnFunction> {
+  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias,
+                            int64_t G, double eps, int64_t act) {
+    const bool cl = is_channels_last(X);
+    const at::Tensor Xf = flatten(X, cl);
+    const at::Tensor w = as_dtype(weight, X.scalar_type()), b = as_dtype(bias, X.scalar_type());
+    auto [Y, means, rstds] = call_fwd(Xf, w, b, G, eps, act);
+    ctx->save_for_backward({Xf, w, b, means, rstds});
+    ctx->saved_data["shape"] = X.sizes().vec();
+    ctx->saved_data["arg"] = std::vector<int64_t>{G, act, cl ? 1 : 0, (int64_t)weight.scalar_type(), (int64_t)bias.scalar_type()};
+    return restore(Y, X.sizes(), cl);
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("gnb200::bwd", "").typed<decltype(gnb200_bwd_op)>();
+    static const auto op32 =
+        c10::Dispatcher::singleton().findSchemaOrThrow("gnb200::bwd_f32", "").typed<decltype(gnb200_bwd_f32_op)>();
+    const auto saved = ctx->get_saved_variables();
+    const auto shape = ctx->saved_data["shape"].toIntVector(), arg = ctx->saved_data["arg"].toIntVector();
+    const at::Tensor& Xf = saved[0];
+    const at::ScalarType dtype = Xf.scalar_type();
+    const auto w_dtype = (at::ScalarType)arg[3], b_dtype = (at::ScalarType)arg[4];
+    const at::Tensor dy = as_dtype(flatten(grads[0], arg[2] != 0), dtype);
+    at::Tensor dx, dgamma, dbeta;
+    if (w_dtype == dtype && b_dtype == dtype) {
+      std::tie(dx, dgamma, dbeta) = op.call(dy, Xf, saved[1], saved[2], saved[3], saved[4], arg[0], arg[1]);
+    } else {
+      at::Tensor dparam;
+      std::tie(dx, dparam) = op32.call(dy, Xf, saved[1], saved[2], saved[3], saved[4], arg[0], arg[1]);
+      dgamma = dparam.select(0, 0).to(w_dtype);
+      dbeta = dparam.select(0, 1).to(b_dtype);
+    }
+    return {restore(dx, shape, arg[2] != 0), dgamma, dbeta, at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+};
+
+at::Tensor group_norm_act_autograd(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
+                                   int64_t act) {
+  return GnFunction::apply(X, weight, bias, G, eps, act);
+}
+
+// below autograd (inference mode)
+at::Tensor group_norm_act_plain(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
+                                int64_t act) {
+  const bool cl = is_channels_last(X);
+  const at::Tensor Y = std::get<0>(call_fwd(flatten(X, cl), as_dtype(weight, X.scalar_type()), as_dtype(bias, X.scalar_type()), G,
+                                            eps, act));
+  return restore(Y, X.sizes(), cl);
+}
+
 }  // namespace
 
 // Schemas are declared apart from the implementations so that Python can attach fake-tensor
@@ -238,13 +334,17 @@ TORCH_LIBRARY(gnb200, m) {
         "(Tensor, Tensor)");
   m.def("bwd_f32_peer(Tensor dy, Tensor X, Tensor weight, Tensor bias, Tensor means, Tensor rstds, int G, int act, "
         "int[] peer_ptrs, int rank) -> (Tensor, Tensor)");
+  m.def("group_norm_act(Tensor X, Tensor weight, Tensor bias, int G, float eps, int act) -> Tensor");
 }
+
+TORCH_LIBRARY_IMPL(gnb200, Autograd, m) { m.impl("group_norm_act", &group_norm_act_autograd); }
 
 TORCH_LIBRARY_IMPL(gnb200, CUDA, m) {
   m.impl("fwd", &gnb200_fwd_op);
   m.impl("bwd", &gnb200_bwd_op);
   m.impl("bwd_f32", &gnb200_bwd_f32_op);
   m.impl("bwd_f32_peer", &gnb200_bwd_f32_peer_op);
+  m.impl("group_norm_act", &group_norm_act_plain);
 }
 
 TORCH_LIBRARY_IMPL(gnb200, CPU, m) {

@@ -132,6 +132,21 @@ def _restore_shape(flat: torch.Tensor, shape, channels_last=True) -> torch.Tenso
     return nhwc.permute(0, nhwc.ndim - 1, *range(1, nhwc.ndim - 1))
 
 
+_group_norm_act = torch.ops.gnb200.group_norm_act.default
+_PLAIN = (torch.Tensor, nn.Parameter)
+
+
+def _plain_eager(*tensors) -> bool:
+    """True for ordinary tensors outside of tracing, `torch.func` transforms and forward-mode autograd: there the
+    native node of `group_norm_act` does what GN_NHWC_Func does.  Everything else (torch.compile, export, jit.trace,
+    vmap / grad transforms, dual tensors, tensor subclasses) takes the Python function as before."""
+    return (not torch.compiler.is_compiling()
+            and all(type(t) in _PLAIN for t in tensors)
+            and not torch._C._are_functorch_transforms_active()
+            and torch._C._get_tracing_state() is None
+            and torch.autograd.forward_ad._current_level < 0)
+
+
 class GN_NHWC(nn.GroupNorm):
     """`nn.GroupNorm` with a fused activation for channels-last inputs.
 
@@ -159,6 +174,8 @@ class GN_NHWC(nn.GroupNorm):
         else:
             w = torch.ones((self.num_channels,), device=x.device, dtype=x.dtype)
             b = torch.zeros((self.num_channels,), device=x.device, dtype=x.dtype)
+        if self.process_group is None and _plain_eager(x, w, b):
+            return _group_norm_act(x, w, b, self.num_groups, self.eps, self.act_code)
         return GN_NHWC_Func.apply(x, w, b, self.num_groups, self.eps, self.act_code, self.process_group)
 
     def extra_repr(self):
