@@ -690,11 +690,12 @@ struct WaveGeom {
 // contiguous row ranges, and a CTA streams its range - whole rows, hence one contiguous run of memory - in
 // tiles of BR rows through a ring of `stages` shared-memory stages.
 constexpr int kResidentThreads = 512;
-constexpr int kResidentRows = 2;  // rows per thread and tile
+// rows per thread and tile: 32 KB of x, or 16 KB each of x and dy
+__host__ __device__ constexpr int resident_rows(int direction) { return direction == 0 ? 4 : 2; }
 struct ResidentGeom {
   Geom g;              // CW = C, ncb = 1, slots = G; rows_per_cta, chunks = cps
   int cps;             // CTAs per sample
-  int BR;              // rows per tile (kResidentRows * TY)
+  int BR;              // rows per tile (resident_rows * TY)
   int tile_bytes;      // BR * C * sizeof(T), one tensor
   int stages;
   int threads;

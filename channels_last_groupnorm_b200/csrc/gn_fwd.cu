@@ -288,55 +288,6 @@ __device__ __forceinline__ void stream_apply(const Pack<T, VE>* __restrict__ src
   }
 }
 
-// CTA-local moments of every group slot of the column block from the per-thread Welford states:
-// first the slot means (sum of cnt * mean / n), then the squared deviations around them.
-//   slot[s]            = local mean      slot[slots + s] = local M2      slot[2 * slots + s] = local count
-// scratch: red (TY * CW floats), tmp (slots floats).
-template <int VE, bool UNI>
-__device__ __forceinline__ void cta_slot_moments(const Geom& g, const float (&mean)[VE], const float (&m2)[VE],
-                                                 float cnt, int tx, int ty, int c0, int nrows, int g_lo, int n_slots,
-                                                 float* red, float* tmp, float* slot) {
-  constexpr int NV = UNI ? 1 : VE;
-  float val[NV];
-  if constexpr (UNI) {
-    float sm = 0.f;
-#pragma unroll
-    for (int e = 0; e < VE; ++e) sm += mean[e];
-    val[0] = cnt * sm;
-  } else {
-#pragma unroll
-    for (int e = 0; e < VE; ++e) val[e] = cnt * mean[e];
-  }
-  cta_group_sum<VE, NV>(g, val, tx, ty, c0, g_lo, n_slots, red, tmp);
-  const int c_end = min(c0 + g.CW, g.C);
-  for (int s = threadIdx.x; s < n_slots; s += blockDim.x) {
-    const int w = min((g_lo + s + 1) * g.D, c_end) - max((g_lo + s) * g.D, c0);
-    const float n_loc = (float)nrows * (float)w;
-    slot[s] = n_loc > 0.f ? tmp[s] / n_loc : 0.f;
-    slot[2 * g.slots + s] = n_loc;
-  }
-  __syncthreads();
-  if constexpr (UNI) {
-    const float lm = slot[g.div_D.div(min(c0 + tx * VE, g.C - 1)) - g_lo];
-    float acc = 0.f, dev = 0.f;
-#pragma unroll
-    for (int e = 0; e < VE; ++e) {
-      const float d = mean[e] - lm;
-      dev = fmaf(d, d, dev);
-      acc += m2[e];
-    }
-    val[0] = fmaf(cnt, dev, acc);
-  } else {
-#pragma unroll
-    for (int e = 0; e < VE; ++e) {
-      const int c = min(c0 + tx * VE + e, g.C - 1);
-      const float d = mean[e] - slot[g.div_D.div(c) - g_lo];
-      val[e] = fmaf(cnt * d, d, m2[e]);
-    }
-  }
-  cta_group_sum<VE, NV>(g, val, tx, ty, c0, g_lo, n_slots, red, slot + g.slots);
-}
-
 // ------------------------------------------------------------------------------------------------
 // fused one-pass kernel.  cluster = (k,1,1); an item is one (sample, column block) slab and each
 // CTA of the cluster owns rows_per_cta of its rows.  The grid holds the clusters that are resident
@@ -732,6 +683,10 @@ static cudaError_t launch_fwd_ve(const FwdCall& c, const Plan& p, cudaStream_t s
 }
 
 cudaError_t launch_forward(const FwdCall& c, const Plan& p, cudaStream_t stream) {
+  if (p.resident) {
+    const cudaError_t err = launch_forward_resident(c, p.rgeom, stream);
+    if (err != cudaErrorCooperativeLaunchTooLarge) return err;
+  }
   if (p.wave) return launch_forward_wave(c, p, stream);
   switch (c.dtype) {
     case 0: return launch_fwd_ve<float>(c, p, stream);

@@ -21,7 +21,7 @@ struct Plan {
   bool chain;         // kernels after the first are launched as programmatic dependents of their predecessor
   Geom geom;
   WaveGeom wgeom;
-  // Backward: the resident kernel (gn_resident.cu) takes the place of the multi-kernel or wave plan described by the
+  // The resident kernel (gn_resident.cu) takes the place of the multi-kernel or wave plan described by the
   // fields above, which stay filled in: they are what runs where the grid cannot be resident at once.
   bool resident;
   ResidentGeom rgeom;
@@ -92,9 +92,10 @@ cudaError_t launch_forward_wave(const FwdCall& c, const Plan& p, cudaStream_t st
 cudaError_t launch_backward_wave(const BwdCall& c, const Plan& p, cudaStream_t stream);
 // resident plan (gn_resident.cu).  cudaErrorCooperativeLaunchTooLarge: nothing was launched, the device (or the
 // share of it that this process has) cannot hold the grid
+cudaError_t launch_forward_resident(const FwdCall& c, const ResidentGeom& r, cudaStream_t stream);
 cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream);
-size_t resident_workspace_bytes(const ResidentGeom& r);
-size_t resident_fixed_smem(const ResidentGeom& r);  // shared memory besides the stages
+size_t resident_workspace_bytes(const ResidentGeom& r, int direction);
+size_t resident_fixed_smem(const ResidentGeom& r, int direction);  // shared memory besides the stages
 // cudaSuccess if `grid` CTAs of this kernel can be resident at once on the current device
 cudaError_t check_resident(const void* func, int threads, size_t smem, long long grid);
 // dgamma / dbeta from `rows` rows of per-channel (S1, S2) pairs (gn_bwd.cu)

@@ -111,6 +111,55 @@ __device__ __forceinline__ void lane_affine_raw(const uint4& ga_raw, const uint4
   }
 }
 
+// CTA-local moments of every group slot of the column block from the per-thread Welford states:
+// first the slot means (sum of cnt * mean / n), then the squared deviations around them.
+//   slot[s]            = local mean      slot[slots + s] = local M2      slot[2 * slots + s] = local count
+// scratch: red (TY * CW floats), tmp (slots floats).
+template <int VE, bool UNI>
+__device__ __forceinline__ void cta_slot_moments(const Geom& g, const float (&mean)[VE], const float (&m2)[VE],
+                                                 float cnt, int tx, int ty, int c0, int nrows, int g_lo, int n_slots,
+                                                 float* red, float* tmp, float* slot) {
+  constexpr int NV = UNI ? 1 : VE;
+  float val[NV];
+  if constexpr (UNI) {
+    float sm = 0.f;
+#pragma unroll
+    for (int e = 0; e < VE; ++e) sm += mean[e];
+    val[0] = cnt * sm;
+  } else {
+#pragma unroll
+    for (int e = 0; e < VE; ++e) val[e] = cnt * mean[e];
+  }
+  cta_group_sum<VE, NV>(g, val, tx, ty, c0, g_lo, n_slots, red, tmp);
+  const int c_end = min(c0 + g.CW, g.C);
+  for (int s = threadIdx.x; s < n_slots; s += blockDim.x) {
+    const int w = min((g_lo + s + 1) * g.D, c_end) - max((g_lo + s) * g.D, c0);
+    const float n_loc = (float)nrows * (float)w;
+    slot[s] = n_loc > 0.f ? tmp[s] / n_loc : 0.f;
+    slot[2 * g.slots + s] = n_loc;
+  }
+  __syncthreads();
+  if constexpr (UNI) {
+    const float lm = slot[g.div_D.div(min(c0 + tx * VE, g.C - 1)) - g_lo];
+    float acc = 0.f, dev = 0.f;
+#pragma unroll
+    for (int e = 0; e < VE; ++e) {
+      const float d = mean[e] - lm;
+      dev = fmaf(d, d, dev);
+      acc += m2[e];
+    }
+    val[0] = fmaf(cnt, dev, acc);
+  } else {
+#pragma unroll
+    for (int e = 0; e < VE; ++e) {
+      const int c = min(c0 + tx * VE + e, g.C - 1);
+      const float d = mean[e] - slot[g.div_D.div(c) - g_lo];
+      val[e] = fmaf(cnt * d, d, m2[e]);
+    }
+  }
+  cta_group_sum<VE, NV>(g, val, tx, ty, c0, g_lo, n_slots, red, slot + g.slots);
+}
+
 template <typename T, int VE>
 struct BwdLane {
   float r[VE];    // rstd of the lane's group

@@ -445,22 +445,32 @@ bool plan_wave(const Shape& sh, Plan* out) {
   return true;
 }
 
-// Resident plan (gn_resident.cu), backward, in place of the multi-kernel or wave plan in *plan.  A sample's rows are
-// cut into cps = 148 / N contiguous ranges, one CTA per SM; at least 85 % of the SMs must get one.  Tiles hold two rows
-// per thread (16 KB each of x and dy); what is left of the SM's shared memory holds as many of them as fit.
-// The line: measured on B200, us, resident / the plan it replaces (w wave, m multi-kernel):
+// Resident plan (gn_resident.cu) in place of the multi-kernel or wave plan in *plan.  A sample's rows are cut into
+// cps = 148 / N contiguous ranges, one CTA per SM; at least 85 % of the SMs must get one.  Tiles are 32 KB of x
+// (backward: 16 KB each of x and dy); what is left of the SM's shared memory holds as many of them as fit.
+// The lines: measured on B200, us, resident / the plan it replaces (w wave, m multi-kernel).
+// Backward:
 //   fp16  512@256^2 64.2 / 68.7 w    256@512^2 118 / 129 w    128@1024^2 226 / 242 m    2 x 256@512x256 117 / 125 w
 //   bf16  3 x 512@200x300 158 / 167 w    20 x 96@320x90, 3 groups 107 / 145 w
 //   bf16, one group per sample  8 x 1024@64^2 72 / 140 m    1 x 512@64^2 16.5 / 100 m (one CTA of that plan's finalize
 //         kernel adds up all channels of a group)    fp32  8 x 512@64^2 79 / 115 m
 //   fp32  256@512^2, 32 groups 258 / 249 w: with fp32 arithmetic both passes are bound by instruction issue, where
 //         sixteen warps per SM do worse - so fp32 takes it only for wide groups.
+// Forward, against the three chained kernels, whose arithmetic is short and which have half as much to keep - so only
+// one large 16-bit sample of eight groups or more takes it:
+//   fp16  512@256^2 39.2 / 39.9    256@512^2 73.9 / 74.6    128@1024^2 145 / 148    512@450^2 112 / 113
+//   bf16  128@300x1000 45.4 / 48.5    and as calls among others 73.2 / 76.2 (256@512^2, with allocation)
+//   not there: 2 x 256@512x256 74.2 / 73.7    3 x 512@200x300 101 / 98    fp32 256@512^2 152 / 150
+//              one group: 8 x 1024@64^2 43 / 37    4 MB, one group 16.5 / 8.8
 // GNB200_RESIDENT_CTAS / _STAGES (tests, experiments) bound the CTAs per sample and the stages.
 bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   const int ve = sh.ve, s = sh.s;
-  if (sh.direction != 1 || ve == 1 || sh.N > kSmCount) return false;
+  if (ve == 1 || sh.N > kSmCount) return false;
   if (sh.G > 128) return false;  // every CTA merges cps * G partials
-  if (!forced && s == 4 && sh.D < 128) return false;
+  if (!forced && sh.direction == 1 && s == 4 && sh.D < 128) return false;
+  if (!forced && sh.direction == 0 &&
+      (s == 4 || sh.G < 8 || sh.N > 1 || (double)sh.R * sh.C * s < 48.0 * 1024 * 1024))
+    return false;
   const int CV = sh.C / ve;
   if (CV > kResidentThreads) return false;
   ResidentGeom r = {};
@@ -485,11 +495,11 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   g.div_chunks = make_fast_div(cps);
   r.g = g;
   r.cps = cps;
-  r.BR = kResidentRows * g.TY;
+  r.BR = resident_rows(sh.direction) * g.TY;
   r.tile_bytes = r.BR * sh.C * s;
   r.threads = round_up(CV * g.TY, 32);
   r.grid = (long long)sh.N * cps;
-  const size_t fixed = resident_fixed_smem(r), stage = (size_t)2 * r.tile_bytes;
+  const size_t fixed = resident_fixed_smem(r, sh.direction), stage = (size_t)(sh.direction == 0 ? 1 : 2) * r.tile_bytes;
   const size_t room = kSmemMaxOptin - 1024;
   if (fixed + 2 * stage > room) return false;
   r.stages = (int)((room - fixed) / stage);
@@ -497,7 +507,7 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   if (r.stages > max_stages) r.stages = max_stages < 2 ? 2 : max_stages;
   if (r.stages > 16) r.stages = 16;
   r.smem_bytes = fixed + (size_t)r.stages * stage;
-  r.ws_bytes = resident_workspace_bytes(r);
+  r.ws_bytes = resident_workspace_bytes(r, sh.direction);
   // The scratch limits of callers stay what they are: a call never asks for less than the plan that this one
   // replaces, nor - beyond the 4 MiB that every backward call may rely on - for more.
   const size_t static_limit = 4u << 20;

@@ -1,25 +1,23 @@
-// "Resident" launch plan for slabs that do not fit a thread-block cluster: backward GroupNorm (+activation) for
-// NHWC tensors as ONE persistent cooperative kernel, one CTA per SM, sm_100a.
+// "Resident" launch plan for slabs that do not fit a thread-block cluster: forward and backward GroupNorm (+activation)
+// for NHWC tensors as ONE persistent cooperative kernel each, one CTA per SM, sm_100a.
 //
-// The sums of dyh and dyh * xh need every row of a sample before the first dx can be written, so these shapes take
-// two passes over x and dy.  What bounds them is HBM: how much of the second pass is read from there again, and what
-// lies between the passes.  Here a CTA owns one contiguous range of a sample's rows for both passes:
+// The statistics (backward: the sums of dyh and dyh * xh) need every row of a sample before the first result can be
+// written, so these shapes take two passes over their rows.  What bounds them is HBM: how much of the second pass is
+// read from there again, and what lies between the passes.  Here a CTA owns one contiguous range of a sample's rows:
 //
 //   pass 1   the range streams through a ring of shared-memory stages (untiled cp.async.bulk copies: whole rows are
 //            one contiguous run, so no thread computes an address and no tensor map is needed); the last `stages`
 //            tiles are not overwritten: 148 x 192 KB, 28 MB, stay on chip
 //   barrier  partial sums to scratch, one arrival per CTA, bounded wait; every CTA merges what it needs
 //   pass 2   the resident tiles first - no read at all - and, as their stages become free, the tiles before them
-//            in reverse order, so that what was read last (and L2 still holds) is read first; dx leaves with
+//            in reverse order, so that what was read last (and L2 still holds) is read first; results leave with
 //            streaming (evict-first) stores
 //
-// dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.  The same kernel for the
-// forward direction gained less over the three chained kernels than it lost on small slabs (fp16, us: 67 MB 39.2 / 39.8,
-// 134 MB 73.6 / 74.8, 4 MB 16.5 / 8.8) and was left out: its arithmetic is short and there is half as much to keep.
-// Measured against the plan it replaces: see the rule in gn_plan.cu.
+// dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.
+// Measured against the plans it replaces: see the rule in gn_plan.cu.
 //
 // Every sum is formed in an order fixed by the launch geometry: bit-identical reruns.
-// The passes restate what src/gnnhwc/csrc/gn_kernel.cu:533-872 of the reference computes.
+// The passes restate what src/gnnhwc/csrc/gn_kernel.cu:132-412 and 533-872 of the reference compute.
 #include "gn_async.cuh"
 #include "gn_kernels.h"
 #include "gn_math.cuh"
@@ -38,7 +36,7 @@ __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, ui
                : "memory");
 }
 
-// Shared memory: [stages * (x tile, dy tile)][full][empty][flags][reduction scratch]
+// Shared memory: [stages * NT tiles][full][empty][flags][reduction scratch]; NT tensors: x, or x and dy
 struct Smem {
   uint32_t stage0;
   uint64_t* full;
@@ -46,10 +44,11 @@ struct Smem {
   int* flags;  // [0] a wait gave up
   float* red;
 };
+template <int NT>
 __device__ __forceinline__ Smem carve(const ResidentGeom& r, unsigned char* base) {
   Smem s;
   s.stage0 = smem_addr(base);
-  unsigned char* p = base + (size_t)r.stages * 2 * r.tile_bytes;  // tile_bytes is a multiple of 16
+  unsigned char* p = base + (size_t)r.stages * NT * r.tile_bytes;  // tile_bytes is a multiple of 16
   s.full = reinterpret_cast<uint64_t*>(p);
   s.empty = s.full + kMaxStages;
   s.flags = reinterpret_cast<int*>(s.empty + kMaxStages);
@@ -60,9 +59,9 @@ constexpr size_t kControlBytes = 2 * kMaxStages * 8 + 16;
 
 // The stage sequence of both passes, as thread 0 (which issues the copies) and all threads walk it.  Tile t
 // lives in stage t % stages in both passes; the parity of a barrier's current phase is one bit per stage.
-template <typename T>
+template <typename T, int NT>
 struct Stream {
-  const T* src[2];  // x, dy: first element of the CTA's row range
+  const T* src[NT];  // x (and dy): first element of the CTA's row range
   int tiles, nrows, BR, stages;
   uint32_t row_bytes, tile_bytes;
   unsigned full_ph, empty_ph;
@@ -70,10 +69,10 @@ struct Stream {
 
   __device__ __forceinline__ void issue(int t, int stage) {  // thread 0
     const uint32_t bytes = (uint32_t)min(BR, nrows - t * BR) * row_bytes;
-    mbar_arrive_expect_tx(&sm.full[stage], 2 * bytes);
+    mbar_arrive_expect_tx(&sm.full[stage], NT * bytes);
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-      bulk_load(sm.stage0 + (uint32_t)(stage * 2 + i) * tile_bytes,
+    for (int i = 0; i < NT; ++i)
+      bulk_load(sm.stage0 + (uint32_t)(stage * NT + i) * tile_bytes,
                 reinterpret_cast<const char*>(src[i]) + (size_t)t * tile_bytes, bytes, &sm.full[stage]);
   }
   // thread 0: waits until every warp has handed the stage back, then refills it.  Without the hand-back
@@ -89,8 +88,8 @@ struct Stream {
   }
 };
 
-template <typename T>
-__device__ __forceinline__ void stream_start(Stream<T>& st, const ResidentGeom& r, const Smem& sm, int nrows) {
+template <typename T, int NT>
+__device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGeom& r, const Smem& sm, int nrows) {
   st.sm = sm;
   st.nrows = nrows;
   st.BR = r.BR;
@@ -137,8 +136,12 @@ __device__ __forceinline__ void grid_barrier(unsigned int* count, int* flags, co
 // acc[w * G + s], acc[(nwarps + w) * G + s] receive the warp's two sums of group s, formed in row order.  All CTAs of
 // a sample read the same rows at the same moment, so what counts is the number of L2 requests: with one warp per
 // group and a lane per row (32 requests of 8 or 16 bytes per load) a merge of 32 groups x 148 rows took 8.1 us.
-__device__ __forceinline__ void merge_rows(const float2* p, int rows, int G, int warp, int nwarps, int lane, float* acc) {
+// add(i, pair, K0, sum1, sum2) takes one pair of row i; K0 is the first value of the group's row 0.
+template <typename Add>
+__device__ __forceinline__ void merge_rows(const float2* p, int rows, int G, int warp, int nwarps, int lane, float* acc,
+                                           Add add) {
   for (int s = lane; s < G; s += 32) {
+    const float K0 = __ldcg(p + s).x;
     float a1 = 0.f, a2 = 0.f;
     for (int i0 = warp; i0 < rows; i0 += nwarps * kMergeRows) {
       float2 v[kMergeRows];
@@ -148,7 +151,8 @@ __device__ __forceinline__ void merge_rows(const float2* p, int rows, int G, int
         v[q] = i < rows ? __ldcg(p + (size_t)i * G + s) : make_float2(0.f, 0.f);
       }
 #pragma unroll
-      for (int q = 0; q < kMergeRows; ++q) a1 += v[q].x, a2 += v[q].y;
+      for (int q = 0; q < kMergeRows; ++q)
+        if (i0 + nwarps * q < rows) add(i0 + nwarps * q, v[q], K0, a1, a2);
     }
     acc[warp * G + s] = a1;
     acc[(nwarps + warp) * G + s] = a2;
@@ -156,7 +160,160 @@ __device__ __forceinline__ void merge_rows(const float2* p, int rows, int G, int
 }
 
 // ------------------------------------------------------------------------------------------------
-// scratch: tpart[cta * C + c] = (S1, S2) of channel c over the CTA's rows,
+// forward.  scratch: part[cta * G + s] = (mean, M2) of group s over the CTA's rows
+// ------------------------------------------------------------------------------------------------
+template <typename T, int ACT, bool UNI>
+__global__ void __launch_bounds__(kResidentThreads, 1)
+    gn_fwd_resident_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
+                           float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, float2* part,
+                           unsigned int* count, const ResidentGeom r) {
+  constexpr int VE = 16 / sizeof(T);
+  constexpr int KR = resident_rows(0);
+  constexpr bool kShifted = sizeof(T) == 2;  // 16-bit tensors: shifted sums about the thread's first row
+  constexpr int KN = UNI ? 1 : VE;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const Geom& g = r.g;
+  const Smem sm = carve<1>(r, smem_raw);
+  float* red = sm.red;
+  float* tmp = red + g.red_floats;
+  float* slot = tmp + g.slots;
+  float* stat = slot + 3 * g.slots;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
+  const int n = g.div_chunks.div((int)blockIdx.x), j = (int)blockIdx.x - n * r.cps;
+  const int r0 = j * g.rows_per_cta;
+  const int nrows = min(g.rows_per_cta, g.R - r0);
+  const int ty = g.div_CV.div(tid), tx = tid - ty * g.CV;
+  const bool streaming = ty < g.TY;
+  const size_t row0 = (size_t)n * g.R + r0;
+
+  Stream<T, 1> st;
+  st.src[0] = x + row0 * g.C;
+  stream_start(st, r, sm, nrows);
+  const int T_ = st.tiles, S = st.stages;
+  const uint32_t my_off = sm.stage0 + (streaming ? (uint32_t)(ty * g.CV + tx) * 16u : 0u);
+  const uint32_t step = (uint32_t)(g.TY * g.CV) * 16u;
+  const int my_row = streaming ? ty : 0x40000000;  // no row of a tile for idle threads
+
+  // ---- pass 1: moments of the thread's rows
+  float mean[VE], m2[VE], K[KN], cnt = 0.f;
+#pragma unroll
+  for (int e = 0; e < VE; ++e) mean[e] = 0.f, m2[e] = 0.f;
+#pragma unroll
+  for (int e = 0; e < KN; ++e) K[e] = 0.f;
+  int stage = 0, prev = 0;
+  for (int t = 0; t < T_; ++t) {
+    st.wait_full(stage, g.wait);
+    const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
+    const int here = nrows - t * st.BR;
+    uint4 w[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
+    if constexpr (kShifted) {
+      if (t == 0) {  // the shift: the values of the thread's first row
+        float f0[VE];
+        unpack16<T, VE>(w[0], f0);
+        if (my_row < here) {
+#pragma unroll
+          for (int e = 0; e < KN; ++e) K[e] = f0[e];
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      if (my_row + u * g.TY < here) {
+        if constexpr (kShifted) {
+          shifted_step<T, VE, KN>(w[u], K, mean, m2);
+        } else {
+          float f[VE];
+          unpack16<T, VE>(w[u], f);
+          welford_step<VE>(f, mean, m2, cnt);
+        }
+      }
+    }
+    pin_regs(mean);
+    pin_regs(m2);
+    if (t + S < T_) release_stage(&sm.empty[stage], lane);
+    if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
+    prev = stage;
+    if (++stage == S) stage = 0;
+  }
+  if constexpr (kShifted) {
+    const int own = my_row < nrows ? (nrows - my_row + g.TY - 1) / g.TY : 0;
+    shifted_finish<VE, KN>(K, own, mean, m2, cnt);
+  }
+  __syncwarp();
+  __syncthreads();
+  cta_slot_moments<VE, UNI>(g, mean, m2, cnt, tx, ty, 0, nrows, 0, g.G, red, tmp, slot);
+  for (int s = tid; s < g.G; s += blockDim.x)
+    part[(size_t)blockIdx.x * g.G + s] = make_float2(slot[s], slot[g.slots + s]);
+  grid_barrier(count, sm.flags, g.wait);
+
+  // ---- statistics of the sample: sums about the first CTA's mean, the counts known from the geometry
+  const bool ok = *(volatile int*)&sm.flags[0] == 0;
+  {
+    const float2* p = part + (size_t)n * r.cps * g.G;
+    float* acc = red;  // [2][nwarps][G]
+    merge_rows(p, r.cps, g.G, warp, nwarps, lane, acc, [&](int i, float2 v, float K0, float& a1, float& a2) {
+      const float cnt_i = (float)min(g.rows_per_cta, g.R - i * g.rows_per_cta) * (float)g.D, d = v.x - K0;
+      a1 = fmaf(cnt_i, d, a1);
+      a2 += fmaf(cnt_i * d, d, v.y);
+    });
+    __syncthreads();
+    for (int s = tid; s < g.G; s += blockDim.x) {
+      float ad = 0.f, aq = 0.f;
+      for (int w = 0; w < nwarps; ++w) {
+        ad += acc[w * g.G + s];
+        aq += acc[(nwarps + w) * g.G + s];
+      }
+      const float an = (float)g.R * (float)g.D, K0 = __ldcg(p + s).x, dm = ad / an;
+      const float mu = ok ? K0 + dm : kNaN;
+      const float rs = ok ? rsqrtf(fmaxf(fmaf(-ad, dm, aq) / an, 0.f) + eps) : kNaN;
+      stat[s] = mu;
+      stat[g.slots + s] = rs;
+      if (j == 0) {
+        mean_out[(size_t)n * g.G + s] = mu;
+        rstd_out[(size_t)n * g.G + s] = rs;
+      }
+    }
+  }
+  __syncthreads();
+
+  // ---- pass 2: y = act(x * a + b), the resident tiles first
+  float a[VE], b[VE];
+#pragma unroll
+  for (int e = 0; e < VE; ++e) a[e] = b[e] = 0.f;
+  if (streaming) lane_affine<T, VE, UNI>(gamma, beta, stat, stat + g.slots, 0, tx * VE, g.div_D, a, b);
+  T* out = y + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
+  const size_t ostep = (size_t)g.TY * g.C;
+  stage = prev;  // of the last tile
+  for (int t = T_ - 1; t >= 0; --t) {
+    if (t < T_ - S) st.wait_full(stage, g.wait);
+    const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
+    const int here = nrows - t * st.BR;
+    T* o = out + (size_t)t * st.BR * g.C;
+    uint4 w[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      if (my_row + u * g.TY < here) {
+        float f[VE];
+        unpack16<T, VE>(w[u], f);
+#pragma unroll
+        for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+        stg128_stream(o + (size_t)u * ostep, act_pack16<T, VE, ACT>(f));
+      }
+    }
+    if (t >= S) release_stage(&sm.empty[stage], lane);
+    if (tid == 0 && t + 1 < T_ && t + 1 >= S) st.refill(t + 1 - S, prev, g.wait);
+    prev = stage;
+    stage = stage == 0 ? S - 1 : stage - 1;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// backward.  scratch: tpart[cta * C + c] = (S1, S2) of channel c over the CTA's rows,
 //          gpart[cta * G + s] = gamma-weighted sums of group s over the CTA's rows.
 // ------------------------------------------------------------------------------------------------
 template <typename T, int ACT, bool UNI>
@@ -167,11 +324,11 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
                            float* __restrict__ dparam_f32, T* __restrict__ dgamma, T* __restrict__ dbeta,
                            const ResidentGeom r) {
   constexpr int VE = 16 / sizeof(T);
-  constexpr int KR = kResidentRows;
+  constexpr int KR = resident_rows(1);
   constexpr bool kRaw = sizeof(T) == 2;  // 16-bit tensors: packed arithmetic, S2 against the raw x
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const Geom& g = r.g;
-  const Smem sm = carve(r, smem_raw);
+  const Smem sm = carve<2>(r, smem_raw);
   float* red = sm.red;              // TY * C
   float* chan = red + g.red_floats;  // S1[C], S2[C]
   float* coef = chan + 2 * g.C;      // A[G], B[G]
@@ -184,7 +341,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   const bool streaming = ty < g.TY;
   const size_t row0 = (size_t)n * g.R + r0;
 
-  Stream<T> st;
+  Stream<T, 2> st;
   st.src[0] = x + row0 * g.C;
   st.src[1] = dy + row0 * g.C;
   stream_start(st, r, sm, nrows);
@@ -285,7 +442,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   const float inv_m = ok ? 1.0f / ((float)g.D * (float)g.R) : kNaN;
   {
     float* acc = red;  // [2][nwarps][G]
-    merge_rows(gpart + (size_t)n * r.cps * g.G, r.cps, g.G, warp, nwarps, lane, acc);
+    merge_rows(gpart + (size_t)n * r.cps * g.G, r.cps, g.G, warp, nwarps, lane, acc,
+               [](int, float2 v, float, float& a1, float& a2) { a1 += v.x, a2 += v.y; });
     __syncthreads();
     for (int s = tid; s < g.G; s += blockDim.x) {
       float w1 = 0.f, w2 = 0.f;
@@ -384,12 +542,12 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
 // host side
 // ------------------------------------------------------------------------------------------------
 struct Scratch {
-  size_t gpart, count, total;  // channel sums first
+  size_t pairs, count, total;  // backward: channel sums first
 };
-Scratch scratch_of(const ResidentGeom& r) {
+Scratch scratch_of(const ResidentGeom& r, int direction) {
   Scratch s;
-  s.gpart = (size_t)r.grid * r.g.C * sizeof(float2);
-  s.count = s.gpart + (size_t)r.grid * r.g.G * sizeof(float2);
+  s.pairs = direction == 0 ? 0 : (size_t)r.grid * r.g.C * sizeof(float2);
+  s.count = s.pairs + (size_t)r.grid * r.g.G * sizeof(float2);
   s.total = (s.count + 4 + 15) & ~(size_t)15;
   return s;
 }
@@ -416,21 +574,29 @@ cudaError_t launch(Kern kern, const ResidentGeom& r, unsigned int* count, cudaSt
 }
 
 template <typename T, int ACT, bool UNI>
+cudaError_t launch_u(const FwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+  const Scratch s = scratch_of(r, 0);
+  char* ws = static_cast<char*>(c.workspace);
+  unsigned int* count = reinterpret_cast<unsigned int*>(ws + s.count);
+  return launch(gn_fwd_resident_kernel<T, ACT, UNI>, r, count, stream, (const T*)c.x, (const T*)c.gamma, (const T*)c.beta,
+                (T*)c.y, c.mean, c.rstd, c.eps, reinterpret_cast<float2*>(ws + s.pairs), count, r);
+}
+template <typename T, int ACT, bool UNI>
 cudaError_t launch_u(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
-  const Scratch s = scratch_of(r);
+  const Scratch s = scratch_of(r, 1);
   char* ws = static_cast<char*>(c.workspace);
   unsigned int* count = reinterpret_cast<unsigned int*>(ws + s.count);
   return launch(gn_bwd_resident_kernel<T, ACT, UNI>, r, count, stream, (const T*)c.dy, (const T*)c.x, (const T*)c.gamma,
                 (const T*)c.beta, c.mean, c.rstd, (T*)c.dx, reinterpret_cast<float2*>(ws),
-                reinterpret_cast<float2*>(ws + s.gpart), count, c.dparam_f32, (T*)c.dgamma, (T*)c.dbeta, r);
+                reinterpret_cast<float2*>(ws + s.pairs), count, c.dparam_f32, (T*)c.dgamma, (T*)c.dbeta, r);
 }
-template <typename T, int ACT>
-cudaError_t launch_t(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+template <typename T, int ACT, typename Call>
+cudaError_t launch_t(const Call& c, const ResidentGeom& r, cudaStream_t stream) {
   constexpr int VE = 16 / sizeof(T);
   return r.g.D % VE == 0 ? launch_u<T, ACT, true>(c, r, stream) : launch_u<T, ACT, false>(c, r, stream);
 }
-template <typename T>
-cudaError_t launch_act(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+template <typename T, typename Call>
+cudaError_t launch_act(const Call& c, const ResidentGeom& r, cudaStream_t stream) {
   switch (c.act) {
     case kActIdentity: return launch_t<T, kActIdentity>(c, r, stream);
     case kActRelu: return launch_t<T, kActRelu>(c, r, stream);
@@ -439,18 +605,8 @@ cudaError_t launch_act(const BwdCall& c, const ResidentGeom& r, cudaStream_t str
     default: return launch_t<T, kActGeluTanh>(c, r, stream);
   }
 }
-
-}  // namespace
-
-size_t resident_workspace_bytes(const ResidentGeom& r) { return scratch_of(r).total; }
-
-size_t resident_fixed_smem(const ResidentGeom& r) {
-  const Geom& g = r.g;
-  return kControlBytes + ((size_t)g.red_floats + 2 * (size_t)g.C + 2 * (size_t)g.G) * 4 + 16;
-}
-
-cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& geom, cudaStream_t stream) {
-  ResidentGeom r = geom;
+template <typename Call>
+cudaError_t launch_resident(const Call& c, ResidentGeom r, cudaStream_t stream) {
   const cudaError_t err = wait_limit_for_device(&r.g.wait);
   if (err != cudaSuccess) return err;
   switch (c.dtype) {
@@ -458,6 +614,23 @@ cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& geom,
     case 1: return launch_act<__half>(c, r, stream);
     default: return launch_act<__nv_bfloat16>(c, r, stream);
   }
+}
+
+}  // namespace
+
+size_t resident_workspace_bytes(const ResidentGeom& r, int direction) { return scratch_of(r, direction).total; }
+
+size_t resident_fixed_smem(const ResidentGeom& r, int direction) {
+  const Geom& g = r.g;
+  const size_t floats = direction == 0 ? 6 * (size_t)g.slots : 2 * (size_t)g.C + 2 * (size_t)g.G;
+  return kControlBytes + ((size_t)g.red_floats + floats) * 4 + 16;
+}
+
+cudaError_t launch_forward_resident(const FwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+  return launch_resident(c, r, stream);
+}
+cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream) {
+  return launch_resident(c, r, stream);
 }
 
 }  // namespace gnb200

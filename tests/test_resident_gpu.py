@@ -1,4 +1,4 @@
-"""GPU parity tests of the resident plan (csrc/gn_resident.cu): both backward passes in one cooperative kernel, one CTA
+"""GPU parity tests of the resident plan (csrc/gn_resident.cu): both passes in one cooperative kernel, one CTA
 per SM, the last tiles of a CTA's row range kept in shared memory between the passes.
 
 GNB200_RESIDENT_CTAS / _STAGES bound the grid and the ring, so that tile remainders, stage reuse in both
@@ -18,7 +18,7 @@ CASES = [
     # (N, C, spatial, G, dtype, act, CTAs per sample, stages)
     (1, 256, (96, 96), 32, "float16", "silu", 0, 16),        # every SM, one or two tiles each, all resident
     (2, 256, (96, 97), 32, "bfloat16", "gelu", 5, 2),         # many tiles through two stages, ragged last tile
-    (3, 128, (40, 57), 32, "float32", "gelu_tanh", 3, 3),     # fp32: xh form
+    (3, 128, (40, 57), 32, "float32", "gelu_tanh", 3, 3),     # fp32: Welford, xh form
     (2, 320, (33, 47), 32, "float16", "silu", 4, 3),          # D = 10: vectors straddle groups; 32 idle threads
     (1, 40, (131, 17), 8, "float32", "relu", 2, 2),           # D = 5, 10 vectors per row
     (1, 64, (57, 31), 64, "float32", "identity", 7, 2),       # D = 1
@@ -44,14 +44,17 @@ def test_resident_plan_against_oracle(nt, case, monkeypatch):
     monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
     monkeypatch.setenv("GNB200_RESIDENT_CTAS", str(ctas))
     monkeypatch.setenv("GNB200_RESIDENT_STAGES", str(stages))
-    assert " resident=1 " in nt.describe_plan(N, sp[0] * sp[1], C, G, DT[dt], 1)
+    for direction in (0, 1):
+        assert " resident=1 " in nt.describe_plan(N, sp[0] * sp[1], C, G, DT[dt], direction)
     x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=23, x_dist="uniform3")
     out = run_cabi(nt, x, ga, be, dy, G, 1e-5, act)
     want = O.oracle_c(x, ga, be, dy, G, 1e-5, act, threads=4)
     check_against(out, want, DT[dt])
+    assert O.rel_err(out["mean"], want["mean"]) < 1e-5
+    assert O.rel_err(out["rstd"] / want["rstd"].cuda().float(), torch.ones_like(want["rstd"])) < 1e-5
     assert O.rel_err(out["dparam"][0], want["dgamma"]) <= O.TOLERANCE[DT[dt]]
     assert O.rel_err(out["dparam"][1], want["dbeta"]) <= O.TOLERANCE[DT[dt]]
     again = run_cabi(nt, x, ga, be, dy, G, 1e-5, act)  # fixed summation order: bit-identical reruns
-    for k in ("dx", "dparam"):
+    for k in ("y", "dx", "dparam", "mean", "rstd"):
         assert torch.equal(out[k], again[k]), k
     assert nt.wait_timeouts() == 0
