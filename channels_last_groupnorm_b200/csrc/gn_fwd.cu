@@ -236,22 +236,66 @@ __device__ __forceinline__ void tile_apply(uint32_t stile, uint32_t sstep_bytes,
   }
 }
 
-// y = act(x * a + b) over the rows this thread owns, global to global (multi-kernel path).  `back`: from the last row
-// to the first, with streaming stores.  All tiles are in flight at once (four CTAs per SM, one wave), so what L2 still
-// holds of x when the statistics are known is the end of every tile, not the tiles with the highest numbers.
-// Measured (fp16 unless stated, us, forwards -> backwards): 67 MB 41.4 -> 39.8, 134 MB 75.9 -> 74.8, 134 MB fp32
-// 75.8 -> 73.7, 67 MB with one group 39.4 -> 37.1; beyond L2's reach nothing is left to find and the order of DRAM
-// pages counts: 268 MB 147.4 -> 149.0, fp32 148.4 -> 149.9.  The planner draws the line (Geom::back).
-template <typename T, int VE, int ACT, bool BACK>
-__device__ __forceinline__ void stream_apply(const Pack<T, VE>* __restrict__ src, Pack<T, VE>* __restrict__ dst,
-                                             size_t stride_vec, int nrows, int ty, int TY, const float (&a)[VE],
-                                             const float (&b)[VE]) {
+// y = act(x * a + b) over the rows this thread owns, global to global (multi-kernel path).
+template <typename T, int VE, int ACT>
+__device__ __forceinline__ void stream_apply(const Pack<T, VE>* __restrict__ src, size_t src_stride_vec,
+                                             Pack<T, VE>* __restrict__ dst, size_t dst_stride_vec, int nrows, int ty,
+                                             int TY, const float (&a)[VE], const float (&b)[VE]) {
+  constexpr bool FAST = sizeof(T) == 2;
+  constexpr int U = 4;
+  const size_t sstep = (size_t)TY * src_stride_vec, dstep = (size_t)TY * dst_stride_vec;
+  const Pack<T, VE>* sp = src + (size_t)ty * src_stride_vec;
+  Pack<T, VE>* dp = dst + (size_t)ty * dst_stride_vec;
+  int left = ty < nrows ? (nrows - ty + TY - 1) / TY : 0;
+  for (; left >= U; left -= U) {
+    Pack<T, VE> v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      v[u] = ld_stream(sp);
+      sp += sstep;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[VE];
+      unpack<T, VE>(v[u], f);
+      if constexpr (sizeof(T) * VE == 16) {
+#pragma unroll
+        for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+        stg128(dp, act_pack16<T, VE, ACT>(f));
+      } else {
+#pragma unroll
+        for (int e = 0; e < VE; ++e) f[e] = act_fwd<ACT, FAST>(fmaf(f[e], a[e], b[e]));
+        st_stream(dp, pack<T, VE>(f));
+      }
+      dp += dstep;
+    }
+  }
+  for (; left > 0; --left) {
+    float f[VE];
+    unpack<T, VE>(ld_stream(sp), f);
+    sp += sstep;
+#pragma unroll
+    for (int e = 0; e < VE; ++e) f[e] = act_fwd<ACT, FAST>(fmaf(f[e], a[e], b[e]));
+    st_stream(dp, pack<T, VE>(f));
+    dp += dstep;
+  }
+}
+
+// The same from the last row to the first, with streaming stores.  All tiles are in flight at once (four CTAs per SM,
+// one wave), so what L2 still holds of x when the statistics are known is the end of every tile, not the tiles with
+// the highest numbers.  Measured (fp16 unless stated, us, forwards -> backwards): 67 MB 41.4 -> 39.8, 134 MB 75.9 ->
+// 74.8, 134 MB fp32 75.8 -> 73.7, 67 MB with one group 39.4 -> 37.1; beyond L2's reach nothing is left to find and the
+// order of DRAM pages counts: 268 MB 147.4 -> 149.0, fp32 148.4 -> 149.9.  The planner draws the line (Geom::back).
+template <typename T, int VE, int ACT>
+__device__ __forceinline__ void stream_apply_back(const Pack<T, VE>* __restrict__ src, Pack<T, VE>* __restrict__ dst,
+                                                  size_t stride_vec, int nrows, int ty, int TY, const float (&a)[VE],
+                                                  const float (&b)[VE]) {
   constexpr bool FAST = sizeof(T) == 2;
   constexpr int U = 4;
   int left = ty < nrows ? (nrows - ty + TY - 1) / TY : 0;
   if (left == 0) return;
-  const ptrdiff_t step = (BACK ? -1 : 1) * (ptrdiff_t)TY * (ptrdiff_t)stride_vec;
-  const size_t start = (size_t)(ty + (BACK ? (left - 1) * TY : 0)) * stride_vec;
+  const ptrdiff_t step = (ptrdiff_t)TY * (ptrdiff_t)stride_vec;
+  const size_t start = ((size_t)ty + (size_t)(left - 1) * TY) * stride_vec;
   const Pack<T, VE>* sp = src + start;
   Pack<T, VE>* dp = dst + start;
   auto one = [&](const Pack<T, VE>& v) {
@@ -260,30 +304,27 @@ __device__ __forceinline__ void stream_apply(const Pack<T, VE>* __restrict__ src
     if constexpr (sizeof(T) * VE == 16) {
 #pragma unroll
       for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
-      if constexpr (BACK)
-        stg128_stream(dp, act_pack16<T, VE, ACT>(f));
-      else
-        stg128(dp, act_pack16<T, VE, ACT>(f));
+      stg128_stream(dp, act_pack16<T, VE, ACT>(f));
     } else {
 #pragma unroll
       for (int e = 0; e < VE; ++e) f[e] = act_fwd<ACT, FAST>(fmaf(f[e], a[e], b[e]));
       st_stream(dp, pack<T, VE>(f));
     }
-    dp += step;
+    dp -= step;
   };
   for (; left >= U; left -= U) {
     Pack<T, VE> v[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       v[u] = ld_stream(sp);
-      sp += step;
+      sp -= step;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) one(v[u]);
   }
   for (; left > 0; --left) {
     const Pack<T, VE> v = ld_stream(sp);
-    sp += step;
+    sp -= step;
     one(v);
   }
 }
@@ -593,9 +634,9 @@ __global__ void __launch_bounds__(kMaxThreads)
   const P* xs = reinterpret_cast<const P*>(x + base);
   P* ys = reinterpret_cast<P*>(y + base);
   if (g.back)
-    stream_apply<T, VE, ACT, true>(xs, ys, rs, nrows, ty, g.TY, a, b);
+    stream_apply_back<T, VE, ACT>(xs, ys, rs, nrows, ty, g.TY, a, b);
   else
-    stream_apply<T, VE, ACT, false>(xs, ys, rs, nrows, ty, g.TY, a, b);
+    stream_apply<T, VE, ACT>(xs, rs, ys, rs, nrows, ty, g.TY, a, b);
 }
 
 // ------------------------------------------------------------------------------------------------
