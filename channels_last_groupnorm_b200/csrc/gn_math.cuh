@@ -19,10 +19,12 @@ __device__ __forceinline__ void welford_step(const float (&f)[VE], float (&mean)
 
 // 16-bit tensors accumulate shifted sums instead: with K a value of the thread's own data (its
 // first row),  s += x - K,  q += (x - K)^2;  the subtraction converts the 16-bit element on the fly
-// (mixed-precision sub), three instructions per element and no division in the loop.  Because K is
-// one of the samples, (K - mean)^2 <= M2, so q <= (n + 1) M2 and the cancellation in
-// M2 = q - s^2 / n costs at most (n + 1) ulp of the thread's M2 - n is the thread's row count, a
-// few hundred at most - where sums of raw squares would lose mean^2 / var.
+// (mixed-precision sub), three instructions per element and no division in the loop.  KN = VE: every
+// lane has a K of its own, one of its samples, so (K - mean)^2 <= M2, q <= (n + 1) M2 and the cancellation
+// in M2 = q - s^2 / n multiplies the rounding of q and s (sqrt(n) ulp or so) by at most n + 1, where sums of raw
+// squares would multiply it by mean^2 / var.  KN = 1 (the lanes lie in one group): all lanes use lane 0's value, and
+// the same holds for the M2 of the thread's VE * n samples about their common mean, with VE * n in the place of
+// n + 1.  The callers keep n, the rows of one such sum, to 128 at most.
 template <typename T, int VE, int KN>
 __device__ __forceinline__ void shifted_step(const uint4& w, const float (&K)[KN], float (&s)[VE], float (&q)[VE]) {
   static_assert(sizeof(T) == 2 && VE == 8, "16-bit elements, 16-byte vectors");
@@ -53,6 +55,21 @@ __device__ __forceinline__ void shifted_finish(const float (&K)[KN], int rows, f
     mean[e] = K[KN == 1 ? 0 : e] + ds;
     m2[e] = fmaxf(fmaf(-s, ds, q), 0.f);
   }
+}
+
+// (pm, pq) of pn rows merged into (mean, m2) of cnt rows, lane by lane.
+template <int VE>
+__device__ __forceinline__ void merge_moments(const float (&pm)[VE], const float (&pq)[VE], float pn, float (&mean)[VE],
+                                              float (&m2)[VE], float& cnt) {
+  const float all = cnt + pn;
+  const float f = all > 0.f ? pn / all : 0.f, h = cnt * f;
+#pragma unroll
+  for (int e = 0; e < VE; ++e) {
+    const float d = pm[e] - mean[e];
+    m2[e] += fmaf(d * h, d, pq[e]);
+    mean[e] = fmaf(d, f, mean[e]);
+  }
+  cnt = all;
 }
 
 // Per-lane affine coefficients  a = rstd * gamma,  b = beta - mean * a  for the thread's channels.

@@ -30,6 +30,13 @@ constexpr int kMaxStages = 16;
 constexpr int kMergeLoads = 5;   // channel-sum rows a lane has in flight in the dgamma / dbeta sums
 constexpr int kMergeRows = 10;   // partial rows a warp has in flight in a merge (148 CTAs / 16 warps)
 
+// A thread's sums run over at most this many rows before they are merged into the totals: its whole range is
+// R / 148 / TY rows - 111 at 256@512^2, 3543 at 128@4096^2 - where the multi-kernel plan has 55 to 128 per tile, and
+// the rounding of the shifted sums grows with n^1.5.  rstd against fp64 with one pixel far from the rest (fp16),
+// multi-kernel plan / whole range / pieces of 128 / of 32: 256@512^2 5e-6 / 1.9e-5 / 1.9e-5 / 2e-6, 128@1024^2 1.5e-5 /
+// 6.6e-5 / 2.2e-5 / 3e-6, 128 x 2^23 rows 1.3e-5 / 9e-4 / 1.2e-5 / 1.7e-6; the time does not change (337 MB 175 us either way).
+constexpr int kFoldRows = 32;
+
 __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
@@ -195,52 +202,59 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   const uint32_t step = (uint32_t)(g.TY * g.CV) * 16u;
   const int my_row = streaming ? ty : 0x40000000;  // no row of a tile for idle threads
 
-  // ---- pass 1: moments of the thread's rows
-  float mean[VE], m2[VE], K[KN], cnt = 0.f;
+  // ---- pass 1: moments of the thread's rows, closed every kFoldRows rows (the shift is the first row of each piece)
+  float mean[VE], m2[VE], cnt = 0.f;  // of the closed pieces
 #pragma unroll
-  for (int e = 0; e < VE; ++e) mean[e] = 0.f, m2[e] = 0.f;
-#pragma unroll
-  for (int e = 0; e < KN; ++e) K[e] = 0.f;
+  for (int e = 0; e < VE; ++e) mean[e] = m2[e] = 0.f;
   int stage = 0, prev = 0;
-  for (int t = 0; t < T_; ++t) {
-    st.wait_full(stage, g.wait);
-    const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
-    const int here = nrows - t * st.BR;
-    uint4 w[KR];
+  for (int t0 = 0; t0 < T_; t0 += kFoldRows / KR) {
+    const int t1 = min(T_, t0 + kFoldRows / KR);
+    float pm[VE], pq[VE], K[KN], pn = 0.f;
 #pragma unroll
-    for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
+    for (int e = 0; e < VE; ++e) pm[e] = pq[e] = 0.f;
+#pragma unroll
+    for (int e = 0; e < KN; ++e) K[e] = 0.f;
+    for (int t = t0; t < t1; ++t) {
+      st.wait_full(stage, g.wait);
+      const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
+      const int here = nrows - t * st.BR;
+      uint4 w[KR];
+#pragma unroll
+      for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
+      if constexpr (kShifted) {
+        if (t == t0) {
+          float f0[VE];
+          unpack16<T, VE>(w[0], f0);
+          if (my_row < here) {
+#pragma unroll
+            for (int e = 0; e < KN; ++e) K[e] = f0[e];
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < KR; ++u) {
+        if (my_row + u * g.TY < here) {
+          if constexpr (kShifted) {
+            shifted_step<T, VE, KN>(w[u], K, pm, pq);
+          } else {
+            float f[VE];
+            unpack16<T, VE>(w[u], f);
+            welford_step<VE>(f, pm, pq, pn);
+          }
+        }
+      }
+      pin_regs(pm);
+      pin_regs(pq);
+      if (t + S < T_) release_stage(&sm.empty[stage], lane);
+      if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
+      prev = stage;
+      if (++stage == S) stage = 0;
+    }
     if constexpr (kShifted) {
-      if (t == 0) {  // the shift: the values of the thread's first row
-        float f0[VE];
-        unpack16<T, VE>(w[0], f0);
-        if (my_row < here) {
-#pragma unroll
-          for (int e = 0; e < KN; ++e) K[e] = f0[e];
-        }
-      }
+      const int left = min(nrows - t0 * st.BR, (t1 - t0) * st.BR);
+      shifted_finish<VE, KN>(K, my_row < left ? (left - my_row + g.TY - 1) / g.TY : 0, pm, pq, pn);
     }
-#pragma unroll
-    for (int u = 0; u < KR; ++u) {
-      if (my_row + u * g.TY < here) {
-        if constexpr (kShifted) {
-          shifted_step<T, VE, KN>(w[u], K, mean, m2);
-        } else {
-          float f[VE];
-          unpack16<T, VE>(w[u], f);
-          welford_step<VE>(f, mean, m2, cnt);
-        }
-      }
-    }
-    pin_regs(mean);
-    pin_regs(m2);
-    if (t + S < T_) release_stage(&sm.empty[stage], lane);
-    if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
-    prev = stage;
-    if (++stage == S) stage = 0;
-  }
-  if constexpr (kShifted) {
-    const int own = my_row < nrows ? (nrows - my_row + g.TY - 1) / g.TY : 0;
-    shifted_finish<VE, KN>(K, own, mean, m2, cnt);
+    merge_moments<VE>(pm, pq, pn, mean, m2, cnt);
   }
   __syncwarp();
   __syncthreads();
@@ -362,44 +376,52 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     b[e] = fmaf(L.nmr[e], L.ga[e], L.be[e]);
   }
 
-  // ---- pass 1: S1, S2 over the thread's rows
-  float s1[VE], s2[VE];
+  // ---- pass 1: S1, S2 over the thread's rows, closed every kFoldRows rows
+  float s1[VE], s2[VE];  // of the closed pieces
 #pragma unroll
-  for (int e = 0; e < VE; ++e) s1[e] = 0.f, s2[e] = 0.f;
+  for (int e = 0; e < VE; ++e) s1[e] = s2[e] = 0.f;
   int stage = 0, prev = 0;
-  for (int t = 0; t < T_; ++t) {
-    st.wait_full(stage, g.wait);
-    const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
-    const int here = nrows - t * st.BR;
-    uint4 xw[KR], dw[KR];
+  for (int t0 = 0; t0 < T_; t0 += kFoldRows / KR) {
+    const int t1 = min(T_, t0 + kFoldRows / KR);
+    float p1[VE], p2[VE];
 #pragma unroll
-    for (int u = 0; u < KR; ++u) {
-      xw[u] = lds128(base + u * step);
-      dw[u] = lds128(base + st.tile_bytes + u * step);
-    }
+    for (int e = 0; e < VE; ++e) p1[e] = p2[e] = 0.f;
+    for (int t = t0; t < t1; ++t) {
+      st.wait_full(stage, g.wait);
+      const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
+      const int here = nrows - t * st.BR;
+      uint4 xw[KR], dw[KR];
 #pragma unroll
-    for (int u = 0; u < KR; ++u) {
-      if (my_row + u * g.TY < here) {
-        if constexpr (kRaw) {
-          bwd_row_sums_packed<T, ACT>(xw[u], dw[u], a, b, s1, s2);
-        } else {
-          float fx[VE], fd[VE];
-          unpack16<T, VE>(xw[u], fx);
-          unpack16<T, VE>(dw[u], fd);
-          bwd_row_sums<T, VE, ACT>(fx, fd, L, s1, s2);
+      for (int u = 0; u < KR; ++u) {
+        xw[u] = lds128(base + u * step);
+        dw[u] = lds128(base + st.tile_bytes + u * step);
+      }
+#pragma unroll
+      for (int u = 0; u < KR; ++u) {
+        if (my_row + u * g.TY < here) {
+          if constexpr (kRaw) {
+            bwd_row_sums_packed<T, ACT>(xw[u], dw[u], a, b, p1, p2);
+          } else {
+            float fx[VE], fd[VE];
+            unpack16<T, VE>(xw[u], fx);
+            unpack16<T, VE>(dw[u], fd);
+            bwd_row_sums<T, VE, ACT>(fx, fd, L, p1, p2);
+          }
         }
       }
+      pin_regs(p1);
+      pin_regs(p2);
+      if (t + S < T_) release_stage(&sm.empty[stage], lane);
+      if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
+      prev = stage;
+      if (++stage == S) stage = 0;
     }
-    pin_regs(s1);
-    pin_regs(s2);
-    if (t + S < T_) release_stage(&sm.empty[stage], lane);
-    if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
-    prev = stage;
-    if (++stage == S) stage = 0;
-  }
-  if constexpr (kRaw) {  // S2 = sum dyh * xh = rstd * (sum dyh * x - mean * sum dyh)
 #pragma unroll
-    for (int e = 0; e < VE; ++e) s2[e] = fmaf(L.r[e], s2[e], L.nmr[e] * s1[e]);
+    for (int e = 0; e < VE; ++e) {
+      s1[e] += p1[e];
+      // packed: S2 = sum dyh * xh = rstd * (sum dyh * x - mean * sum dyh)
+      s2[e] += kRaw ? fmaf(L.r[e], p2[e], L.nmr[e] * p1[e]) : p2[e];
+    }
   }
   // channel sums over the row lanes, S1 and S2 one after the other through the same scratch
 #pragma unroll
