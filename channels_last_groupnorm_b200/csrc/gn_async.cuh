@@ -81,7 +81,7 @@ __device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw,
     if constexpr (ACT != kActIdentity) {
       const float yh0 = fmaf(fx[2 * p], a[2 * p], b[2 * p]);
       const float yh1 = fmaf(fx[2 * p + 1], a[2 * p + 1], b[2 * p + 1]);
-      const float2 gf = __half22float2(act_grad_h2<ACT>(f32x2_to_h2_sat(yh0, yh1)));
+      const float2 gf = __half22float2(act_grad_pair<ACT>(yh0, yh1));
       g0 = gf.x;
       g1 = gf.y;
     }

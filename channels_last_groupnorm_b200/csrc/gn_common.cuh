@@ -474,9 +474,8 @@ __device__ __forceinline__ __half2 act_fwd_h2(__half2 v) {
 template <int ACT>
 __device__ __forceinline__ __half2 act_grad_h2(__half2 v) {
   const __half2 half_ = __float2half2_rn(0.5f), one = __float2half2_rn(1.0f);
-  if constexpr (ACT == kActRelu) {
-    return __hgt2(v, __float2half2_rn(0.0f));  // 1.0 where v > 0, else 0.0
-  } else if constexpr (ACT == kActSilu) {
+  static_assert(ACT == kActSilu || ACT == kActGelu || ACT == kActGeluTanh, "smooth activations only");
+  if constexpr (ACT == kActSilu) {
     const __half2 t = tanh_h2(__hmul2(v, half_));
     const __half2 s = __hfma2(half_, t, half_);
     return __hmul2(s, __hfma2(v, __hsub2(one, s), one));
@@ -488,6 +487,18 @@ __device__ __forceinline__ __half2 act_grad_h2(__half2 v) {
     // |v| beyond a few tens it is exactly 0, so the product cannot overflow to inf (and inf * 0 = NaN)
     // when v * u' exceeds the half-precision range (|v| above about 1.7e4).
     return __hfma2(__hmul2(__hmul2(v, half_), __hfma2(__hneg2(t), t, one)), du, __hfma2(half_, t, half_));
+  }
+}
+
+// act'(lo), act'(hi) from fp32 pre-activations.  ReLU's gate is decided in fp32: rounded to half precision,
+// everything in (0, 2^-25] would become 0 and lose its gradient.
+template <int ACT>
+__device__ __forceinline__ __half2 act_grad_pair(float lo, float hi) {
+  if constexpr (ACT == kActRelu) {
+    const uint32_t one = 0x3c00u, r = (lo > 0.f ? one : 0u) | (hi > 0.f ? one << 16 : 0u);
+    return *reinterpret_cast<const __half2*>(&r);
+  } else {
+    return act_grad_h2<ACT>(f32x2_to_h2_sat(lo, hi));
   }
 }
 
@@ -523,7 +534,7 @@ __device__ __forceinline__ void act_grad_vec(const float (&yh)[VE], float (&g)[V
   if constexpr (use_h2_bwd<T, ACT>() && VE % 2 == 0) {
 #pragma unroll
     for (int e = 0; e < VE; e += 2) {
-      const float2 f = __half22float2(act_grad_h2<ACT>(f32x2_to_h2_sat(yh[e], yh[e + 1])));
+      const float2 f = __half22float2(act_grad_pair<ACT>(yh[e], yh[e + 1]));
       g[e] = f.x;
       g[e + 1] = f.y;
     }

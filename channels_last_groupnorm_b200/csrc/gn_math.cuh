@@ -253,7 +253,7 @@ __device__ __forceinline__ uint4 bwd_row_sums_packed(const uint4& xw, const uint
     if constexpr (ACT != kActIdentity) {
       const float yh0 = fmaf(mixed_add<T>(x0, -0.0f), a[2 * p], b[2 * p]);
       const float yh1 = fmaf(mixed_add<T>(x1, -0.0f), a[2 * p + 1], b[2 * p + 1]);
-      const __half2 g = act_grad_h2<ACT>(f32x2_to_h2_sat(yh0, yh1));
+      const __half2 g = act_grad_pair<ACT>(yh0, yh1);
       if constexpr (std::is_same<T, __half>::value) {
         const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&dr[p]), g);
         dyh = *reinterpret_cast<const uint32_t*>(&r);
