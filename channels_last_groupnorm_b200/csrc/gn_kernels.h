@@ -90,10 +90,17 @@ void debug_set_trace(void* ptr, size_t bytes);
 size_t wave_workspace_bytes(const WaveGeom& g, int direction);
 cudaError_t launch_forward_wave(const FwdCall& c, const Plan& p, cudaStream_t stream);
 cudaError_t launch_backward_wave(const BwdCall& c, const Plan& p, cudaStream_t stream);
-// resident plan (gn_resident.cu).  cudaErrorCooperativeLaunchTooLarge: nothing was launched, the device (or the
-// share of it that this process has) cannot hold the grid
+// resident plan (gn_resident.cu).  cudaErrorCooperativeLaunchTooLarge: no kernel was launched (a counter in the
+// scratch may have been cleared) and no error is left behind; the device, or the share of it that this process has,
+// cannot hold the grid, and the caller takes the plan that the resident one stands in for
 cudaError_t launch_forward_resident(const FwdCall& c, const ResidentGeom& r, cudaStream_t stream);
 cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream);
+// test hook: applies to the calling thread's next resident launch
+enum { kDebugNone = 0, kDebugRefusedByCheck = 1, kDebugRefusedByRuntime = 2 };
+struct ResidentDebug {
+  int what;
+};
+void debug_next_resident(const ResidentDebug& d);
 size_t resident_workspace_bytes(const ResidentGeom& r, int direction);
 size_t resident_fixed_smem(const ResidentGeom& r, int direction);  // shared memory besides the stages
 // cudaSuccess if `grid` CTAs of this kernel can be resident at once on the current device

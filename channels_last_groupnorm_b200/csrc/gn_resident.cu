@@ -574,11 +574,32 @@ Scratch scratch_of(const ResidentGeom& r, int direction) {
   return s;
 }
 
+// Tests of the fall-back (gnb200_debug_next_resident): what the calling thread's next launch meets.
+thread_local ResidentDebug t_debug = {};
+
+__global__ void gn_resident_refused_kernel() {}
+
+// What the runtime says to a cooperative grid that cannot be resident: a million CTAs of an empty kernel.
+cudaError_t launch_too_large(cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1u << 20, 1, 1);
+  cfg.blockDim = dim3(1024, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, gn_resident_refused_kernel);
+}
+
 template <typename Kern, typename... Args>
 cudaError_t launch(Kern kern, const ResidentGeom& r, unsigned int* count, cudaStream_t stream, Args... args) {
   cudaError_t err = ensure_kernel_attributes((const void*)kern, r.smem_bytes, false);
   if (err != cudaSuccess) return err;
-  err = check_resident((const void*)kern, r.threads, r.smem_bytes, r.grid);
+  const ResidentDebug debug = t_debug;
+  t_debug = ResidentDebug{};
+  err = check_resident((const void*)kern, r.threads, r.smem_bytes, debug.what == kDebugRefusedByCheck ? 1LL << 20 : r.grid);
   if (err != cudaSuccess) return err;
   err = cudaMemsetAsync(count, 0, sizeof(unsigned int), stream);
   if (err != cudaSuccess) return err;
@@ -592,7 +613,10 @@ cudaError_t launch(Kern kern, const ResidentGeom& r, unsigned int* count, cudaSt
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
+  err = debug.what == kDebugRefusedByRuntime ? launch_too_large(stream) : cudaLaunchKernelEx(&cfg, kern, args...);
+  // the runtime notes the refusal as its last error too, which the fall-back plan's launches would report as theirs
+  if (err == cudaErrorCooperativeLaunchTooLarge) (void)cudaGetLastError();
+  return err;
 }
 
 template <typename T, int ACT, bool UNI>
@@ -639,6 +663,8 @@ cudaError_t launch_resident(const Call& c, ResidentGeom r, cudaStream_t stream) 
 }
 
 }  // namespace
+
+void debug_next_resident(const ResidentDebug& d) { t_debug = d; }
 
 size_t resident_workspace_bytes(const ResidentGeom& r, int direction) { return scratch_of(r, direction).total; }
 

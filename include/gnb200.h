@@ -269,6 +269,14 @@ int gnb200_selftest_exchange_timeout(const void* x, const void* gamma, const voi
  */
 void gnb200_debug_set_trace(void* device_buffer, size_t bytes);
 
+/*
+ * For test suites only: what the calling thread's next launch of the resident plan (the cooperative kernel for large
+ * slabs, one CTA per SM) meets.  0 nothing; 1 the occupancy check, 2 the CUDA runtime refuses the grid, as on a device
+ * that this process shares: the call must then run the plan that the resident one stands in for.
+ * No counterpart in the reference.
+ */
+int gnb200_debug_next_resident(int what);
+
 /* Number of kernel launches gnb200_fwd / gnb200_bwd enqueue for this problem. */
 int gnb200_launch_count(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction);
 

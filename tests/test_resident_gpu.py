@@ -58,3 +58,30 @@ def test_resident_plan_against_oracle(nt, case, monkeypatch):
     for k in ("y", "dx", "dparam", "mean", "rstd"):
         assert torch.equal(out[k], again[k]), k
     assert nt.wait_timeouts() == 0
+
+
+@pytest.mark.parametrize("dt", ["float16", "float32"])
+@pytest.mark.parametrize("refused_by", [1, 2], ids=["check", "runtime"])
+def test_a_grid_that_cannot_be_resident_takes_the_other_plan(nt, refused_by, dt, monkeypatch):
+    """A device that this process shares may refuse the cooperative grid, in the occupancy check or at the launch itself.
+    The call then runs the multi-kernel (or wave) plan and leaves no error behind."""
+    from .test_parity_gpu import _flat
+
+    N, C, sp, G, act = 1, 64, (65, 41), 8, O.ACT_CODES["silu"]
+    x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=29)
+    want = O.oracle_c(x, ga, be, dy, G, 1e-5, "silu", threads=4)
+    xd, dyd, gd, bd = _flat(x.cuda()), _flat(dy.cuda()), ga.cuda(), be.cuda()
+    monkeypatch.setenv("GNB200_FORCE_PATH", "twopass")
+    plain = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)
+    monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
+    nt.check(nt.lib.gnb200_debug_next_resident(refused_by))
+    y, mean, rstd = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)
+    assert torch.equal(y, plain[0]) and torch.equal(mean, plain[1]) and torch.equal(rstd, plain[2])
+    nt.check(nt.lib.gnb200_debug_next_resident(refused_by))
+    dx, dparam, dgamma, dbeta = nt.bwd_raw(dyd, xd, gd, bd, mean, rstd, G, act)
+    assert O.rel_err(dx.reshape(N, *sp, C).permute(0, 3, 1, 2), want["dx"]) <= O.TOLERANCE[DT[dt]]
+    assert O.rel_err(dgamma, want["dgamma"]) <= O.TOLERANCE[DT[dt]] and O.rel_err(dbeta, want["dbeta"]) <= O.TOLERANCE[DT[dt]]
+    assert torch.equal(xd + 1, 1 + xd)  # (a torch launch checks the last error)
+    torch.cuda.synchronize()
+    again = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)  # the hook held for one launch: resident again
+    assert O.rel_err(again[1], want["mean"]) < 1e-5
