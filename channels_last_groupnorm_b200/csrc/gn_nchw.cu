@@ -55,10 +55,24 @@ __device__ __forceinline__ void store16(void* p, const uint4 v, int evict) {
   else
     stg128(p, v);
 }
+// The same without a branch, for the dx kernel, whose arithmetic for the four vectors in flight a branch would keep
+// apart.  (The forward's output pass is the other way round: 8 x 256@64^2 bf16 11.9 us with the branch, 12.8 without, 4 x
+// 320@48^2 8.2 and 9.3.)
+__device__ __forceinline__ void store16_predicated(void* p, const uint4 v, int evict) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.s32 p, %5, 0;\n"
+      "@p st.global.cs.v4.u32 [%0], {%1, %2, %3, %4};\n"
+      "@!p st.global.v4.u32 [%0], {%1, %2, %3, %4};\n"
+      "}\n" ::"l"(p),
+      "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(evict)
+      : "memory");
+}
 template <typename T, int VE>
 __device__ __forceinline__ void store_vec(T* p, const float (&f)[VE], int evict) {
   if constexpr (sizeof(T) * VE == 16) {
-    store16(p, pack16<T, VE>(f), evict);
+    store16_predicated(p, pack16<T, VE>(f), evict);
   } else {
 #pragma unroll
     for (int e = 0; e < VE; ++e) p[e] = store_param<T>(f[e]);
@@ -373,7 +387,7 @@ __global__ void __launch_bounds__(128)
 // backward 4: dx = rstd * (gamma_c * dyh - A - xh * B), one warp per piece as in the reduce kernel, the pieces in
 // reverse order and from their ends (see forward 2)
 template <typename T, int VE, int ACT>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 4)
     gn_nchw_dx_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                       const T* __restrict__ beta, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
                       const float* __restrict__ coef, T* __restrict__ dx, long long pieces, const NchwGeom g) {
@@ -396,7 +410,12 @@ __global__ void __launch_bounds__(kThreads)
   const T* xs = x + row * g.R;
   const T* ds = dy + row * g.R;
   T* os = dx + row * g.R;
-  auto one = [&](long long v, const float (&fx)[VE], const float (&fd)[VE]) {
+  // x and dy are read-only, so the compiler may move the first loads in front of the wait above: then the CTAs that are
+  // placed early read their rows while the reduce kernel still streams its own through L2.  With at least four CTAs per SM (three
+  // without the bound) it measured, us, loads in front / behind / behind and four CTAs: 64 x 256@64^2 bf16 136 / 127 / 123,
+  // 512@256^2 fp16 75 / 70 / 68, 8 x 256@64^2 bf16 22.3 / 22.0 / 21.3; five CTAs: 123 / 68.8 / 23.0 and spills in fp32.
+  asm volatile("" : "+l"(xs), "+l"(ds));
+  auto one = [&](T* out, const float (&fx)[VE], const float (&fd)[VE]) {
     float xh[VE], yh[VE], gr[VE], o[VE];
 #pragma unroll
     for (int e = 0; e < VE; ++e) {
@@ -406,24 +425,43 @@ __global__ void __launch_bounds__(kThreads)
     act_grad_vec<T, VE, ACT>(yh, gr);
 #pragma unroll
     for (int e = 0; e < VE; ++e) o[e] = fmaf(ag, fd[e] * gr[e], fmaf(nb, xh[e], na));
-    store_vec<T, VE>(os + v * VE, o, g.evict);
+    store_vec<T, VE>(out, o, g.evict);
   };
+  constexpr int kStep = 32 * VE;
   long long v = v1 - 1 - lane;
   for (; v - (kUnroll - 1) * 32 >= v0; v -= kUnroll * 32) {
-    float fx[kUnroll][VE], fd[kUnroll][VE];
+    const T *px = xs + v * VE, *pd = ds + v * VE;
+    T* po = os + v * VE;
+    if constexpr (sizeof(T) * VE == 16) {  // packed while in flight
+      uint4 wx[kUnroll], wd[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      load_vec<T, VE>(xs + (v - u * 32) * VE, fx[u]);
-      load_vec<T, VE>(ds + (v - u * 32) * VE, fd[u]);
+      for (int u = 0; u < kUnroll; ++u) {
+        wx[u] = ldg128(px - u * kStep);
+        wd[u] = ldg128(pd - u * kStep);
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        float fx[VE], fd[VE];
+        unpack16<T, VE>(wx[u], fx);
+        unpack16<T, VE>(wd[u], fd);
+        one(po - u * kStep, fx, fd);
+      }
+    } else {
+      float fx[kUnroll][VE], fd[kUnroll][VE];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        load_vec<T, VE>(px - u * kStep, fx[u]);
+        load_vec<T, VE>(pd - u * kStep, fd[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) one(po - u * kStep, fx[u], fd[u]);
     }
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) one(v - u * 32, fx[u], fd[u]);
   }
   for (; v >= v0; v -= 32) {
     float fx[VE], fd[VE];
     load_vec<T, VE>(xs + v * VE, fx);
     load_vec<T, VE>(ds + v * VE, fd);
-    one(v, fx, fd);
+    one(os + v * VE, fx, fd);
   }
 }
 
