@@ -488,27 +488,39 @@ NchwGeom make_geom(long long N, long long R, long long C, long long G, int ve) {
   g.row_vecs = R / ve;
   g.div_R = fast_div(R);
   g.evict = (double)N * C * R * (16 / ve) > 32.0 * 1024 * 1024;  // (single elements are stored plainly)
-  // forward: sixteen chunks per SM, at least 2048 vectors (32 KB) each.  Several waves of CTAs even out the SMs and
-  // let the reverse order of the output pass work across CTAs too: with four chunks per SM (all in flight at once)
-  // 43.6 us at 512@256^2 fp16, 90 us at 2 x 256@256^2 fp32, 114 us at 3 x 128@300x301 bf16; with sixteen 39.0, 77.6, 78.6
-  // (with the statistics of that time; the first is 36.2 now).
-  const long long slabs = N * G;
+  // forward: sixteen chunks per SM, at least 2048 vectors (32 KB; single elements: 4096) each.  Several waves of CTAs
+  // even out the SMs and let the reverse order of the output pass work across CTAs too: with four chunks per SM (all in
+  // flight at once) 39.3 us at 512@256^2 fp16, 90 us at 2 x 256@256^2 fp32, 113 us at 3 x 128@300x301 bf16; with sixteen
+  // 36.1, 75.9, 76.2.  What does not fill a batch of kUnroll vectors per thread goes vector by vector, so chunks are whole
+  // batches where that saves steps (2 x 32@300x200 fp32 18.1 -> 15.5, 64 x 64@112^2 bf16 with chunks of 1568 vectors 61.9
+  // -> 56.8, 4 x 512@33^2 12.3 -> 10.9 and with 4096 elements 10.5, 16 x 1024@14^2 18.4 -> 16.7 and 14.7) and of equal
+  // length elsewhere (640@32^2: twice 1280 vectors 5.8, 2048 and 512 6.1).
+  const long long slabs = N * G, fwd_batch = kUnroll * kThreads, min_chunk = ve == 1 ? 4096 : 2048;
   long long chunks = (16LL * kSmCount + slabs - 1) / slabs;
-  const long long max_chunks = (g.slab_vecs + 2047) / 2048;
+  const long long max_chunks = (g.slab_vecs + min_chunk - 1) / min_chunk;
   if (chunks > max_chunks) chunks = max_chunks;
   if (chunks < 1) chunks = 1;
   if (chunks > 1024) chunks = 1024;
   g.chunk_vecs = (g.slab_vecs + chunks - 1) / chunks;
+  const long long steps = g.chunk_vecs / fwd_batch + (g.chunk_vecs % fwd_batch + kThreads - 1) / kThreads;
+  const long long batches = (g.chunk_vecs + fwd_batch - 1) / fwd_batch;
+  if (batches < steps) g.chunk_vecs = batches * fwd_batch;
   g.chunks = (int)((g.slab_vecs + g.chunk_vecs - 1) / g.chunk_vecs);
-  // backward: one warp per piece of a channel row; about 96 warps per SM, 128 .. 2048 vectors per piece, for the same
-  // reason: 512@256^2 fp16 101 us with 16, 78 with 64, 74.7 with 96, 74.9 with 128 (320 CTAs of the first kind lie
-  // three on some SMs and two on the others); 2 x 256@256^2 fp32 119 / 131 / 117.6 / 118.7
-  const long long rows = N * C;
+  // backward: one warp per piece of a channel row; about 96 warps per SM for the same reason (512@256^2 fp16 93 us with
+  // 16, 71.9 with 64, 70.8 with 96, 71.6 with 128: 320 CTAs of the first kind lie three on some SMs and two on the others;
+  // 2 x 256@256^2 fp32 133 / 127 / 120 / 124), up to 2048 vectors per piece and at least 128, or 256 where that still makes 28
+  // warps per SM: a piece of 128 is one batch of loads and nothing to hide them behind (8 x 256@64^2 bf16 22.5 / 21.3,
+  // 8 x 256@48^2 17.8 / 16.8, but 4 x 320@96^2, 1280 rows, 28.4 / 32.3).
+  const long long rows = N * C, bwd_batch = kUnroll * 32, min_piece = rows >= 2048 ? 2 * bwd_batch : bwd_batch;
   long long ppr = (96LL * kSmCount + rows - 1) / rows;
-  const long long max_ppr = (g.row_vecs + 127) / 128;
+  const long long max_ppr = (g.row_vecs + min_piece - 1) / min_piece;
   if (ppr > max_ppr) ppr = max_ppr;
   if (ppr < 1) ppr = 1;
-  long long piece = (g.row_vecs + ppr - 1) / ppr;
+  // as few pieces as whole batches of that length make, of equal length (8 x 256@64^2 fp32: four of 256 37.1, seven of 160
+  // 41.7; 512@256^2 fp16: 22 of 384 68.9, 26 of 320 70.8)
+  long long piece = ((g.row_vecs + ppr - 1) / ppr + bwd_batch - 1) / bwd_batch * bwd_batch;
+  ppr = (g.row_vecs + piece - 1) / piece;
+  piece = (g.row_vecs + ppr - 1) / ppr;
   if (piece > 2048) piece = 2048;
   piece = (piece + 31) / 32 * 32;
   g.piece_vecs = piece;

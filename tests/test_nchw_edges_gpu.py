@@ -17,6 +17,10 @@ pytestmark = pytest.mark.gpu
     (1, 33, (32, 40), 1, "float16", "gelu_tanh"),  # one group of 33 channels: warps take unequal shares
     (1, 2, (1, 8), 1, "float16", "identity"),      # one vector per row
     (1, 8, (200, 331), 1, "float32", "silu"),      # many chunks per slab, remainder at both ends
+    (1, 8, (64, 98), 1, "float16", "silu"),        # 6272 vectors: three chunks of two whole batches and a rest of 128
+    (1, 6, (61, 67), 2, "bfloat16", "gelu"),       # 12261 single elements: chunks of 4096, four batches
+    (1, 2048, (24, 25), 32, "float32", "silu"),    # 2048 rows of 150 vectors: pieces of 256 at least, so one of 160
+    (2, 8, (100, 92), 2, "float16", "relu"),       # rows of 1150 vectors: nine equal pieces, the last one shorter
 ], ids=lambda c: "%dx%dx%s-g%d-%s-%s" % (c[0], c[1], "x".join(map(str, c[2])), *c[3:]))
 def test_channels_first_edges_against_oracle(case):
     from channels_last_groupnorm_b200 import _native as nt
