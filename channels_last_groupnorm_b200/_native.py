@@ -117,7 +117,7 @@ lib.gnb200_selftest_exchange_timeout.argtypes = [_c_void_p, _c_void_p, _c_void_p
                                                  ctypes.c_double, ctypes.c_int, ctypes.c_int, _c_void_p, _c_void_p,
                                                  _c_void_p, _c_void_p]
 lib.gnb200_debug_next_resident.restype = ctypes.c_int
-lib.gnb200_debug_next_resident.argtypes = [ctypes.c_int]
+lib.gnb200_debug_next_resident.argtypes = [ctypes.c_int, ctypes.c_int]
 ERR_EXCHANGE_TIMEOUT = -5
 
 

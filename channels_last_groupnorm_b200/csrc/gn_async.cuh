@@ -55,14 +55,14 @@ __device__ __forceinline__ void producer_wait(uint64_t* bar, unsigned parity, vo
 // consumers (whole warps): if the phase is not complete yet, lane 0 alone polls - 256 polling threads
 // would take issue slots from the CTAs that share the SM - and afterwards every lane observes the
 // completed phase with one more try_wait of its own, which is what makes the TMA's writes visible
-// to it.
-__device__ __forceinline__ void consumer_wait(uint64_t* bar, unsigned parity, volatile int* gave_up, const WaitLimit& lim) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return;
+// to it.  Returns, alike in all lanes, whether the phase is complete.
+__device__ __forceinline__ bool consumer_wait(uint64_t* bar, unsigned parity, volatile int* gave_up, const WaitLimit& lim) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   if ((threadIdx.x & 31) == 0 && *gave_up == 0) {
     if (!mbar_wait_bounded(bar, parity, lim)) *gave_up = 1;
   }
   __syncwarp();
-  (void)mbar_try_wait(bar, parity);
+  return __all_sync(0xffffffffu, mbar_try_wait(bar, parity));
 }
 
 // dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half

@@ -447,10 +447,10 @@ int gnb200_describe_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, 
 
 void gnb200_debug_set_trace(void* device_buffer, size_t bytes) { gnb200::debug_set_trace(device_buffer, bytes); }
 
-int gnb200_debug_next_resident(int what) {
-  if (what < gnb200::kDebugNone || what > gnb200::kDebugRefusedByRuntime)
+int gnb200_debug_next_resident(int what, int cta) {
+  if (what < gnb200::kDebugNone || what > gnb200::kDebugNoSecondCopy)
     return fail(GNB200_ERR_INVALID_ARGUMENT, "gnb200_debug_next_resident: unknown code %d", what);
-  gnb200::debug_next_resident({what});
+  gnb200::debug_next_resident({what, cta});
   return GNB200_OK;
 }
 

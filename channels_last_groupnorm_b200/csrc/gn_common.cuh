@@ -713,7 +713,9 @@ struct ResidentGeom {
   long long grid;      // N * cps
   size_t smem_bytes;
   size_t ws_bytes;     // scratch the kernel itself needs
+  int test_what, test_cta;  // tests only (set by the launcher): what goes wrong, and in which CTA
 };
+enum { kDebugNone = 0, kDebugRefusedByCheck, kDebugRefusedByRuntime, kDebugNoArrival, kDebugNoFirstCopy, kDebugNoSecondCopy };
 
 // Groups touched by column block starting at channel c0 (width CW, clipped to C):
 // first group and how many.

@@ -96,9 +96,8 @@ cudaError_t launch_backward_wave(const BwdCall& c, const Plan& p, cudaStream_t s
 cudaError_t launch_forward_resident(const FwdCall& c, const ResidentGeom& r, cudaStream_t stream);
 cudaError_t launch_backward_resident(const BwdCall& c, const ResidentGeom& r, cudaStream_t stream);
 // test hook: applies to the calling thread's next resident launch
-enum { kDebugNone = 0, kDebugRefusedByCheck = 1, kDebugRefusedByRuntime = 2 };
 struct ResidentDebug {
-  int what;
+  int what, cta;
 };
 void debug_next_resident(const ResidentDebug& d);
 size_t resident_workspace_bytes(const ResidentGeom& r, int direction);

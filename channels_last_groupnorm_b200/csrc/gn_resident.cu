@@ -43,6 +43,11 @@ __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, ui
                : "memory");
 }
 
+// tests only: this CTA is the one that goes wrong in that way
+__device__ __forceinline__ bool test_at(const ResidentGeom& r, int what) {
+  return r.test_what == what && (int)blockIdx.x == r.test_cta;
+}
+
 // Shared memory: [stages * NT tiles][full][empty][flags][reduction scratch]; NT tensors: x, or x and dy
 struct Smem {
   uint32_t stage0;
@@ -71,11 +76,12 @@ struct Stream {
   const T* src[NT];  // x (and dy): first element of the CTA's row range
   int tiles, nrows, BR, stages;
   uint32_t row_bytes, tile_bytes;
-  unsigned full_ph, empty_ph;
+  unsigned full_ph, empty_ph, last_ph;  // last_ph: the phase of each stage's last copy
   Smem sm;
 
   __device__ __forceinline__ void issue(int t, int stage) {  // thread 0
     const uint32_t bytes = (uint32_t)min(BR, nrows - t * BR) * row_bytes;
+    last_ph ^= 1u << stage;
     mbar_arrive_expect_tx(&sm.full[stage], NT * bytes);
 #pragma unroll
     for (int i = 0; i < NT; ++i)
@@ -84,14 +90,21 @@ struct Stream {
   }
   // thread 0: waits until every warp has handed the stage back, then refills it.  Without the hand-back
   // (its wait gave up) nothing is copied over a stage that may still be read.
-  __device__ __forceinline__ void refill(int t, int stage, const WaitLimit& lim) {
+  __device__ __forceinline__ void refill(int t, int stage, const WaitLimit& lim, bool withhold = false) {
     producer_wait(&sm.empty[stage], (empty_ph >> stage) & 1u, &sm.flags[0], lim);
     empty_ph ^= 1u << stage;
-    if (*(volatile int*)&sm.flags[0] == 0) issue(t, stage);
+    if (*(volatile int*)&sm.flags[0] == 0 && !withhold) issue(t, stage);
   }
-  __device__ __forceinline__ void wait_full(int stage, const WaitLimit& lim) {
-    consumer_wait(&sm.full[stage], (full_ph >> stage) & 1u, &sm.flags[0], lim);
+  __device__ __forceinline__ bool wait_full(int stage, const WaitLimit& lim) {
+    const bool ok = consumer_wait(&sm.full[stage], (full_ph >> stage) & 1u, &sm.flags[0], lim);
     full_ph ^= 1u << stage;
+    return ok;
+  }
+  // A wait that gave up leaves copies behind that nobody waited for: they must not land after the CTA has left.
+  __device__ __forceinline__ void drain(const WaitLimit& lim) {  // thread 0
+    if (*(volatile int*)&sm.flags[0] == 0) return;
+    for (int s = 0; s < stages; ++s)
+      if (!mbar_wait_bounded(&sm.full[s], (last_ph >> s) & 1u, lim)) return;
   }
 };
 
@@ -105,6 +118,7 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
   st.row_bytes = (uint32_t)(r.g.C * (int)sizeof(T));
   st.tile_bytes = (uint32_t)r.tile_bytes;
   st.full_ph = st.empty_ph = 0;
+  st.last_ph = ~0u;
   if (threadIdx.x == 0) {
     for (int s = 0; s < r.stages; ++s) {
       mbar_init(&sm.full[s], 1);
@@ -112,31 +126,42 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
     }
     sm.flags[0] = 0;
     fence_mbar_init_cluster();
-    for (int t = 0; t < min(r.stages, st.tiles); ++t) st.issue(t, t);
+    for (int t = test_at(r, kDebugNoFirstCopy) ? 1 : 0; t < min(r.stages, st.tiles); ++t) st.issue(t, t);
   }
   __syncthreads();
 }
 
-// Grid barrier: every CTA has written its partial sums.  `count` starts at 0 (cleared in stream order
-// before the launch).  A wait that gives up sets flags[0]; the caller then writes NaN.
-__device__ __forceinline__ void grid_barrier(unsigned int* count, int* flags, const WaitLimit& lim) {
+// Grid barrier: every CTA has written its partial sums.  `count` starts at 0 (cleared in stream order before the
+// launch); its low half counts the CTAs, its high half those whose partial sums are worthless, because a copy they
+// needed did not arrive in time.  In every CTA that learns of one, or that gives up waiting here, flags[0] is set
+// afterwards; the caller then writes NaN.
+__device__ __forceinline__ void grid_barrier(unsigned int* count, int* flags, const ResidentGeom& r) {
+  const WaitLimit& lim = r.g.wait;
   __syncwarp();
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    atomicAdd(count, 1u);
+    if (!test_at(r, kDebugNoArrival)) atomicAdd(count, *(volatile int*)flags == 0 ? 1u : 0x10001u);
     const long long t0 = clock64();
-    unsigned int polls = 0;
-    while (ld_acquire_u32(count) < gridDim.x) {
+    unsigned int polls = 0, seen;
+    while (((seen = ld_acquire_u32(count)) & 0xffffu) < gridDim.x) {
       if (++polls > lim.polls && clock64() - t0 > lim.clocks) {
         wait_gave_up(lim);
         flags[0] = 1;
         break;
       }
     }
+    if (seen >> 16) flags[0] = 1;
     __threadfence();
   }
   __syncthreads();
+}
+
+// The thread's rows among the first `rows` of the CTA's range, whose values are not known: all bits set is a NaN in
+// every element type.  `first` is the thread's first row.
+__device__ __forceinline__ void store_nan_rows(void* first, size_t row_bytes, int my_row, int TY, int rows) {
+  for (int i = my_row; i < rows; i += TY)
+    stg128_stream(static_cast<char*>(first) + (size_t)(i - my_row) * row_bytes, make_uint4(~0u, ~0u, ~0u, ~0u));
 }
 
 // Sums over `rows` partial rows of G pairs each: warp w takes the rows w, w + nwarps, ..., lane l the groups l, l + 32, ...;
@@ -261,7 +286,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   cta_slot_moments<VE, UNI>(g, mean, m2, cnt, tx, ty, 0, nrows, 0, g.G, red, tmp, slot);
   for (int s = tid; s < g.G; s += blockDim.x)
     part[(size_t)blockIdx.x * g.G + s] = make_float2(slot[s], slot[g.slots + s]);
-  grid_barrier(count, sm.flags, g.wait);
+  grid_barrier(count, sm.flags, r);
 
   // ---- statistics of the sample: sums about the first CTA's mean, the counts known from the geometry
   const bool ok = *(volatile int*)&sm.flags[0] == 0;
@@ -301,8 +326,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   T* out = y + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
   const size_t ostep = (size_t)g.TY * g.C;
   stage = prev;  // of the last tile
-  for (int t = T_ - 1; t >= 0; --t) {
-    if (t < T_ - S) st.wait_full(stage, g.wait);
+  int t = ok ? T_ - 1 : -1;
+  for (; t >= 0; --t) {
+    if (t < T_ - S && !st.wait_full(stage, g.wait)) break;
     const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
     const int here = nrows - t * st.BR;
     T* o = out + (size_t)t * st.BR * g.C;
@@ -320,10 +346,14 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       }
     }
     if (t >= S) release_stage(&sm.empty[stage], lane);
-    if (tid == 0 && t + 1 < T_ && t + 1 >= S) st.refill(t + 1 - S, prev, g.wait);
+    if (tid == 0 && t + 1 < T_ && t + 1 >= S)
+      st.refill(t + 1 - S, prev, g.wait, t == T_ - 2 && test_at(r, kDebugNoSecondCopy));
     prev = stage;
     stage = stage == 0 ? S - 1 : stage - 1;
   }
+  if (!ok) t = T_ - 1;
+  store_nan_rows(out, (size_t)g.C * sizeof(T), my_row, g.TY, min(nrows, (t + 1) * st.BR));  // none, unless a wait gave up
+  if (tid == 0) st.drain(g.wait);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -457,7 +487,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     w2 = warp_sum_all(w2);
     if (lane == 0) gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2);
   }
-  grid_barrier(count, sm.flags, g.wait);
+  grid_barrier(count, sm.flags, r);
 
   // ---- A, B of the sample's groups
   const bool ok = *(volatile int*)&sm.flags[0] == 0;
@@ -495,8 +525,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   T* out = dx + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
   const size_t ostep = (size_t)g.TY * g.C;
   stage = prev;
-  for (int t = T_ - 1; t >= 0; --t) {
-    if (t < T_ - S) st.wait_full(stage, g.wait);
+  int t = ok ? T_ - 1 : -1;
+  for (; t >= 0; --t) {
+    if (t < T_ - S && !st.wait_full(stage, g.wait)) break;
     const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
     const int here = nrows - t * st.BR;
     T* o = out + (size_t)t * st.BR * g.C;
@@ -528,14 +559,18 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       }
     }
     if (t >= S) release_stage(&sm.empty[stage], lane);
-    if (tid == 0 && t + 1 < T_ && t + 1 >= S) st.refill(t + 1 - S, prev, g.wait);
+    if (tid == 0 && t + 1 < T_ && t + 1 >= S)
+      st.refill(t + 1 - S, prev, g.wait, t == T_ - 2 && test_at(r, kDebugNoSecondCopy));
     prev = stage;
     stage = stage == 0 ? S - 1 : stage - 1;
   }
+  if (!ok) t = T_ - 1;
+  store_nan_rows(out, (size_t)g.C * sizeof(T), my_row, g.TY, min(nrows, (t + 1) * st.BR));  // none, unless a wait gave up
 
   // ---- dgamma / dbeta: the grid's warps share the channels; all channel sums are visible since the barrier
   const int rows = g.N * r.cps;
   const bool bad = *(volatile int*)&sm.flags[0] != 0;
+  if (tid == 0) st.drain(g.wait);
   for (int c = (int)blockIdx.x + (int)gridDim.x * warp; c < g.C; c += (int)gridDim.x * nwarps) {
     float t1 = 0.f, t2 = 0.f;
     for (int i0 = lane; i0 < rows + lane; i0 += 32 * kMergeLoads) {
@@ -574,7 +609,7 @@ Scratch scratch_of(const ResidentGeom& r, int direction) {
   return s;
 }
 
-// Tests of the fall-back (gnb200_debug_next_resident): what the calling thread's next launch meets.
+// tests (gnb200_debug_next_resident): what the calling thread's next launch meets
 thread_local ResidentDebug t_debug = {};
 
 __global__ void gn_resident_refused_kernel() {}
@@ -597,9 +632,7 @@ template <typename Kern, typename... Args>
 cudaError_t launch(Kern kern, const ResidentGeom& r, unsigned int* count, cudaStream_t stream, Args... args) {
   cudaError_t err = ensure_kernel_attributes((const void*)kern, r.smem_bytes, false);
   if (err != cudaSuccess) return err;
-  const ResidentDebug debug = t_debug;
-  t_debug = ResidentDebug{};
-  err = check_resident((const void*)kern, r.threads, r.smem_bytes, debug.what == kDebugRefusedByCheck ? 1LL << 20 : r.grid);
+  err = check_resident((const void*)kern, r.threads, r.smem_bytes, r.test_what == kDebugRefusedByCheck ? 1LL << 20 : r.grid);
   if (err != cudaSuccess) return err;
   err = cudaMemsetAsync(count, 0, sizeof(unsigned int), stream);
   if (err != cudaSuccess) return err;
@@ -613,7 +646,7 @@ cudaError_t launch(Kern kern, const ResidentGeom& r, unsigned int* count, cudaSt
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  err = debug.what == kDebugRefusedByRuntime ? launch_too_large(stream) : cudaLaunchKernelEx(&cfg, kern, args...);
+  err = r.test_what == kDebugRefusedByRuntime ? launch_too_large(stream) : cudaLaunchKernelEx(&cfg, kern, args...);
   // the runtime notes the refusal as its last error too, which the fall-back plan's launches would report as theirs
   if (err == cudaErrorCooperativeLaunchTooLarge) (void)cudaGetLastError();
   return err;
@@ -655,6 +688,10 @@ template <typename Call>
 cudaError_t launch_resident(const Call& c, ResidentGeom r, cudaStream_t stream) {
   const cudaError_t err = wait_limit_for_device(&r.g.wait);
   if (err != cudaSuccess) return err;
+  r.test_what = t_debug.what;
+  r.test_cta = t_debug.cta;
+  t_debug = ResidentDebug{};
+  if (r.test_what >= kDebugNoArrival) r.g.wait.clocks = 2000000, r.g.wait.polls = 256;  // about a millisecond
   switch (c.dtype) {
     case 0: return launch_act<float>(c, r, stream);
     case 1: return launch_act<__half>(c, r, stream);

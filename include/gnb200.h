@@ -272,10 +272,13 @@ void gnb200_debug_set_trace(void* device_buffer, size_t bytes);
 /*
  * For test suites only: what the calling thread's next launch of the resident plan (the cooperative kernel for large
  * slabs, one CTA per SM) meets.  0 nothing; 1 the occupancy check, 2 the CUDA runtime refuses the grid, as on a device
- * that this process shares: the call must then run the plan that the resident one stands in for.
+ * that this process shares: the call must then run the plan that the resident one stands in for.  With a wait limit of
+ * about a millisecond, CTA `cta` does not arrive at the grid's barrier (3), does not start its first copy (4), or not the
+ * first copy of its second pass (5): waits run out, nothing faults or hangs, and the outputs that depend on what is
+ * missing are NaN (3, 4: all; 5: that CTA's rows from the missing ones on, and parameter gradients).
  * No counterpart in the reference.
  */
-int gnb200_debug_next_resident(int what);
+int gnb200_debug_next_resident(int what, int cta);
 
 /* Number of kernel launches gnb200_fwd / gnb200_bwd enqueue for this problem. */
 int gnb200_launch_count(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction);

@@ -74,10 +74,10 @@ def test_a_grid_that_cannot_be_resident_takes_the_other_plan(nt, refused_by, dt,
     monkeypatch.setenv("GNB200_FORCE_PATH", "twopass")
     plain = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)
     monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
-    nt.check(nt.lib.gnb200_debug_next_resident(refused_by))
+    nt.check(nt.lib.gnb200_debug_next_resident(refused_by, 0))
     y, mean, rstd = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)
     assert torch.equal(y, plain[0]) and torch.equal(mean, plain[1]) and torch.equal(rstd, plain[2])
-    nt.check(nt.lib.gnb200_debug_next_resident(refused_by))
+    nt.check(nt.lib.gnb200_debug_next_resident(refused_by, 0))
     dx, dparam, dgamma, dbeta = nt.bwd_raw(dyd, xd, gd, bd, mean, rstd, G, act)
     assert O.rel_err(dx.reshape(N, *sp, C).permute(0, 3, 1, 2), want["dx"]) <= O.TOLERANCE[DT[dt]]
     assert O.rel_err(dgamma, want["dgamma"]) <= O.TOLERANCE[DT[dt]] and O.rel_err(dbeta, want["dbeta"]) <= O.TOLERANCE[DT[dt]]
@@ -85,3 +85,59 @@ def test_a_grid_that_cannot_be_resident_takes_the_other_plan(nt, refused_by, dt,
     torch.cuda.synchronize()
     again = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)  # the hook held for one launch: resident again
     assert O.rel_err(again[1], want["mean"]) < 1e-5
+
+
+@pytest.mark.parametrize("what", [3, 4, 5], ids=["no arrival", "no first copy", "no copy of the second pass"])
+@pytest.mark.parametrize("dt,act", [("float16", "relu"), ("float32", "silu")])
+def test_waits_that_run_out_leave_nan_and_a_status(nt, what, dt, act, monkeypatch):
+    """One CTA withholds what others, or its own threads, wait for (decided on the host, wait limit one millisecond).  The
+    call returns, the outputs that depend on it are NaN - for ReLU too, which maps a NaN pre-activation to 0 - the rest is
+    what it should be, the next call reports the failure, and after re-arming everything runs as before."""
+    from .test_parity_gpu import _flat
+
+    N, C, sp, G, code, ctas, cta = 2, 64, (32, 120), 8, O.ACT_CODES[act], 3, 1
+    monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
+    monkeypatch.setenv("GNB200_RESIDENT_CTAS", str(ctas))
+    monkeypatch.setenv("GNB200_RESIDENT_STAGES", "2")
+    x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=37)
+    xd, dyd, gd, bd = _flat(x.cuda()), _flat(dy.cuda()), ga.cuda(), be.cuda()
+    good = nt.fwd_raw(xd, gd, bd, G, 1e-5, code)
+    mean, rstd = good[1], good[2]
+    good_b = nt.bwd_raw(dyd, xd, gd, bd, mean, rstd, G, code)
+    plans = [dict(kv.split("=") for kv in nt.describe_plan(N, sp[0] * sp[1], C, G, DT[dt], d).split()[2:]) for d in (0, 1)]
+
+    def run(direction):
+        nt.check(nt.lib.gnb200_debug_next_resident(what, cta))
+        try:
+            out = nt.fwd_raw(xd, gd, bd, G, 1e-5, code) if direction == 0 else nt.bwd_raw(dyd, xd, gd, bd, mean, rstd, G, code)
+            torch.cuda.synchronize()  # the call returns and the GPU still answers
+            assert nt.wait_timeouts() > 0
+            with pytest.raises(nt.Gnb200Error) as err:
+                nt.fwd_raw(xd, gd, bd, G, 1e-5, code)
+            assert err.value.status == nt.ERR_EXCHANGE_TIMEOUT
+        finally:
+            nt.clear_wait_timeouts()
+        return out
+
+    for direction, want in ((0, good), (1, good_b)):
+        got = run(direction)
+        if what != 5:
+            assert all(torch.isnan(t.float()).all() for t in got)
+            continue
+        # the CTA's rows: tiles of `tile` rows; the second pass takes them from the last to the first, two stages hold the
+        # last two, so the third from the end is missing, with all before it
+        rows, tile = int(plans[direction]["rows"]), int(plans[direction]["tile"].split("x")[1])
+        tiles = -(-rows // tile)
+        assert tiles >= 4
+        missing = torch.zeros(sp[0] * sp[1], dtype=torch.bool, device="cuda")
+        missing[cta * rows:cta * rows + (tiles - 2) * tile] = True
+        assert torch.isnan(got[0][0, missing].float()).all()
+        assert torch.equal(got[0][0, ~missing], want[0][0, ~missing]) and torch.equal(got[0][1], want[0][1])
+        if direction == 0:
+            assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+        else:  # parameter gradients: those that this CTA adds up
+            lost = torch.isnan(got[1][0])
+            assert lost.any() and torch.equal(got[1][:, ~lost], want[1][:, ~lost])
+    assert nt.wait_timeouts() == 0
+    again = nt.fwd_raw(xd, gd, bd, G, 1e-5, code)
+    assert all(torch.equal(a, b) for a, b in zip(again, good))
