@@ -417,13 +417,13 @@ int gnb200_describe_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, 
     snprintf(text, sizeof(text), "unsupported");
   } else {
     const gnb200::Geom& g = p.geom;
-    if (p.resident) {  // named after the plan whose place the kernel takes
+    if (p.resident) {  // fallback: what runs where the grid cannot be resident
       const gnb200::ResidentGeom& r = p.rgeom;
       snprintf(text, sizeof(text),
-               "%s %s ve=%d cw=%d ncb=1 ty=%d threads=%d rows=%d chunks=%d k=1 persist=1 grid=%lld smem=%zu ws=%zu "
-               "launches=%d resident=1 tile=%dx%d stages=%d",
-               direction == 0 ? "fwd" : "bwd", p.wave ? "wave" : "twopass", p.ve, r.g.C, r.g.TY, r.threads, r.g.rows_per_cta,
-               r.cps, r.grid, r.smem_bytes, p.ws_bytes, p.launches, r.g.C, r.BR, r.stages);
+               "%s resident ve=%d cw=%d ncb=1 ty=%d threads=%d rows=%d chunks=%d k=1 persist=1 grid=%lld smem=%zu ws=%zu "
+               "launches=%d resident=1 fallback=%s tile=%dx%d stages=%d",
+               direction == 0 ? "fwd" : "bwd", p.ve, r.g.C, r.g.TY, r.threads, r.g.rows_per_cta, r.cps, r.grid, r.smem_bytes,
+               p.ws_bytes, p.launches, p.wave ? "wave" : "twopass", r.g.C, r.BR, r.stages);
     } else if (p.wave) {
       const gnb200::WaveGeom& w = p.wgeom;
       snprintf(text, sizeof(text),

@@ -446,8 +446,11 @@ bool plan_wave(const Shape& sh, Plan* out) {
 }
 
 // Resident plan (gn_resident.cu) in place of the multi-kernel or wave plan in *plan.  A sample's rows are cut into
-// cps = 148 / N contiguous ranges, one CTA per SM; at least 85 % of the SMs must get one.  Tiles are 32 KB of x
-// (backward: 16 KB each of x and dy); what is left of the SM's shared memory holds as many of them as fit.
+// cps = 148 / N contiguous ranges of whole rows, one CTA per SM; N * cps must be at least 85 % of the SMs.  Few rows
+// beyond 148 / N fill fewer (149 rows: 75 CTAs of two), and those calls stay here all the same: such short samples are
+// not fused only when a group is very wide, where the multi-kernel plan takes 250 us (its finalize kernel has one CTA per
+// group) and 75 CTAs 22 (1 x 149 x 4096, one group; 1 x 300 x 4096 329 / 23, 1 x 200 x 2048 fp32 176 / 18).  Tiles are
+// 32 KB of x (backward: 16 KB each of x and dy); what is left of the SM's shared memory holds as many of them as fit.
 // The lines: measured on B200, us, resident / the plan it replaces (w wave, m multi-kernel).
 // Backward:
 //   fp16  512@256^2 64.2 / 68.7 w    256@512^2 118 / 129 w    128@1024^2 226 / 242 m    2 x 256@512x256 117 / 125 w
@@ -480,7 +483,7 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   if (cps > sh.R) cps = sh.R;
   if (!forced && sh.N * cps < kSmCount * 85 / 100) return false;
   const int rows = (sh.R + cps - 1) / cps;
-  cps = (sh.R + rows - 1) / rows;
+  cps = (sh.R + rows - 1) / rows;  // ranges of whole rows: 149 rows make 75 CTAs of two rows
   Geom g = {};
   g.N = sh.N, g.R = sh.R, g.C = sh.C, g.G = sh.G, g.D = sh.D;
   g.CW = sh.C, g.CV = CV, g.TY = kResidentThreads / CV;
@@ -526,7 +529,7 @@ static bool plan_streaming(const Shape& sh, bool twopass_only, bool wave_only, P
 
 // Plans a thread has made lately: a plan is a function of these seven numbers alone (no pointer, no device state),
 // and a call asks for it three times - the two alignments of the workspace query, then the launch.  Direct-mapped,
-// 64 entries (30 KB) per thread, so it needs no lock and cannot grow; a colliding problem replaces the entry.  Not
+// 64 entries of about 650 bytes (41 KB) per calling thread, the autograd engine's among them, so it needs no lock and cannot grow; a colliding problem replaces the entry.  Not
 // used while an override is set in the environment.  Measured for one plan: 10 - 25 us searched anew with a getenv
 // per candidate, 1 - 3 us without those, 0.1 us from here.
 struct PlanKey {

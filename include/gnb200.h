@@ -217,8 +217,9 @@ int gnb200_allreduce_param_grads(float* dgamma_dbeta_f32, void* dgamma, void* db
                                  const void* const* peer_bufs, int rank, int world, void* stream);
 
 /*
- * Describes the launch plan chosen for a problem ("fwd fused k=4 cw=64 ..."), for logs, tests
- * and benchmarks.  Writes at most buf_len bytes including the terminating NUL; returns the
+ * Describes the launch plan chosen for a problem ("fwd fused k=4 cw=64 ..."; the plans are fused,
+ * twopass, wave and resident, the last with the plan that takes over where its grid cannot be
+ * resident: "fallback=twopass"), for logs, tests and benchmarks.  Writes at most buf_len bytes including the terminating NUL; returns the
  * number of bytes the full text needs.  direction: 0 = forward, 1 = backward.
  */
 int gnb200_describe_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction,
