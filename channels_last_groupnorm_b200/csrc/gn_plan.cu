@@ -5,10 +5,12 @@
 // up to 8 (16 non-portable) CTAs.
 //
 // Environment overrides (for experiments and benchmarks only):
-//   GNB200_FORCE_PATH = fused | twopass     GNB200_CW = channels per column block
-//   GNB200_K = cluster size                 GNB200_THREADS = target CTA size
-//   GNB200_TILE_KB = shared-memory tile budget per CTA (fused path)
-//   GNB200_ROWS = rows per CTA tile (multi-kernel path)
+//   GNB200_FORCE_PATH = twopass | wave | resident (anything else: as without it)
+//   GNB200_CW = channels per column block   GNB200_K = cluster size       GNB200_THREADS = target CTA size
+//   GNB200_ROWS = rows per CTA tile (multi-kernel path)                   GNB200_PERSIST = 0: one cluster per item
+//   GNB200_NO_SHUF: generic reductions      GNB200_CHAIN = 0: plain stream order between the kernels of a call
+//   GNB200_WAVE_MB, _TEAMS, _CW, _KR, _STAGES, _PAD, _PER_SM, _GRID, _OVERLAP: the wave plan (plan_wave)
+//   GNB200_RESIDENT_CTAS, _STAGES: the resident plan (plan_resident)
 #include <stdlib.h>
 #include <string.h>
 #include <unistd.h>  // environ
@@ -35,12 +37,17 @@ long long gcd_ll(long long a, long long b) {
   return a;
 }
 
-// One walk over the environment tells whether any override is set at all (about 0.1 us; every getenv walks it too,
-// and the search below used to call it some hundred times: 10 - 25 us per plan).  make_plan notes the answer for
-// its own thread, and without overrides no name is looked up.
+// One walk over the environment tells whether any override of the planner is set (about 0.1 us; every getenv walks it
+// too, and the search below used to call it some hundred times: 10 - 25 us per plan).  make_plan notes the answer for its
+// own thread, and without overrides no name is looked up.  What env_int / env_text are asked for must be on this list;
+// other variables of the library (GNB200_WAIT_CLOCKS, GNB200_PEER_LANES) do not concern plans.
+constexpr const char* kOverrides[] = {"FORCE_PATH=", "CW=", "K=", "THREADS=", "ROWS=", "PERSIST=", "NO_SHUF=", "CHAIN=", "WAVE_", "RESIDENT_"};
 bool overrides_present() {
-  for (char** e = environ; e && *e; ++e)
-    if (!strncmp(*e, "GNB200_", 7)) return true;
+  for (char** e = environ; e && *e; ++e) {
+    if (strncmp(*e, "GNB200_", 7)) continue;
+    for (const char* name : kOverrides)
+      if (!strncmp(*e + 7, name, strlen(name))) return true;
+  }
   return false;
 }
 thread_local bool t_overrides = true;
