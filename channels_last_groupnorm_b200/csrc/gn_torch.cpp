@@ -271,6 +271,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> call_fwd(const at::Tensor& X, con
 }
 
 struct GnFunction : torch::autograd::Function<GnFunction> {
+  // everything that backward uses is saved through ctx, and it calls dispatcher ops only: compiled autograd may trace it
+  static constexpr bool is_traceable = true;
+
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias,
                             int64_t G, double eps, int64_t act) {
     const bool cl = is_channels_last(X);

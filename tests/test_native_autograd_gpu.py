@@ -110,3 +110,33 @@ def test_cuda_graph_capture_of_a_training_step():
     torch.cuda.synchronize()
     for a, b in zip(out, step()):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("pdtype", [torch.float16, torch.float32], ids=["typed", "fp32-params"])
+@pytest.mark.parametrize("order", ["last", "first"])
+def test_compiled_autograd_traces_the_backward(order, pdtype):
+    """As it does with a Python function: the node is part of the captured graph, not a call back into eager mode, and the
+    gradients are those of the plain engine, also when a second input has another size."""
+    from torch._dynamo import compiled_autograd
+
+    m = pkg.GN_NHWC(4, 32, activation="silu", device="cuda", dtype=pdtype)
+    graphs = []
+
+    def run(x):
+        m.zero_grad()
+        x = x.clone().requires_grad_(True)
+        (m(x) ** 2).sum().backward()
+        return [x.grad] + [p.grad.clone() for p in m.parameters()]
+
+    def capture(gm):
+        graphs.append(" ".join(str(n.target) for n in gm.graph.nodes))
+        return gm
+
+    for shape in ((2, 32, 6, 6), (3, 32, 5, 7)):
+        x = _tensor(shape, order, torch.float16)
+        want = run(x)
+        for compiler in (capture, torch.compile(backend="aot_eager")):
+            with compiled_autograd._enable(compiler, dynamic=False):
+                got = run(x)
+            assert all(torch.equal(a, b) and a.stride() == b.stride() for a, b in zip(got, want))
+    assert graphs and all("GnFunction" in g and "non_traceable" not in g for g in graphs)
