@@ -175,7 +175,7 @@ class GN_NHWC(nn.GroupNorm):
             w = torch.ones((self.num_channels,), device=x.device, dtype=x.dtype)
             b = torch.zeros((self.num_channels,), device=x.device, dtype=x.dtype)
         if self.process_group is None and _plain_eager(x, w, b):
-            return _group_norm_act(x, w, b, self.num_groups, self.eps, self.act_code)
+            return _group_norm_act(x, w, b, int(self.num_groups), float(self.eps), self.act_code)
         return GN_NHWC_Func.apply(x, w, b, self.num_groups, self.eps, self.act_code, self.process_group)
 
     def extra_repr(self):

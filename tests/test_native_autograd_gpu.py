@@ -140,3 +140,12 @@ def test_compiled_autograd_traces_the_backward(order, pdtype):
                 got = run(x)
             assert all(torch.equal(a, b) and a.stride() == b.stride() for a, b in zip(got, want))
     assert graphs and all("GnFunction" in g and "non_traceable" not in g for g in graphs)
+
+
+def test_num_groups_and_eps_are_converted_as_before():
+    """num_groups from a division and eps as text (a value read from a configuration file) are what int() and float()
+    make of them."""
+    x = _tensor((2, 32, 6, 6), "last", torch.float32)
+    m = pkg.GN_NHWC(32 / 8, 32, eps="1e-5", device="cuda")
+    assert torch.equal(m(x), pkg.GN_NHWC_Func.apply(x, m.weight, m.bias, 32 / 8, "1e-5", 0))
+    assert torch.equal(m(x), pkg.GN_NHWC(4, 32, eps=1e-5, device="cuda")(x))
