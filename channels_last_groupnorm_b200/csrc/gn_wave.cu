@@ -738,10 +738,12 @@ cudaError_t check_resident(const void* func, int threads, size_t smem, long long
   struct Key {
     int dev;
     const void* func;
+    int threads;  // the resident plan's CTAs are not all of one size
     size_t smem;
     bool operator<(const Key& o) const {
       if (dev != o.dev) return dev < o.dev;
       if (func != o.func) return func < o.func;
+      if (threads != o.threads) return threads < o.threads;
       return smem < o.smem;
     }
   };
@@ -751,7 +753,7 @@ cudaError_t check_resident(const void* func, int threads, size_t smem, long long
   cudaError_t err = cudaGetDevice(&dev);
   if (err != cudaSuccess) return err;
   std::lock_guard<std::mutex> lock(mu);
-  const Key key = {dev, func, smem};
+  const Key key = {dev, func, threads, smem};
   auto it = cache.find(key);
   if (it == cache.end()) {
     int per_sm = 0, sms = 0;
