@@ -141,3 +141,48 @@ def test_waits_that_run_out_leave_nan_and_a_status(nt, what, dt, act, monkeypatc
     assert nt.wait_timeouts() == 0
     again = nt.fwd_raw(xd, gd, bd, G, 1e-5, code)
     assert all(torch.equal(a, b) for a, b in zip(again, good))
+
+
+def test_peer_entry_points_with_one_rank_after_the_resident_backward(nt, monkeypatch):
+    """The exchange of the parameter gradients follows the resident kernel as it follows the wave kernel: with one rank
+    the results are those of the plain call.  (Several ranks need one GPU each: tests/test_peer_multigpu.py, bench.py.)"""
+    from .test_parity_gpu import _flat
+
+    monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
+    N, C, sp, G, act = 2, 64, (40, 41), 8, O.ACT_CODES["gelu"]
+    x, ga, be, dy = O.make_inputs(N, C, sp, torch.bfloat16, seed=41)
+    xd, dyd, gd, bd = _flat(x.cuda()), _flat(dy.cuda()), ga.cuda(), be.cuda()
+    _, mean, rstd = nt.fwd_raw(xd, gd, bd, G, 1e-5, act)
+    want = nt.bwd_raw(dyd, xd, gd, bd, mean, rstd, G, act)
+    buf = torch.zeros(nt.peer_exchange_bytes(C, 1) // 4, device="cuda")
+    for collect in (True, False):
+        dx, dparam = nt.bwd_peer_raw(dyd, xd, gd, bd, mean, rstd, G, act, [buf.data_ptr()], 0, collect=collect)
+        assert torch.equal(dx, want[0]) and torch.equal(dparam, want[1])
+    torch.cuda.synchronize()
+    assert int(buf.abs().sum().item()) == 0 and nt.wait_timeouts() == 0
+
+
+def test_resident_plan_in_a_captured_graph(nt):
+    """Unforced, both directions: one memset node and one cooperative kernel each; replays see new inputs."""
+    N, R, C, G = 1, 98304, 256, 8
+    x, dy = (torch.randn(N, R, C, device="cuda", dtype=torch.float16) for _ in range(2))
+    ga, be = torch.ones(C, device="cuda", dtype=torch.float16), torch.zeros(C, device="cuda", dtype=torch.float16)
+    for d in (0, 1):
+        assert " resident " in nt.describe_plan(N, R, C, G, torch.float16, d)
+
+    def step():
+        y, mean, rstd = nt.fwd_raw(x, ga, be, G, 1e-5, 2)
+        return (y, mean, rstd) + nt.bwd_raw(dy, x, ga, be, mean, rstd, G, 2)
+
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        step()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        out = step()
+    x.mul_(0.5).add_(1.0)
+    g.replay()
+    g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(out, step())) and nt.wait_timeouts() == 0
