@@ -488,14 +488,16 @@ NchwGeom make_geom(long long N, long long R, long long C, long long G, int ve) {
   g.row_vecs = R / ve;
   g.div_R = fast_div(R);
   g.evict = (double)N * C * R * (16 / ve) > 32.0 * 1024 * 1024;  // (single elements are stored plainly)
-  // forward: sixteen chunks per SM, at least 2048 vectors (32 KB; single elements: 4096) each.  Several waves of CTAs
+  // forward: sixteen chunks per SM, at least 2048 vectors (32 KB) each, or 4096 single elements where that still gives every
+  // SM a chunk (3 x 40@17x33 fp32, 24 slabs of 2805: 5.8 us in two chunks each, 7.1 in one).  Several waves of CTAs
   // even out the SMs and let the reverse order of the output pass work across CTAs too: with four chunks per SM (all in
   // flight at once) 39.3 us at 512@256^2 fp16, 90 us at 2 x 256@256^2 fp32, 113 us at 3 x 128@300x301 bf16; with sixteen
   // 36.1, 75.9, 76.2.  What does not fill a batch of kUnroll vectors per thread goes vector by vector, so chunks are whole
   // batches where that saves steps (2 x 32@300x200 fp32 18.1 -> 15.5, 64 x 64@112^2 bf16 with chunks of 1568 vectors 61.9
   // -> 56.8, 4 x 512@33^2 12.3 -> 10.9 and with 4096 elements 10.5, 16 x 1024@14^2 18.4 -> 16.7 and 14.7) and of equal
   // length elsewhere (640@32^2: twice 1280 vectors 5.8, 2048 and 512 6.1).
-  const long long slabs = N * G, fwd_batch = kUnroll * kThreads, min_chunk = ve == 1 ? 4096 : 2048;
+  const long long slabs = N * G, fwd_batch = kUnroll * kThreads;
+  const long long min_chunk = ve == 1 && slabs * ((g.slab_vecs + 4095) / 4096) >= kSmCount ? 4096 : 2048;
   long long chunks = (16LL * kSmCount + slabs - 1) / slabs;
   const long long max_chunks = (g.slab_vecs + min_chunk - 1) / min_chunk;
   if (chunks > max_chunks) chunks = max_chunks;
@@ -510,8 +512,11 @@ NchwGeom make_geom(long long N, long long R, long long C, long long G, int ve) {
   // 16, 71.9 with 64, 70.8 with 96, 71.6 with 128: 320 CTAs of the first kind lie three on some SMs and two on the others;
   // 2 x 256@256^2 fp32 133 / 127 / 120 / 124), up to 2048 vectors per piece and at least 128, or 256 where that still makes 28
   // warps per SM: a piece of 128 is one batch of loads and nothing to hide them behind (8 x 256@64^2 bf16 22.5 / 21.3,
-  // 8 x 256@48^2 17.8 / 16.8, but 4 x 320@96^2, 1280 rows, 28.4 / 32.3).
-  const long long rows = N * C, bwd_batch = kUnroll * 32, min_piece = rows >= 2048 ? 2 * bwd_batch : bwd_batch;
+  // 8 x 256@48^2 17.8 / 16.8, but 4 x 320@96^2, 1280 rows, 28.4 / 32.3).  Of single elements such a batch is a few hundred
+  // bytes, and 16 warps per SM of the longer pieces do (320@63^2 13.5 / 11.5, 640@31^2 9.9 / 9.2; not 128@33x31 7.7 / 9.1).
+  const long long rows = N * C, bwd_batch = kUnroll * 32, twice = 2 * bwd_batch;
+  const bool longer = rows >= 2048 || (ve == 1 && rows * ((g.row_vecs + twice - 1) / twice) >= 16 * kSmCount);
+  const long long min_piece = longer ? twice : bwd_batch;
   long long ppr = (96LL * kSmCount + rows - 1) / rows;
   const long long max_ppr = (g.row_vecs + min_piece - 1) / min_piece;
   if (ppr > max_ppr) ppr = max_ppr;
