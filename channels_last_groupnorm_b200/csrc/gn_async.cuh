@@ -43,6 +43,49 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
 }
 #define kNaN __int_as_float(0x7fc00000)
 
+// ---------------------------------------------------------------------------------------------
+// Tensor memory as storage.  No matrix instruction runs here, so an SM's 256 KB of tensor memory are free to hold rows
+// between two passes: 512 columns of 128 lanes x 4 bytes.  A warp reaches the 32 lanes of its rank in its warpgroup, so
+// the warpgroups of a CTA share the columns out and a thread has kTmemColumns words of its own, i.e. 32 vectors of 16
+// bytes that nobody else touches: a store and the load that gets it back need no barrier, only wait::st.
+// ---------------------------------------------------------------------------------------------
+constexpr int kTmemColumns = 128;                  // per warpgroup, hence words per thread
+constexpr uint32_t kTmemTotal = 4 * kTmemColumns;  // all of the SM's
+
+// by one whole warp; the base address is valid for the CTA's threads after their next __syncthreads
+__device__ __forceinline__ void tmem_alloc(uint32_t* smem_slot) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(smem_slot)), "r"(kTmemTotal)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+// by the same warp, when every thread of the CTA is done with its words
+__device__ __forceinline__ void tmem_free(uint32_t base) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(kTmemTotal) : "memory");
+}
+// the calling thread's first word: lane in bits 31..16, column below
+__device__ __forceinline__ uint32_t tmem_own(uint32_t base, int warp) {
+  return base + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * kTmemColumns;
+}
+// 16 words from column `col` of the thread's own on; whole converged warps
+__device__ __forceinline__ void tmem_store16(uint32_t col, const uint4& a, const uint4& b, const uint4& c, const uint4& d) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(col),
+      "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w),
+      "r"(d.x), "r"(d.y), "r"(d.z), "r"(d.w)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// the same 16 words back; load and wait are one statement, so that no use of them moves in between
+__device__ __forceinline__ void tmem_load16(uint32_t col, uint4& a, uint4& b, uint4& c, uint4& d) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w), "=r"(c.x), "=r"(c.y), "=r"(c.z),
+        "=r"(c.w), "=r"(d.x), "=r"(d.y), "=r"(d.z), "=r"(d.w)
+      : "r"(col)
+      : "memory");
+}
+
 // mbarrier waits of the streaming kernels.  `gave_up` is the CTA's shared flag: the first wait that runs
 // out sets it (and poisons the results, see the callers); from then on no wait of this CTA spends
 // its limit again, so a broken run ends after about one limit instead of one limit per stage.

@@ -703,12 +703,14 @@ struct WaveGeom {
 constexpr int kResidentThreads = 512;
 // rows per thread and tile: 32 KB of x, or 16 KB each of x and dy
 __host__ __device__ constexpr int resident_rows(int direction) { return direction == 0 ? 4 : 2; }
+constexpr int kResidentPark = 8;  // tiles that tensor memory holds: 128 words a thread, 16 of them per tile
 struct ResidentGeom {
   Geom g;              // CW = C, ncb = 1, slots = G; rows_per_cta, chunks = cps
   int cps;             // CTAs per sample
   int BR;              // rows per tile (resident_rows * TY)
   int tile_bytes;      // BR * C * sizeof(T), one tensor
   int stages;
+  int park;            // tiles of a range that are kept in tensor memory besides those in the stages
   int threads;
   long long grid;      // N * cps
   size_t smem_bytes;

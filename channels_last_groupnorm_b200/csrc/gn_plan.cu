@@ -10,7 +10,7 @@
 //   GNB200_ROWS = rows per CTA tile (multi-kernel path)                   GNB200_PERSIST = 0: one cluster per item
 //   GNB200_NO_SHUF: generic reductions      GNB200_CHAIN = 0: plain stream order between the kernels of a call
 //   GNB200_WAVE_MB, _TEAMS, _CW, _KR, _STAGES, _PAD, _PER_SM, _GRID, _OVERLAP: the wave plan (plan_wave)
-//   GNB200_RESIDENT_CTAS, _STAGES: the resident plan (plan_resident)
+//   GNB200_RESIDENT_CTAS, _STAGES, _PARK: the resident plan (plan_resident)
 #include <stdlib.h>
 #include <string.h>
 #include <unistd.h>  // environ
@@ -472,7 +472,7 @@ bool plan_wave(const Shape& sh, Plan* out) {
 //   bf16  128@300x1000 45.4 / 48.5    and as calls among others 73.2 / 76.2 (256@512^2, with allocation)
 //   not there: 2 x 256@512x256 74.2 / 73.7    3 x 512@200x300 101 / 98    fp32 256@512^2 152 / 150
 //              one group: 8 x 1024@64^2 43 / 37    4 MB, one group 16.5 / 8.8
-// GNB200_RESIDENT_CTAS / _STAGES (tests, experiments) bound the CTAs per sample and the stages.
+// GNB200_RESIDENT_CTAS / _STAGES / _PARK (tests, experiments) bound the CTAs per sample, the stages and the tiles in tensor memory.
 bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   const int ve = sh.ve, s = sh.s;
   if (ve == 1 || sh.N > kSmCount) return false;
@@ -516,6 +516,9 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   const int max_stages = env_int("GNB200_RESIDENT_STAGES", 16);
   if (r.stages > max_stages) r.stages = max_stages < 2 ? 2 : max_stages;
   if (r.stages > 16) r.stages = 16;
+  // GNB200_RESIDENT_STAGES alone bounds what stays on chip
+  r.park = env_int("GNB200_RESIDENT_PARK", max_stages < 16 ? 0 : kResidentPark);
+  if (r.park < 0 || r.park > kResidentPark) r.park = kResidentPark;
   r.smem_bytes = fixed + (size_t)r.stages * stage;
   r.ws_bytes = resident_workspace_bytes(r, sh.direction);
   // The scratch limits of callers stay what they are: a call never asks for less than the plan that this one

@@ -7,11 +7,15 @@
 //
 //   pass 1   the range streams through a ring of shared-memory stages (untiled cp.async.bulk copies: whole rows are
 //            one contiguous run, so no thread computes an address and no tensor map is needed); the last `stages`
-//            tiles are not overwritten: 148 x 192 KB, 28 MB, stay on chip
+//            tiles are not overwritten, and the eight before them are parked in tensor memory as they pass through:
+//            148 x (192 + 256) KB, 67 MB, stay on chip
 //   barrier  partial sums to scratch, one arrival per CTA, bounded wait; every CTA merges what it needs
-//   pass 2   the resident tiles first - no read at all - and, as their stages become free, the tiles before them
-//            in reverse order, so that what was read last (and L2 still holds) is read first; results leave with
-//            streaming (evict-first) stores
+//   pass 2   the resident tiles first - no read at all; those in the stages before those in tensor memory, so that the
+//            stages fill again early - and then the tiles before them in reverse order, so that what was read last (and
+//            L2 still holds) is read first; results leave with streaming (evict-first) stores
+//
+// What the tensor memory gave (fp16 SiLU, calls among others): forward 256@512^2 74.1 -> 71.8 us, forward and backward
+// of 128@1024^2 375 -> 369.
 //
 // dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.
 // Measured against the plans it replaces: see the rule in gn_plan.cu.
@@ -53,7 +57,7 @@ struct Smem {
   uint32_t stage0;
   uint64_t* full;
   uint64_t* empty;
-  int* flags;  // [0] a wait gave up
+  int* flags;  // [0] a wait gave up, [1] tensor-memory address
   float* red;
 };
 template <int NT>
@@ -106,6 +110,28 @@ struct Stream {
     for (int s = 0; s < stages; ++s)
       if (!mbar_wait_bounded(&sm.full[s], (last_ph >> s) & 1u, lim)) return;
   }
+
+  // Where the tiles of the range are between the passes: [0, held0) must be read again, [held0, held0 + parked) are in
+  // tensor memory, the last `stages` of them in the stages.
+  int parked, held0;
+  uint32_t tmem;  // the thread's first word
+
+  // Pass 2 takes the tiles that pass through the stages as items 0, 1, ...: those held there newest first, then the
+  // others in reverse order.  Item i lies in the i-th stage before the last tile's.
+  int next, next_stage;  // thread 0: the item to be copied next, and its stage
+  __device__ __forceinline__ int items() const { return tiles - parked; }
+  __device__ __forceinline__ int tile_of(int item) const { return tiles - 1 - item - (item < stages ? 0 : parked); }
+  __device__ __forceinline__ void start_pass2(int last_stage) {
+    next = stages;
+    next_stage = last_stage;
+  }
+  // thread 0, once item `done` has been read: the item that takes its stage
+  __device__ __forceinline__ void refill_behind(int done, const ResidentGeom& r) {
+    if (done + stages < next || next >= items()) return;
+    refill(tile_of(next), next_stage, r.g.wait, next == stages && test_at(r, kDebugNoSecondCopy));
+    ++next;
+    next_stage = next_stage == 0 ? stages - 1 : next_stage - 1;
+  }
 };
 
 template <typename T, int NT>
@@ -119,6 +145,11 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
   st.tile_bytes = (uint32_t)r.tile_bytes;
   st.full_ph = st.empty_ph = 0;
   st.last_ph = ~0u;
+  st.parked = max(0, min(r.park, st.tiles - r.stages));
+  st.held0 = max(0, st.tiles - r.stages - st.parked);
+  const int alloc_warp = 1 % (int)(blockDim.x >> 5);  // not the one that issues the copies, where there is another
+  __syncwarp();
+  if (st.parked && (int)(threadIdx.x >> 5) == alloc_warp) tmem_alloc(reinterpret_cast<uint32_t*>(&sm.flags[1]));
   if (threadIdx.x == 0) {
     for (int s = 0; s < r.stages; ++s) {
       mbar_init(&sm.full[s], 1);
@@ -128,7 +159,17 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
     fence_mbar_init_cluster();
     for (int t = test_at(r, kDebugNoFirstCopy) ? 1 : 0; t < min(r.stages, st.tiles); ++t) st.issue(t, t);
   }
+  __syncwarp();
   __syncthreads();
+  st.tmem = st.parked ? tmem_own(*(volatile uint32_t*)&sm.flags[1], threadIdx.x >> 5) : 0u;
+}
+template <typename T, int NT>
+__device__ __forceinline__ void stream_end(Stream<T, NT>& st, const WaitLimit& lim) {
+  if (threadIdx.x == 0) st.drain(lim);
+  if (!st.parked) return;
+  __syncwarp();
+  __syncthreads();
+  if ((int)(threadIdx.x >> 5) == 1 % (int)(blockDim.x >> 5)) tmem_free(*(volatile uint32_t*)&st.sm.flags[1]);
 }
 
 // Grid barrier: every CTA has written its partial sums.  `count` starts at 0 (cleared in stream order before the
@@ -246,6 +287,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       uint4 w[KR];
 #pragma unroll
       for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
+      if (t >= st.held0 && t < T_ - S) tmem_store16(st.tmem + (t - st.held0) * 16, w[0], w[1], w[2], w[3]);
       if constexpr (kShifted) {
         if (t == t0) {
           float f0[VE];
@@ -325,16 +367,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   if (streaming) lane_affine<T, VE, UNI>(gamma, beta, stat, stat + g.slots, 0, tx * VE, g.div_D, a, b);
   T* out = y + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
   const size_t ostep = (size_t)g.TY * g.C;
-  stage = prev;  // of the last tile
-  int t = ok ? T_ - 1 : -1;
-  for (; t >= 0; --t) {
-    if (t < T_ - S && !st.wait_full(stage, g.wait)) break;
-    const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
+  // one tile's vectors of the thread, wherever they were kept
+  auto emit = [&](int t, const uint4 (&w)[KR]) {
     const int here = nrows - t * st.BR;
     T* o = out + (size_t)t * st.BR * g.C;
-    uint4 w[KR];
-#pragma unroll
-    for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
 #pragma unroll
     for (int u = 0; u < KR; ++u) {
       if (my_row + u * g.TY < here) {
@@ -345,15 +381,38 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
         stg128_stream(o + (size_t)u * ostep, act_pack16<T, VE, ACT>(f));
       }
     }
-    if (t >= S) release_stage(&sm.empty[stage], lane);
-    if (tid == 0 && t + 1 < T_ && t + 1 >= S)
-      st.refill(t + 1 - S, prev, g.wait, t == T_ - 2 && test_at(r, kDebugNoSecondCopy));
-    prev = stage;
+  };
+  stage = prev;  // of the last tile
+  st.start_pass2(stage);
+  int lost = ok ? -1 : T_ - 1;  // the rows of the tiles up to this one are not known
+  for (int i = 0; ok; ++i) {
+    if (i == S && st.parked) {  // the stages fill again meanwhile
+      tmem_store_wait();
+      for (int p = st.parked - 1; p >= 0; --p) {
+        uint4 w[KR];
+        __syncwarp();
+        tmem_load16(st.tmem + p * 16, w[0], w[1], w[2], w[3]);
+        emit(st.held0 + p, w);
+        if (tid == 0) st.refill_behind(S - 1, r);
+      }
+    }
+    if (i >= st.items()) break;
+    const int t = st.tile_of(i);
+    if (i >= S && !st.wait_full(stage, g.wait)) {
+      lost = t;
+      break;
+    }
+    const uint32_t base = my_off + (uint32_t)stage * st.tile_bytes;
+    uint4 w[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) w[u] = lds128(base + u * step);
+    emit(t, w);
+    if (i + S < st.items()) release_stage(&sm.empty[stage], lane);
+    if (tid == 0 && i > 0) st.refill_behind(i - 1, r);
     stage = stage == 0 ? S - 1 : stage - 1;
   }
-  if (!ok) t = T_ - 1;
-  store_nan_rows(out, (size_t)g.C * sizeof(T), my_row, g.TY, min(nrows, (t + 1) * st.BR));  // none, unless a wait gave up
-  if (tid == 0) st.drain(g.wait);
+  store_nan_rows(out, (size_t)g.C * sizeof(T), my_row, g.TY, min(nrows, (lost + 1) * st.BR));  // none, unless a wait gave up
+  stream_end(st, g.wait);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -426,6 +485,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
         xw[u] = lds128(base + u * step);
         dw[u] = lds128(base + st.tile_bytes + u * step);
       }
+      if (t >= st.held0 && t < T_ - S) tmem_store16(st.tmem + (t - st.held0) * 16, xw[0], xw[1], dw[0], dw[1]);
 #pragma unroll
       for (int u = 0; u < KR; ++u) {
         if (my_row + u * g.TY < here) {
@@ -524,19 +584,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   }
   T* out = dx + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
   const size_t ostep = (size_t)g.TY * g.C;
-  stage = prev;
-  int t = ok ? T_ - 1 : -1;
-  for (; t >= 0; --t) {
-    if (t < T_ - S && !st.wait_full(stage, g.wait)) break;
-    const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
+  auto emit = [&](int t, const uint4 (&xw)[KR], const uint4 (&dw)[KR]) {
     const int here = nrows - t * st.BR;
     T* o = out + (size_t)t * st.BR * g.C;
-    uint4 xw[KR], dw[KR];
-#pragma unroll
-    for (int u = 0; u < KR; ++u) {
-      xw[u] = lds128(base + u * step);
-      dw[u] = lds128(base + st.tile_bytes + u * step);
-    }
 #pragma unroll
     for (int u = 0; u < KR; ++u) {
       if (my_row + u * g.TY < here) {
@@ -558,19 +608,44 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
         }
       }
     }
-    if (t >= S) release_stage(&sm.empty[stage], lane);
-    if (tid == 0 && t + 1 < T_ && t + 1 >= S)
-      st.refill(t + 1 - S, prev, g.wait, t == T_ - 2 && test_at(r, kDebugNoSecondCopy));
-    prev = stage;
+  };
+  stage = prev;
+  st.start_pass2(stage);
+  int lost = ok ? -1 : T_ - 1;
+  for (int i = 0; ok; ++i) {
+    if (i == S && st.parked) {
+      tmem_store_wait();
+      for (int p = st.parked - 1; p >= 0; --p) {
+        uint4 xw[KR], dw[KR];
+        __syncwarp();
+        tmem_load16(st.tmem + p * 16, xw[0], xw[1], dw[0], dw[1]);
+        emit(st.held0 + p, xw, dw);
+        if (tid == 0) st.refill_behind(S - 1, r);
+      }
+    }
+    if (i >= st.items()) break;
+    const int t = st.tile_of(i);
+    if (i >= S && !st.wait_full(stage, g.wait)) {
+      lost = t;
+      break;
+    }
+    const uint32_t base = my_off + (uint32_t)(2 * stage) * st.tile_bytes;
+    uint4 xw[KR], dw[KR];
+#pragma unroll
+    for (int u = 0; u < KR; ++u) {
+      xw[u] = lds128(base + u * step);
+      dw[u] = lds128(base + st.tile_bytes + u * step);
+    }
+    emit(t, xw, dw);
+    if (i + S < st.items()) release_stage(&sm.empty[stage], lane);
+    if (tid == 0 && i > 0) st.refill_behind(i - 1, r);
     stage = stage == 0 ? S - 1 : stage - 1;
   }
-  if (!ok) t = T_ - 1;
-  store_nan_rows(out, (size_t)g.C * sizeof(T), my_row, g.TY, min(nrows, (t + 1) * st.BR));  // none, unless a wait gave up
+  store_nan_rows(out, (size_t)g.C * sizeof(T), my_row, g.TY, min(nrows, (lost + 1) * st.BR));  // none, unless a wait gave up
 
   // ---- dgamma / dbeta: the grid's warps share the channels; all channel sums are visible since the barrier
   const int rows = g.N * r.cps;
   const bool bad = *(volatile int*)&sm.flags[0] != 0;
-  if (tid == 0) st.drain(g.wait);
   for (int c = (int)blockIdx.x + (int)gridDim.x * warp; c < g.C; c += (int)gridDim.x * nwarps) {
     float t1 = 0.f, t2 = 0.f;
     for (int i0 = lane; i0 < rows + lane; i0 += 32 * kMergeLoads) {
@@ -593,6 +668,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       if (dbeta) dbeta[c] = store_param<T>(t1);
     }
   }
+  stream_end(st, g.wait);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -1,0 +1,41 @@
+"""GPU tests of the tiles that the resident plan keeps in tensor memory (csrc/gn_resident.cu): where a tile waits between
+the passes must not change a bit, whatever its row remainder, the number of stages or the number of parked tiles."""
+import pytest
+import torch
+
+from oracle import gn_oracle as O
+
+from .test_parity_gpu import DT, check_against, run_cabi
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # (N, C, spatial, G, dtype, act, CTAs per sample): tiles of 128 / 64 rows at C = 128 (fp16) and so on
+    (1, 128, (128, 9), 32, "float16", "silu", 1),       # forward: 9 tiles of 128 rows, backward: 18 of 64
+    (1, 128, (1281, 1), 32, "bfloat16", "gelu", 1),     # one row beyond a whole tile
+    (2, 320, (33, 47), 32, "float16", "silu", 3),       # D = 10; 480 of 512 threads, fifteen warps
+    (1, 128, (40, 57), 32, "float32", "gelu_tanh", 3),  # fp32
+    (1, 4096, (7, 11), 1, "float16", "relu", 1),        # one row lane
+    (1, 1536, (61, 1), 4, "bfloat16", "identity", 1),   # two row lanes of 192 threads: twelve warps
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "%dx%dx%s-g%d-%s-%s-%d" % (c[0], c[1], "x".join(map(str, c[2])), *c[3:]))
+def test_parked_tiles_change_no_bit(case, monkeypatch):
+    from channels_last_groupnorm_b200 import _native as nt
+
+    N, C, sp, G, dt, act, ctas = case
+    monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
+    monkeypatch.setenv("GNB200_RESIDENT_CTAS", str(ctas))
+    x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=5, x_dist="uniform3")
+    want = None
+    for stages, park in ((2, 0), (2, 1), (2, 8), (3, 7), (5, 4), (16, 8)):
+        monkeypatch.setenv("GNB200_RESIDENT_STAGES", str(stages))
+        monkeypatch.setenv("GNB200_RESIDENT_PARK", str(park))
+        out = run_cabi(nt, x, ga, be, dy, G, 1e-5, act)
+        if want is None:
+            want = out
+            check_against(out, O.oracle_c(x, ga, be, dy, G, 1e-5, act, threads=4), DT[dt])
+        for k in ("y", "dx", "dparam", "mean", "rstd"):
+            assert torch.equal(out[k], want[k]), (k, stages, park)
+    assert nt.wait_timeouts() == 0
