@@ -108,6 +108,12 @@ __device__ __forceinline__ bool consumer_wait(uint64_t* bar, unsigned parity, vo
   return __all_sync(0xffffffffu, mbar_try_wait(bar, parity));
 }
 
+// untiled bulk copy: both addresses and the size are multiples of 16
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar))
+               : "memory");
+}
 // dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half
 // precision, dx = ag * dyh + c1 * x + c2.
 template <typename T, int ACT>

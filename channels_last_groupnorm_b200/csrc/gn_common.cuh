@@ -697,6 +697,13 @@ struct WaveGeom {
   unsigned long long* trace;  // optional timeline buffer (tuning aid), else null
 };
 
+// Layout of the reductions of gn_reduce.cuh: 2^part_shift neighbouring threads share a group's sum, the scratch has
+// rows of `stride` (odd) floats, div_W divides by the entries that a group has in such a row.
+struct ReduceGeom {
+  int part_shift, stride;
+  FastDiv div_W;
+};
+
 // Geometry of the resident plan (gn_resident.cu): one CTA per SM; every sample's rows are cut into `cps`
 // contiguous row ranges, and a CTA streams its range - whole rows, hence one contiguous run of memory - in
 // tiles of BR rows through a ring of `stages` shared-memory stages.
@@ -706,6 +713,7 @@ __host__ __device__ constexpr int resident_rows(int direction) { return directio
 constexpr int kResidentPark = 8;  // tiles that tensor memory holds: 128 words a thread, 16 of them per tile
 struct ResidentGeom {
   Geom g;              // CW = C, ncb = 1, slots = G; rows_per_cta, chunks = cps
+  ReduceGeom ex;
   int cps;             // CTAs per sample
   int BR;              // rows per tile (resident_rows * TY)
   int tile_bytes;      // BR * C * sizeof(T), one tensor

@@ -212,6 +212,35 @@ __device__ __forceinline__ void lane_setup(const T* gamma, const T* beta, const 
   }
 }
 
+// The same in two steps, loads and arithmetic, for kernels that have something to start in between.
+template <typename T, int VE, bool UNI>
+struct LaneParams {
+  static_assert(sizeof(T) * VE == 16, "16-byte vectors only");
+  static constexpr int NS = UNI ? 1 : VE;
+  uint4 ga, be;
+  float mean[NS], rstd[NS];
+  __device__ __forceinline__ void load(const T* gamma, const T* beta, const float* mean_n, const float* rstd_n, int c_first,
+                                       const FastDiv div_D) {
+    ga = *reinterpret_cast<const uint4*>(gamma + c_first);
+    be = *reinterpret_cast<const uint4*>(beta + c_first);
+#pragma unroll
+    for (int e = 0; e < NS; ++e) {
+      const int grp = div_D.div(c_first + e);
+      mean[e] = mean_n[grp];
+      rstd[e] = rstd_n[grp];
+    }
+  }
+  __device__ __forceinline__ void unpack(BwdLane<T, VE>& L) const {
+    unpack16<T, VE>(ga, L.ga);
+    unpack16<T, VE>(be, L.be);
+#pragma unroll
+    for (int e = 0; e < VE; ++e) {
+      L.r[e] = rstd[UNI ? 0 : e];
+      L.nmr[e] = -mean[UNI ? 0 : e] * L.r[e];
+    }
+  }
+};
+
 // One row of phase 1: dyh = dy * act'(yh) for the thread's VE channels, sums updated.
 template <typename T, int VE, int ACT>
 __device__ __forceinline__ void bwd_row_sums(const float (&fx)[VE], float (&fd)[VE], const BwdLane<T, VE>& L,

@@ -5,7 +5,8 @@
 // up to 8 (16 non-portable) CTAs.
 //
 // Environment overrides (for experiments and benchmarks only):
-//   GNB200_FORCE_PATH = twopass | wave | resident (anything else: as without it)
+//   GNB200_FORCE_PATH = twopass | wave | resident | streaming: whichever of them there would be without the fused plan
+//                       (anything else: as without it)
 //   GNB200_CW = channels per column block   GNB200_K = cluster size       GNB200_THREADS = target CTA size
 //   GNB200_ROWS = rows per CTA tile (multi-kernel path)                   GNB200_PERSIST = 0: one cluster per item
 //   GNB200_NO_SHUF: generic reductions      GNB200_CHAIN = 0: plain stream order between the kernels of a call
@@ -452,6 +453,19 @@ bool plan_wave(const Shape& sh, Plan* out) {
   return true;
 }
 
+// Layout of the reductions in gn_reduce.cuh for `threads` threads; returns the floats of their scratch: the row lanes' values
+// (forward where vectors lie in one group: a mean and an M2 per vector, else one value per channel), later the warps' sums
+// of a merge.
+int reduce_layout(const Shape& sh, int CV, int TY, int threads, ReduceGeom* ex) {
+  const bool per_vector = sh.direction == 0 && sh.D % sh.ve == 0;
+  ex->stride = (per_vector ? CV : sh.C) | 1;
+  ex->div_W = make_fast_div(per_vector ? sh.D / sh.ve : sh.D);
+  ex->part_shift = 0;
+  while (ex->part_shift < 5 && (sh.G << (ex->part_shift + 1)) <= threads) ++ex->part_shift;
+  const int rows = TY * ex->stride * (per_vector ? 2 : 1), merge = 2 * (threads / 32) * sh.G;
+  return rows > merge ? rows : merge;
+}
+
 // Resident plan (gn_resident.cu) in place of the multi-kernel or wave plan in *plan.  A sample's rows are cut into
 // cps = 148 / N contiguous ranges of whole rows, one CTA per SM; N * cps must be at least 85 % of the SMs.  Few rows
 // beyond 148 / N fill fewer (149 rows: 75 CTAs of two), and those calls stay here all the same: such short samples are
@@ -496,8 +510,7 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   g.CW = sh.C, g.CV = CV, g.TY = kResidentThreads / CV;
   g.ncb = 1, g.rows_per_cta = rows, g.chunks = cps, g.slots = sh.G, g.k = 1;
   g.persist = 1, g.skip_push_rank = -1;
-  g.red_floats = g.TY * sh.C;  // reductions over the row lanes; later the warps' sums of a merge
-  if (g.red_floats < 2 * (kResidentThreads / 32) * sh.G) g.red_floats = 2 * (kResidentThreads / 32) * sh.G;
+  g.red_floats = reduce_layout(sh, CV, g.TY, round_up(CV * g.TY, 32), &r.ex);
   g.div_D = make_fast_div(sh.D);
   g.div_CV = make_fast_div(CV);
   g.div_CW = make_fast_div(sh.C);
@@ -605,7 +618,8 @@ static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
   const char* force = env_text("GNB200_FORCE_PATH");
   const bool twopass_only = force && !strcmp(force, "twopass");
   const bool wave_only = force && !strcmp(force, "wave"), resident_only = force && !strcmp(force, "resident");
-  if (!twopass_only && !wave_only && !resident_only && plan_fused(sh, plan)) return true;
+  const bool streaming_only = force && !strcmp(force, "streaming");
+  if (!twopass_only && !wave_only && !resident_only && !streaming_only && plan_fused(sh, plan)) return true;
   if (!plan_streaming(sh, twopass_only, wave_only, plan)) return false;
   if (!twopass_only && !wave_only) plan_resident(sh, resident_only, plan);
   return true;

@@ -14,8 +14,8 @@
 //            stages fill again early - and then the tiles before them in reverse order, so that what was read last (and
 //            L2 still holds) is read first; results leave with streaming (evict-first) stores
 //
-// What the tensor memory gave (fp16 SiLU, calls among others): forward 256@512^2 74.1 -> 71.8 us, forward and backward
-// of 128@1024^2 375 -> 369.
+// What the tensor memory gave (fp16 SiLU, calls among others): forward 256@512^2 74.0 -> 71.7 us; reductions of all groups
+// at once and parameters asked for early: 71.7 -> 70.2, and 128@1024^2 forward + backward 368 -> 356.5.
 //
 // dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.
 // Measured against the plans it replaces: see the rule in gn_plan.cu.
@@ -25,6 +25,7 @@
 #include "gn_async.cuh"
 #include "gn_kernels.h"
 #include "gn_math.cuh"
+#include "gn_reduce.cuh"
 
 namespace gnb200 {
 
@@ -32,7 +33,6 @@ namespace {
 
 constexpr int kMaxStages = 16;
 constexpr int kMergeLoads = 5;   // channel-sum rows a lane has in flight in the dgamma / dbeta sums
-constexpr int kMergeRows = 10;   // partial rows a warp has in flight in a merge (148 CTAs / 16 warps)
 
 // A thread's sums run over at most this many rows before they are merged into the totals: its whole range is
 // R / 148 / TY rows - 111 at 256@512^2, 3543 at 128@4096^2 - where the multi-kernel plan has 55 to 128 per tile, and
@@ -40,12 +40,6 @@ constexpr int kMergeRows = 10;   // partial rows a warp has in flight in a merge
 // multi-kernel plan / whole range / pieces of 128 / of 32: 256@512^2 5e-6 / 1.9e-5 / 1.9e-5 / 2e-6, 128@1024^2 1.5e-5 /
 // 6.6e-5 / 2.2e-5 / 3e-6, 128 x 2^23 rows 1.3e-5 / 9e-4 / 1.2e-5 / 1.7e-6; the time does not change (337 MB 175 us either way).
 constexpr int kFoldRows = 32;
-
-__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
 
 // tests only: this CTA is the one that goes wrong in that way
 __device__ __forceinline__ bool test_at(const ResidentGeom& r, int what) {
@@ -205,33 +199,6 @@ __device__ __forceinline__ void store_nan_rows(void* first, size_t row_bytes, in
     stg128_stream(static_cast<char*>(first) + (size_t)(i - my_row) * row_bytes, make_uint4(~0u, ~0u, ~0u, ~0u));
 }
 
-// Sums over `rows` partial rows of G pairs each: warp w takes the rows w, w + nwarps, ..., lane l the groups l, l + 32, ...;
-// acc[w * G + s], acc[(nwarps + w) * G + s] receive the warp's two sums of group s, formed in row order.  All CTAs of
-// a sample read the same rows at the same moment, so what counts is the number of L2 requests: with one warp per
-// group and a lane per row (32 requests of 8 or 16 bytes per load) a merge of 32 groups x 148 rows took 8.1 us.
-// add(i, pair, K0, sum1, sum2) takes one pair of row i; K0 is the first value of the group's row 0.
-template <typename Add>
-__device__ __forceinline__ void merge_rows(const float2* p, int rows, int G, int warp, int nwarps, int lane, float* acc,
-                                           Add add) {
-  for (int s = lane; s < G; s += 32) {
-    const float K0 = __ldcg(p + s).x;
-    float a1 = 0.f, a2 = 0.f;
-    for (int i0 = warp; i0 < rows; i0 += nwarps * kMergeRows) {
-      float2 v[kMergeRows];
-#pragma unroll
-      for (int q = 0; q < kMergeRows; ++q) {
-        const int i = i0 + nwarps * q;
-        v[q] = i < rows ? __ldcg(p + (size_t)i * G + s) : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int q = 0; q < kMergeRows; ++q)
-        if (i0 + nwarps * q < rows) add(i0 + nwarps * q, v[q], K0, a1, a2);
-    }
-    acc[warp * G + s] = a1;
-    acc[(nwarps + warp) * G + s] = a2;
-  }
-}
-
 // ------------------------------------------------------------------------------------------------
 // forward.  scratch: part[cta * G + s] = (mean, M2) of group s over the CTA's rows
 // ------------------------------------------------------------------------------------------------
@@ -248,9 +215,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   const Geom& g = r.g;
   const Smem sm = carve<1>(r, smem_raw);
   float* red = sm.red;
-  float* tmp = red + g.red_floats;
-  float* slot = tmp + g.slots;
-  float* stat = slot + 3 * g.slots;
+  float* slot = red + g.red_floats;
+  float* stat = slot + g.slots;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
   const int n = g.div_chunks.div((int)blockIdx.x), j = (int)blockIdx.x - n * r.cps;
@@ -323,11 +289,14 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     }
     merge_moments<VE>(pm, pq, pn, mean, m2, cnt);
   }
-  __syncwarp();
-  __syncthreads();
-  cta_slot_moments<VE, UNI>(g, mean, m2, cnt, tx, ty, 0, nrows, 0, g.G, red, tmp, slot);
-  for (int s = tid; s < g.G; s += blockDim.x)
-    part[(size_t)blockIdx.x * g.G + s] = make_float2(slot[s], slot[g.slots + s]);
+  const Crew cr = {tid, (int)blockDim.x, lane, warp, nwarps, 0};
+  crew_moments<VE, UNI>(cr, g, r.ex, mean, m2, cnt, tx, ty, nrows, red, slot,
+                        [&](int s, float mu, float q) { part[(size_t)blockIdx.x * g.G + s] = make_float2(mu, q); });
+  uint4 ga_raw = make_uint4(0, 0, 0, 0), be_raw = ga_raw;
+  if (streaming) {  // (they arrive during the wait)
+    ga_raw = ldg128(gamma + tx * VE);
+    be_raw = ldg128(beta + tx * VE);
+  }
   grid_barrier(count, sm.flags, r);
 
   // ---- statistics of the sample: sums about the first CTA's mean, the counts known from the geometry
@@ -364,7 +333,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   float a[VE], b[VE];
 #pragma unroll
   for (int e = 0; e < VE; ++e) a[e] = b[e] = 0.f;
-  if (streaming) lane_affine<T, VE, UNI>(gamma, beta, stat, stat + g.slots, 0, tx * VE, g.div_D, a, b);
+  if (streaming) lane_affine_raw<T, VE, UNI>(ga_raw, be_raw, stat, stat + g.slots, 0, tx * VE, g.div_D, a, b);
   T* out = y + (row0 + (streaming ? ty : 0)) * g.C + (streaming ? tx * VE : 0);
   const size_t ostep = (size_t)g.TY * g.C;
   // one tile's vectors of the thread, wherever they were kept
@@ -432,9 +401,10 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const Geom& g = r.g;
   const Smem sm = carve<2>(r, smem_raw);
-  float* red = sm.red;              // TY * C
+  float* red = sm.red;
   float* chan = red + g.red_floats;  // S1[C], S2[C]
-  float* coef = chan + 2 * g.C;      // A[G], B[G]
+  float* gam = chan + 2 * g.C;       // gamma[C]
+  float* coef = gam + g.C;           // A[G], B[G]
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (int)blockDim.x >> 5;
   const int n = g.div_chunks.div((int)blockIdx.x), j = (int)blockIdx.x - n * r.cps;
@@ -444,6 +414,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   const bool streaming = ty < g.TY;
   const size_t row0 = (size_t)n * g.R + r0;
 
+  // what the caller gave is asked for before the ring's copies: behind 28 MB of them it would arrive 3 us later
+  LaneParams<T, VE, UNI> lp;
+  if (streaming) lp.load(gamma, beta, mean_in + (size_t)n * g.G, rstd_in + (size_t)n * g.G, tx * VE, g.div_D);
   Stream<T, 2> st;
   st.src[0] = x + row0 * g.C;
   st.src[1] = dy + row0 * g.C;
@@ -457,8 +430,13 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   float a[VE], b[VE];
 #pragma unroll
   for (int e = 0; e < VE; ++e) L.r[e] = L.nmr[e] = L.ga[e] = L.be[e] = 0.f;
-  if (streaming)
-    lane_setup<T, VE, UNI>(gamma, beta, mean_in + (size_t)n * g.G, rstd_in + (size_t)n * g.G, tx * VE, g.div_D, L);
+  if (streaming) {
+    lp.unpack(L);
+    if (ty == 0) {
+#pragma unroll
+      for (int e = 0; e < VE; ++e) gam[tx * VE + e] = L.ga[e];
+    }
+  }
 #pragma unroll
   for (int e = 0; e < VE; ++e) {
     a[e] = L.r[e] * L.ga[e];
@@ -513,40 +491,14 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       s2[e] += kRaw ? fmaf(L.r[e], p2[e], L.nmr[e] * p1[e]) : p2[e];
     }
   }
-  // channel sums over the row lanes, S1 and S2 one after the other through the same scratch
-#pragma unroll
-  for (int which = 0; which < 2; ++which) {
-    __syncwarp();
-    __syncthreads();
-    if (streaming) {
-#pragma unroll
-      for (int e = 0; e < VE; e += 4) {
-        const float4 v = which == 0 ? make_float4(s1[e], s1[e + 1], s1[e + 2], s1[e + 3])
-                                    : make_float4(s2[e], s2[e + 1], s2[e + 2], s2[e + 3]);
-        *reinterpret_cast<float4*>(red + (size_t)ty * g.C + tx * VE + e) = v;
-      }
-    }
-    __syncthreads();
-    for (int c = tid; c < g.C; c += blockDim.x) {
-      float acc = 0.f;
-#pragma unroll 4
-      for (int q = 0; q < g.TY; ++q) acc += red[(size_t)q * g.C + c];
-      chan[which * g.C + c] = acc;
-    }
-  }
-  __syncthreads();
+  const Crew cr = {tid, (int)blockDim.x, lane, warp, nwarps, 0};
+  crew_channel_sums<VE>(cr, g, r.ex, s1, tx, ty, red, chan);
+  cr.sync();
+  crew_channel_sums<VE>(cr, g, r.ex, s2, tx, ty, red, chan + g.C);
+  cr.sync();
+  crew_group_sums(cr, g, r.ex, gam, chan,
+                  [&](int s, float w1, float w2) { gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2); });
   for (int c = tid; c < g.C; c += blockDim.x) tpart[(size_t)blockIdx.x * g.C + c] = make_float2(chan[c], chan[g.C + c]);
-  for (int s = warp; s < g.G; s += nwarps) {  // gamma-weighted group sums of the CTA's rows
-    float w1 = 0.f, w2 = 0.f;
-    for (int c = s * g.D + lane; c < (s + 1) * g.D; c += 32) {
-      const float ga = load_param<T>(gamma, c);
-      w1 = fmaf(ga, chan[c], w1);
-      w2 = fmaf(ga, chan[g.C + c], w2);
-    }
-    w1 = warp_sum_all(w1);
-    w2 = warp_sum_all(w2);
-    if (lane == 0) gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2);
-  }
   grid_barrier(count, sm.flags, r);
 
   // ---- A, B of the sample's groups
@@ -783,7 +735,7 @@ size_t resident_workspace_bytes(const ResidentGeom& r, int direction) { return s
 
 size_t resident_fixed_smem(const ResidentGeom& r, int direction) {
   const Geom& g = r.g;
-  const size_t floats = direction == 0 ? 6 * (size_t)g.slots : 2 * (size_t)g.C + 2 * (size_t)g.G;
+  const size_t floats = direction == 0 ? 3 * (size_t)g.slots : 3 * (size_t)g.C + 2 * (size_t)g.G;
   return kControlBytes + ((size_t)g.red_floats + floats) * 4 + 16;
 }
 

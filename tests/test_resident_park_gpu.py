@@ -39,3 +39,30 @@ def test_parked_tiles_change_no_bit(case, monkeypatch):
         for k in ("y", "dx", "dparam", "mean", "rstd"):
             assert torch.equal(out[k], want[k]), (k, stages, park)
     assert nt.wait_timeouts() == 0
+
+
+@pytest.mark.parametrize("N,C,sp,G,dt,ctas", [
+    (1, 1024, (37, 5), 128, "float16", 3),    # the most groups, a vector each: four threads to a group
+    (2, 512, (29, 7), 128, "float32", 4),     # the same with four lanes
+    (1, 128, (61, 3), 128, "bfloat16", 2),    # one channel per group, 32 row lanes
+    (1, 24, (331, 5), 3, "bfloat16", 2),      # three groups, 170 row lanes, two idle threads
+    (1, 240, (47, 9), 30, "float16", 2),      # 17 row lanes of 30 threads: half a warp without work
+    (2, 264, (31, 11), 3, "float16", 3),      # eleven vectors per group
+    (1, 2048, (19, 3), 1, "float32", 2),      # one row lane of 512 threads
+    (1, 40, (3, 1), 8, "float16", 2),         # fewer rows than row lanes
+], ids=lambda v: str(v).replace(" ", ""))
+def test_reductions_over_the_cta(N, C, sp, G, dt, ctas, monkeypatch):
+    """csrc/gn_reduce.cuh: group moments, channel sums and group sums at the edges of its layout, against the fp64 oracle."""
+    from channels_last_groupnorm_b200 import _native as nt
+
+    monkeypatch.setenv("GNB200_FORCE_PATH", "resident")
+    monkeypatch.setenv("GNB200_RESIDENT_CTAS", str(ctas))
+    assert " resident=1 " in nt.describe_plan(N, sp[0] * sp[1], C, G, DT[dt], 0)
+    x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=31, x_dist="uniform3")
+    out = run_cabi(nt, x, ga, be, dy, G, 1e-5, "silu")
+    want = O.oracle_c(x, ga, be, dy, G, 1e-5, "silu", threads=4)
+    check_against(out, want, DT[dt])
+    # fp32 sums over at most a few thousand values of one group or channel
+    assert O.rel_err(out["mean"], want["mean"]) < 1e-5
+    assert O.rel_err(out["rstd"] / want["rstd"].cuda().float(), torch.ones_like(want["rstd"])) < 1e-5
+    assert O.rel_err(out["dparam"][0], want["dgamma"]) <= O.TOLERANCE[DT[dt]] and O.rel_err(out["dparam"][1], want["dbeta"]) <= O.TOLERANCE[DT[dt]]
