@@ -4,6 +4,8 @@ There is no Python, PyTorch-eager or CPU fallback anywhere in this package: if t
 cannot be loaded (or built from the in-tree sources), importing the package raises.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
@@ -27,10 +29,14 @@ def _load():
         core_path, torch_path = _build.CORE_LIB, _build.TORCH_LIB
     core = ctypes.CDLL(core_path, mode=ctypes.RTLD_GLOBAL)
     torch.ops.load_library(torch_path)
-    return core
+    # the same library is a Python module too (gn_torch.cpp: plain_call)
+    loader = importlib.machinery.ExtensionFileLoader("gnb200_torch", torch_path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("gnb200_torch", torch_path, loader=loader))
+    loader.exec_module(module)
+    return core, module
 
 
-lib = _load()
+lib, torch_module = _load()
 
 lib.gnb200_version.restype = ctypes.c_int
 lib.gnb200_last_error.restype = ctypes.c_char_p

@@ -114,7 +114,7 @@ def build_torch(verbose=False):
     torch_lib = ce.library_paths()[0]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(CSRC, "gn_torch.cpp"), "-o", TORCH_LIB,
            "-DTORCH_API_INCLUDE_EXTENSION_H"] + inc + [
-        "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
+        "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
         "-L", LIB_DIR, "-lgnb200", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + torch_lib]
     if verbose:
         print("+", " ".join(cmd), flush=True)

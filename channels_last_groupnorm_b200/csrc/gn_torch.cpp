@@ -14,14 +14,21 @@
 // [2, C] tensor in the statistics' dtype (the buffer a data-parallel caller all-reduces), and the ops
 // carry explicit schemas with a CUDA implementation (the reference registers catch-all functions, which
 // cannot be traced).
+#include <Python.h>
+
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/Tensor.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/core/dispatch/Dispatcher.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
+#include <ATen/record_function.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
 #include <vector>
@@ -270,6 +277,134 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> call_fwd(const at::Tensor& X, con
   return op.call(X, w, b, G, eps, act);
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same without views and inner dispatches, for plain calls.  A small call is bound by the host: of 19.5 us for one
+// without gradients about half went into seven view ops, the second dispatch, three allocations and the autograd node that
+// nothing needed.  A call is plain when nothing but autograd and CUDA kernels would see its ops (no dispatch mode, functorch
+// transform, tracer, lazy negation, profiler) and its tensor has the storage order that the kernels want; every other call
+// goes through the ops as before.  The kernels, their arguments and the results' sizes and strides are the same.
+// ------------------------------------------------------------------------------------------------
+bool only_cuda_sees(std::initializer_list<const at::Tensor*> tensors) {
+  static const c10::DispatchKeySet allowed =
+      c10::autograd_dispatch_keyset_with_ADInplaceOrView | c10::autocast_dispatch_keyset |
+      c10::DispatchKeySet({c10::DispatchKey::BackendSelect, c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA});
+  c10::DispatchKeySet ks;
+  for (const at::Tensor* t : tensors) ks = ks | t->key_set();
+  const auto tls = c10::impl::tls_local_dispatch_key_set();
+  ks = (ks | tls.included_) - tls.excluded_;
+  return (ks.raw_repr() & ~allowed.raw_repr()) == 0 && !at::hasCallbacks();
+}
+
+// Storage of a plain tensor of rank >= 3, by the rules of flatten() and layout_of(); false where it would be copied.
+struct Dense {
+  bool channels_last;  // by is_channels_last(): decides the strides of results
+  Layout layout;
+  int64_t N, C, R;
+};
+bool dense_order(const at::Tensor& t, bool channels_last) {
+  if (!channels_last) return t.is_contiguous();
+  const auto sizes = t.sizes(), strides = t.strides();
+  if (sizes[1] != 1 && strides[1] != 1) return false;
+  int64_t want = sizes[1];
+  for (int64_t d = t.dim() - 1; d >= 2; --d) {
+    if (sizes[d] != 1 && strides[d] != want) return false;
+    want *= sizes[d];
+  }
+  return sizes[0] == 1 || strides[0] == want;
+}
+bool plain_tensor(const at::Tensor& t, Dense* out) {
+  if (t.dim() < 3 || t.numel() == 0 || !t.is_cuda()) return false;
+  const auto st = t.scalar_type();
+  if (st != at::kFloat && st != at::kHalf && st != at::kBFloat16) return false;
+  const bool cl = is_channels_last(t);
+  if (!dense_order(t, cl)) return false;
+  const int64_t n = t.size(0), c = t.size(1), r = t.numel() / (n * c);
+  *out = Dense{cl, cl || r == 1 ? kNHWC : kNCHW, n, c, r};
+  return true;
+}
+// uninitialised, with the sizes of `like` and the strides that restore() gives
+at::Tensor empty_result(const at::Tensor& like, const Dense& d) {
+  const auto sizes = like.sizes();
+  at::DimVector strides(sizes.size());
+  int64_t step = d.channels_last ? d.C : 1;
+  for (int64_t i = (int64_t)sizes.size() - 1; i >= 2; --i) strides[i] = step, step *= sizes[i];
+  strides[1] = d.channels_last ? 1 : step;
+  strides[0] = d.channels_last ? step : step * d.C;
+  return at::detail::empty_strided_cuda(sizes, strides, like.scalar_type(), like.device());
+}
+at::Tensor empty_vector(std::initializer_list<int64_t> sizes, at::ScalarType st, const at::Tensor& like) {
+  return at::detail::empty_cuda(at::IntArrayRef(sizes.begin(), sizes.size()), st, like.device(), std::nullopt);
+}
+
+// Y; where `means` is given the statistics are results too, otherwise they share the scratch.
+at::Tensor direct_fwd(const at::Tensor& X, const Dense& d, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
+                      int64_t act, at::Tensor* means, at::Tensor* rstds) {
+  const int dtype = dtype_code(X, "X");
+  check_param(weight, X, d.C, "weight");
+  check_param(bias, X, d.C, "bias");
+  TORCH_CHECK(G >= 1 && d.C % G == 0, "gnb200: num_channels ", d.C, " is not divisible by num_groups ", G);
+  TORCH_CHECK(act >= 0 && act <= 4, "gnb200: activation code ", act, " is not in 0..4");
+  c10::cuda::CUDAGuard guard(X.device());
+  at::Tensor Y = empty_result(X, d);
+  const size_t ws_bytes = d.layout == kNHWC ? gnb200_fwd_workspace_bytes(d.N, d.R, d.C, G, dtype)
+                                            : gnb200_fwd_nchw_workspace_bytes(d.N, d.R, d.C, G, dtype);
+  const size_t ws_end = (ws_bytes + 15) & ~(size_t)15, stat_bytes = (size_t)d.N * G * sizeof(float);
+  at::Tensor ws;
+  float *mean, *rstd;
+  if (means) {
+    *means = empty_vector({d.N, G}, at::kFloat, X);
+    *rstds = empty_vector({d.N, G}, at::kFloat, X);
+    mean = means->mutable_data_ptr<float>();
+    rstd = rstds->mutable_data_ptr<float>();
+    if (ws_bytes) ws = empty_vector({(int64_t)ws_bytes}, at::kByte, X);
+  } else {
+    ws = empty_vector({(int64_t)(ws_end + 2 * stat_bytes)}, at::kByte, X);
+    mean = reinterpret_cast<float*>(ws.mutable_data_ptr<uint8_t>() + ws_end);
+    rstd = mean + d.N * G;
+  }
+  auto fn = d.layout == kNHWC ? &gnb200_fwd : &gnb200_fwd_nchw;
+  check_status(fn(X.const_data_ptr(), weight.const_data_ptr(), bias.const_data_ptr(), d.N, d.R, d.C, G, eps, (int)act, dtype,
+                  Y.mutable_data_ptr(), mean, rstd, ws_bytes ? ws.mutable_data_ptr() : nullptr, ws_bytes,
+                  c10::cuda::getCurrentCUDAStream().stream()));
+  return Y;
+}
+
+// typed: dgamma, dbeta in X's dtype; otherwise the two rows of one fp32 tensor
+void direct_bwd(const at::Tensor& dy, const at::Tensor& X, const Dense& d, const at::Tensor& weight, const at::Tensor& bias,
+                const at::Tensor& means, const at::Tensor& rstds, int64_t G, int64_t act, bool typed, at::Tensor* dx,
+                at::Tensor* dgamma, at::Tensor* dbeta) {
+  const int dtype = dtype_code(X, "X");
+  check_param(weight, X, d.C, "weight");
+  check_param(bias, X, d.C, "bias");
+  check_stats(means, X, dtype, d.N, G, "means");
+  check_stats(rstds, X, dtype, d.N, G, "rstds");
+  c10::cuda::CUDAGuard guard(X.device());
+  *dx = empty_result(X, d);
+  const size_t ws_bytes = d.layout == kNHWC ? gnb200_bwd_workspace_bytes(d.N, d.R, d.C, G, dtype)
+                                            : gnb200_bwd_nchw_workspace_bytes(d.N, d.R, d.C, G, dtype);
+  const size_t ws_end = (ws_bytes + 15) & ~(size_t)15;
+  at::Tensor ws = empty_vector({(int64_t)(ws_end + (typed ? 2 * d.C * sizeof(float) : 0))}, at::kByte, X), dparam;
+  float* dp32;
+  if (typed) {
+    dp32 = reinterpret_cast<float*>(ws.mutable_data_ptr<uint8_t>() + ws_end);
+    *dgamma = empty_vector({d.C}, X.scalar_type(), X);
+    *dbeta = empty_vector({d.C}, X.scalar_type(), X);
+  } else {
+    dparam = empty_vector({2, d.C}, at::kFloat, X);
+    dp32 = dparam.mutable_data_ptr<float>();
+  }
+  auto fn = d.layout == kNHWC ? &gnb200_bwd : &gnb200_bwd_nchw;
+  check_status(fn(dy.const_data_ptr(), X.const_data_ptr(), weight.const_data_ptr(), bias.const_data_ptr(),
+                  means.const_data_ptr<float>(), rstds.const_data_ptr<float>(), d.N, d.R, d.C, G, (int)act, dtype,
+                  dx->mutable_data_ptr(), dp32, typed ? dgamma->mutable_data_ptr() : nullptr,
+                  typed ? dbeta->mutable_data_ptr() : nullptr, ws_bytes ? ws.mutable_data_ptr() : nullptr, ws_bytes,
+                  c10::cuda::getCurrentCUDAStream().stream()));
+  if (!typed) {
+    *dgamma = dparam.select(0, 0);
+    *dbeta = dparam.select(0, 1);
+  }
+}
+
 struct GnFunction : torch::autograd::Function<GnFunction> {
   // everything that backward uses is saved through ctx, and it calls dispatcher ops only: compiled autograd may trace it
   static constexpr bool is_traceable = true;
@@ -277,12 +412,19 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias,
                             int64_t G, double eps, int64_t act) {
     const bool cl = is_channels_last(X);
-    const at::Tensor Xf = flatten(X, cl);
     const at::Tensor w = as_dtype(weight, X.scalar_type()), b = as_dtype(bias, X.scalar_type());
+    ctx->saved_data["arg"] = std::vector<int64_t>{G, act, cl ? 1 : 0, (int64_t)weight.scalar_type(), (int64_t)bias.scalar_type()};
+    Dense d;
+    if (only_cuda_sees({&X, &w, &b}) && plain_tensor(X, &d)) {  // X itself is saved, in the order that flatten() would give
+      at::Tensor means, rstds;
+      at::Tensor Y = direct_fwd(X, d, w, b, G, eps, act, &means, &rstds);
+      ctx->save_for_backward({X, w, b, means, rstds});
+      return Y;
+    }
+    const at::Tensor Xf = flatten(X, cl);
     auto [Y, means, rstds] = call_fwd(Xf, w, b, G, eps, act);
     ctx->save_for_backward({Xf, w, b, means, rstds});
     ctx->saved_data["shape"] = X.sizes().vec();
-    ctx->saved_data["arg"] = std::vector<int64_t>{G, act, cl ? 1 : 0, (int64_t)weight.scalar_type(), (int64_t)bias.scalar_type()};
     return restore(Y, X.sizes(), cl);
   }
 
@@ -291,12 +433,26 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
     static const auto op32 =
         c10::Dispatcher::singleton().findSchemaOrThrow("gnb200::bwd_f32", "").typed<decltype(gnb200_bwd_f32_op)>();
     const auto saved = ctx->get_saved_variables();
-    const auto shape = ctx->saved_data["shape"].toIntVector(), arg = ctx->saved_data["arg"].toIntVector();
-    const at::Tensor& Xf = saved[0];
-    const at::ScalarType dtype = Xf.scalar_type();
+    const auto arg = ctx->saved_data["arg"].toIntVector();
+    const at::ScalarType dtype = saved[0].scalar_type();
     const auto w_dtype = (at::ScalarType)arg[3], b_dtype = (at::ScalarType)arg[4];
-    const at::Tensor dy = as_dtype(flatten(grads[0], arg[2] != 0), dtype);
     at::Tensor dx, dgamma, dbeta;
+    const auto flat_shape = ctx->saved_data.find("shape");
+    const bool unflattened = flat_shape == ctx->saved_data.end();
+    const at::Tensor& g = grads[0];
+    Dense d;
+    if (unflattened && !c10::GradMode::is_enabled() && g.defined() &&
+        only_cuda_sees({&g, &saved[0], &saved[1], &saved[2], &saved[3], &saved[4]}) && plain_tensor(saved[0], &d) &&
+        d.channels_last == (arg[2] != 0) && g.scalar_type() == dtype && g.device() == saved[0].device() &&
+        g.sizes() == saved[0].sizes() && dense_order(g, d.channels_last)) {
+      const bool typed = w_dtype == dtype && b_dtype == dtype;
+      direct_bwd(g, saved[0], d, saved[1], saved[2], saved[3], saved[4], arg[0], arg[1], typed, &dx, &dgamma, &dbeta);
+      return {dx, as_dtype(dgamma, w_dtype), as_dtype(dbeta, b_dtype), at::Tensor(), at::Tensor(), at::Tensor()};
+    }
+    // (under create_graph the saved input must not bring a graph of its own along, as its flattened view does not)
+    const at::Tensor Xf = unflattened ? flatten(c10::GradMode::is_enabled() ? saved[0].detach() : saved[0], arg[2] != 0) : saved[0];
+    const auto shape = unflattened ? saved[0].sizes().vec() : flat_shape->second.toIntVector();
+    const at::Tensor dy = as_dtype(flatten(g, arg[2] != 0), dtype);
     if (w_dtype == dtype && b_dtype == dtype) {
       std::tie(dx, dgamma, dbeta) = op.call(dy, Xf, saved[1], saved[2], saved[3], saved[4], arg[0], arg[1]);
     } else {
@@ -312,6 +468,19 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
 at::Tensor group_norm_act_autograd(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
                                    int64_t act) {
   return GnFunction::apply(X, weight, bias, G, eps, act);
+}
+
+// The module's call, if it is a plain one; an undefined tensor otherwise.
+at::Tensor group_norm_act_direct(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
+                                 int64_t act) {
+  Dense d;
+  if (!only_cuda_sees({&X, &weight, &bias}) || !plain_tensor(X, &d)) return at::Tensor();
+  for (const at::Tensor* t : {&X, &weight, &bias})
+    if (t->_fw_grad(0).defined()) return at::Tensor();  // dual tensors
+  if (c10::GradMode::is_enabled() && (X.requires_grad() || weight.requires_grad() || bias.requires_grad()))
+    return GnFunction::apply(X, weight, bias, G, eps, act);
+  at::AutoDispatchBelowADInplaceOrView guard;
+  return direct_fwd(X, d, as_dtype(weight, X.scalar_type()), as_dtype(bias, X.scalar_type()), G, eps, act, nullptr, nullptr);
 }
 
 // below autograd (inference mode)
@@ -355,3 +524,43 @@ TORCH_LIBRARY_IMPL(gnb200, CPU, m) {
   m.impl("bwd", &gnb200_bwd_op);
   m.impl("bwd_f32", &gnb200_bwd_f32_op);
 }
+
+// ------------------------------------------------------------------------------------------------
+// plain_call(x, weight, bias, num_groups, eps, act, num_channels) -> tensor, or None where the module's Python code has
+// to look at the call: anything but exact tensors and parameters, a torch-function mode, other argument types, a shape that it
+// refuses.  Called without torch.ops' argument matching, which took 3 us.
+// ------------------------------------------------------------------------------------------------
+namespace {
+
+const at::Tensor* exact_tensor(PyObject* o) {
+  if (Py_TYPE(o) != (PyTypeObject*)THPVariableClass && Py_TYPE(o) != (PyTypeObject*)ParameterClass) return nullptr;
+  return &THPVariable_Unpack(o);
+}
+
+PyObject* plain_call(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 7 || !PyLong_CheckExact(args[3]) || !PyFloat_CheckExact(args[4]) || !PyLong_CheckExact(args[5]) ||
+      !PyLong_CheckExact(args[6]) || at::impl::torch_function_mode_enabled())
+    Py_RETURN_NONE;
+  const at::Tensor *x = exact_tensor(args[0]), *w = exact_tensor(args[1]), *b = exact_tensor(args[2]);
+  if (!x || !w || !b) Py_RETURN_NONE;
+  const long long G = PyLong_AsLongLong(args[3]), act = PyLong_AsLongLong(args[5]), C = PyLong_AsLongLong(args[6]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!x->is_cuda() || x->dim() < 3 || x->size(1) != C) Py_RETURN_NONE;
+  const double eps = PyFloat_AS_DOUBLE(args[4]);
+  at::Tensor y;
+  {
+    pybind11::gil_scoped_release no_gil;
+    y = group_norm_act_direct(*x, *w, *b, G, eps, act);
+  }
+  if (!y.defined()) Py_RETURN_NONE;
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef kMethods[] = {{"plain_call", (PyCFunction)(void (*)())plain_call, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "gnb200_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_gnb200_torch(void) { return PyModule_Create(&kModule); }

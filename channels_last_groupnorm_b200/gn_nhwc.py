@@ -133,6 +133,7 @@ def _restore_shape(flat: torch.Tensor, shape, channels_last=True) -> torch.Tenso
 
 
 _group_norm_act = torch.ops.gnb200.group_norm_act.default
+_plain_call = _native.torch_module.plain_call
 _PLAIN = (torch.Tensor, nn.Parameter)
 
 
@@ -164,6 +165,11 @@ class GN_NHWC(nn.GroupNorm):
         self.process_group = process_group
 
     def forward(self, x):
+        if self.process_group is None and not torch.compiler.is_compiling():
+            # the whole call natively where it is an ordinary one; what follows is for every other kind, errors included
+            y = _plain_call(x, self.weight, self.bias, self.num_groups, self.eps, self.act_code, self.num_channels)
+            if y is not None:
+                return y
         if not x.is_cuda:
             raise ValueError("GN_NHWC: input must be a CUDA tensor; this package has no CPU path")
         if x.ndim < 3 or x.shape[1] != self.num_channels:
