@@ -128,14 +128,15 @@ __device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw,
   for (int p = 0; p < 4; ++p) {
     float g0 = 1.f, g1 = 1.f;
     if constexpr (ACT != kActIdentity) {
-      const float yh0 = fmaf(fx[2 * p], a[2 * p], b[2 * p]);
-      const float yh1 = fmaf(fx[2 * p + 1], a[2 * p + 1], b[2 * p + 1]);
+      float yh0, yh1;
+      fma2(yh0, yh1, fx[2 * p], fx[2 * p + 1], a[2 * p], a[2 * p + 1], b[2 * p], b[2 * p + 1]);
       const float2 gf = __half22float2(act_grad_pair<ACT>(yh0, yh1));
       g0 = gf.x;
       g1 = gf.y;
     }
-    o[2 * p] = fmaf(ag[2 * p], fd[2 * p] * g0, fmaf(c1[2 * p], fx[2 * p], c2[2 * p]));
-    o[2 * p + 1] = fmaf(ag[2 * p + 1], fd[2 * p + 1] * g1, fmaf(c1[2 * p + 1], fx[2 * p + 1], c2[2 * p + 1]));
+    float t0, t1;
+    fma2(t0, t1, c1[2 * p], c1[2 * p + 1], fx[2 * p], fx[2 * p + 1], c2[2 * p], c2[2 * p + 1]);
+    fma2(o[2 * p], o[2 * p + 1], ag[2 * p], ag[2 * p + 1], fd[2 * p] * g0, fd[2 * p + 1] * g1, t0, t1);
   }
   return pack16<T, 8>(o);
 }

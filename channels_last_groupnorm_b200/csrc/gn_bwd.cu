@@ -271,11 +271,13 @@ __device__ __forceinline__ void tile_bwd_dx(const T* __restrict__ gx, uint32_t r
         gx += gstep_elems;
       }
       cp_async_commit();
+      if constexpr (kFold) {
+        affine<VE>(fx, c1, c2);
 #pragma unroll
-      for (int e = 0; e < VE; ++e) {
-        if constexpr (kFold) {
-          fx[e] = fmaf(ag[e], fd[e], fmaf(c1[e], fx[e], c2[e]));
-        } else {
+        for (int e = 0; e < VE; e += 2) fma2(fx[e], fx[e + 1], ag[e], ag[e + 1], fd[e], fd[e + 1], fx[e], fx[e + 1]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < VE; ++e) {
           const float xh = fmaf(fx[e], L.r[e], L.nmr[e]);
           fx[e] = fmaf(ag[e], fd[e], fmaf(nb[e], xh, na[e]));
         }

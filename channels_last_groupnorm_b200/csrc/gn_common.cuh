@@ -260,6 +260,44 @@ __device__ __forceinline__ float mixed_fma(uint16_t a, uint16_t b, float c) {
   return d;
 }
 
+// Two fp32 operations in one instruction (PTX .f32x2, sm_100): each half rounds as the scalar one does, so results are
+// the same bits.  The 16-bit cluster kernels keep three quarters of the issue slots busy and a third of the FMA pipe: 64 x
+// 256 x 64^2 bf16 GELU forward 55.6 -> 54.8 us, backward 92.7 -> 92.3; fp16 SiLU 51.7 -> 50.9, 95.4 -> 92.6.
+__device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0, float c1) {
+  asm("{\n\t"
+      ".reg .b64 a, b, c, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "mov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
+__device__ __forceinline__ void add2(float& d0, float& d1, float a0, float a1, float b0, float b1) {
+  asm("{\n\t"
+      ".reg .b64 a, b, d;\n\t"
+      "mov.b64 a, {%2, %3};\n\t"
+      "mov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 d, a, b;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t"
+      "}"
+      : "=f"(d0), "=f"(d1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+}
+// f = f * a + b, lane by lane
+template <int VE>
+__device__ __forceinline__ void affine(float (&f)[VE], const float (&a)[VE], const float (&b)[VE]) {
+  if constexpr (VE % 2 == 0) {
+#pragma unroll
+    for (int e = 0; e < VE; e += 2) fma2(f[e], f[e + 1], f[e], f[e + 1], a[e], a[e + 1], b[e], b[e + 1]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+  }
+}
+
 // 16 bytes of T viewed as a uint4 <-> fp32 lanes
 template <typename T, int VE>
 __device__ __forceinline__ void unpack16(const uint4& w, float (&f)[VE]) {

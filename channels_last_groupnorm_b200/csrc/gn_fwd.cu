@@ -215,8 +215,7 @@ __device__ __forceinline__ void tile_apply(uint32_t stile, uint32_t sstep_bytes,
         gnext += gstep_elems;
       }
       sp += sstep_bytes;
-#pragma unroll
-      for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+      affine<VE>(f, a, b);
       stg128(gp, act_pack16<T, VE, ACT>(f));
       gp += gstep_elems;
     }
@@ -259,8 +258,7 @@ __device__ __forceinline__ void stream_apply(const Pack<T, VE>* __restrict__ src
       float f[VE];
       unpack<T, VE>(v[u], f);
       if constexpr (sizeof(T) * VE == 16) {
-#pragma unroll
-        for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+        affine<VE>(f, a, b);
         stg128(dp, act_pack16<T, VE, ACT>(f));
       } else {
 #pragma unroll
@@ -302,8 +300,7 @@ __device__ __forceinline__ void stream_apply_back(const Pack<T, VE>* __restrict_
     float f[VE];
     unpack<T, VE>(v, f);
     if constexpr (sizeof(T) * VE == 16) {
-#pragma unroll
-      for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+      affine<VE>(f, a, b);
       stg128_stream(dp, act_pack16<T, VE, ACT>(f));
     } else {
 #pragma unroll

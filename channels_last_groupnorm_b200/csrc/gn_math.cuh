@@ -35,10 +35,8 @@ __device__ __forceinline__ void shifted_step(const uint4& w, const float (&K)[KN
     split_halves(r[e], lo, hi);
     const float d0 = mixed_sub<T>(lo, K[KN == 1 ? 0 : 2 * e]);
     const float d1 = mixed_sub<T>(hi, K[KN == 1 ? 0 : 2 * e + 1]);
-    s[2 * e] += d0;
-    s[2 * e + 1] += d1;
-    q[2 * e] = fmaf(d0, d0, q[2 * e]);
-    q[2 * e + 1] = fmaf(d1, d1, q[2 * e + 1]);
+    add2(s[2 * e], s[2 * e + 1], s[2 * e], s[2 * e + 1], d0, d1);
+    fma2(q[2 * e], q[2 * e + 1], d0, d1, d0, d1, q[2 * e], q[2 * e + 1]);
   }
 }
 
@@ -280,8 +278,8 @@ __device__ __forceinline__ uint4 bwd_row_sums_packed(const uint4& xw, const uint
     split_halves(xr[p], x0, x1);
     uint32_t dyh = dr[p];
     if constexpr (ACT != kActIdentity) {
-      const float yh0 = fmaf(mixed_add<T>(x0, -0.0f), a[2 * p], b[2 * p]);
-      const float yh1 = fmaf(mixed_add<T>(x1, -0.0f), a[2 * p + 1], b[2 * p + 1]);
+      float yh0, yh1;
+      fma2(yh0, yh1, mixed_add<T>(x0, -0.0f), mixed_add<T>(x1, -0.0f), a[2 * p], a[2 * p + 1], b[2 * p], b[2 * p + 1]);
       const __half2 g = act_grad_pair<ACT>(yh0, yh1);
       if constexpr (std::is_same<T, __half>::value) {
         const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&dr[p]), g);

@@ -345,8 +345,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       if (my_row + u * g.TY < here) {
         float f[VE];
         unpack16<T, VE>(w[u], f);
-#pragma unroll
-        for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+        affine<VE>(f, a, b);
         stg128_stream(o + (size_t)u * ostep, act_pack16<T, VE, ACT>(f));
       }
     }

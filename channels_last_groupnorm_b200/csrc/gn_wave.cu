@@ -439,8 +439,7 @@ __global__ void __launch_bounds__(kWaveThreads, 3)
               if (r + ty + j * g.TY < t.r1) {
                 float f[VE];
                 unpack16<T, VE>(w[j], f);
-#pragma unroll
-                for (int e = 0; e < VE; ++e) f[e] = fmaf(f[e], a[e], b[e]);
+                affine<VE>(f, a, b);
                 stg128_stream(yrow + (size_t)j * ystep, act_pack16<T, VE, ACT>(f));
               }
             }
