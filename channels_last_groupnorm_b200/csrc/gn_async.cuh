@@ -114,6 +114,18 @@ __device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, ui
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
+// The same for rows that are not read again: their lines are the first that L2 gives up, so the others stay.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
+__device__ __forceinline__ void bulk_load_once(uint32_t smem_dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(smem_dst),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(policy)
+               : "memory");
+}
+
 // dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half
 // precision, dx = ag * dyh + c1 * x + c2.
 template <typename T, int ACT>

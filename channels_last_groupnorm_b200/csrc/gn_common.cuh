@@ -756,6 +756,7 @@ struct ResidentGeom {
   int BR;              // rows per tile (resident_rows * TY)
   int tile_bytes;      // BR * C * sizeof(T), one tensor
   int stages;
+  int evict;           // rows that are not read again are marked evict-first in L2
   int park;            // tiles of a range that are kept in tensor memory besides those in the stages
   int threads;
   long long grid;      // N * cps

@@ -530,6 +530,11 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   if (r.stages > max_stages) r.stages = max_stages < 2 ? 2 : max_stages;
   if (r.stages > 16) r.stages = 16;
   // GNB200_RESIDENT_STAGES alone bounds what stays on chip
+  // Rows that are on chip between the passes, and those on their second read, need no place in L2: the rows that pass 2 reads
+  // again find more of it.  Device us, without / with (fp16): forward 512@256^2 37.0 / 35.0, 256@512^2 71.5 / 67.8,
+  // 128@1024^2 143.5 / 139.1; backward 512@256^2 64.8 / 63.8, bf16 75 MB 72.0 / 71.0, but 256@512^2 119.2 / 121.0 and
+  // 128@1024^2 228.7 / 234.0: with x and dy of twice L2 what is found there is what the second reads leave behind.
+  r.evict = sh.direction == 0 || 2.0 * sh.N * sh.R * sh.C * s <= 192.0 * 1024 * 1024;
   r.park = env_int("GNB200_RESIDENT_PARK", max_stages < 16 ? 0 : kResidentPark);
   if (r.park < 0 || r.park > kResidentPark) r.park = kResidentPark;
   r.smem_bytes = fixed + (size_t)r.stages * stage;

@@ -15,7 +15,8 @@
 //            L2 still holds) is read first; results leave with streaming (evict-first) stores
 //
 // What the tensor memory gave (fp16 SiLU, calls among others): forward 256@512^2 74.0 -> 71.7 us; reductions of all groups
-// at once and parameters asked for early: 71.7 -> 70.2, and 128@1024^2 forward + backward 368 -> 356.5.
+// at once and parameters asked for early: 71.7 -> 70.2, and 128@1024^2 forward + backward 368 -> 356.5.  Evict-first marks
+// (Stream::issue, the rule in gn_plan.cu): 69.9 -> 66.8.
 //
 // dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.
 // Measured against the plans it replaces: see the rule in gn_plan.cu.
@@ -77,21 +78,28 @@ struct Stream {
   unsigned full_ph, empty_ph, last_ph;  // last_ph: the phase of each stage's last copy
   Smem sm;
 
-  __device__ __forceinline__ void issue(int t, int stage) {  // thread 0
+  // `once`: the tile is not read from global memory again
+  __device__ __forceinline__ void issue(int t, int stage, bool once) {  // thread 0
     const uint32_t bytes = (uint32_t)min(BR, nrows - t * BR) * row_bytes;
     last_ph ^= 1u << stage;
     mbar_arrive_expect_tx(&sm.full[stage], NT * bytes);
+    const uint64_t policy = evict_first_policy();
 #pragma unroll
-    for (int i = 0; i < NT; ++i)
-      bulk_load(sm.stage0 + (uint32_t)(stage * NT + i) * tile_bytes,
-                reinterpret_cast<const char*>(src[i]) + (size_t)t * tile_bytes, bytes, &sm.full[stage]);
+    for (int i = 0; i < NT; ++i) {
+      const uint32_t dst = sm.stage0 + (uint32_t)(stage * NT + i) * tile_bytes;
+      const char* from = reinterpret_cast<const char*>(src[i]) + (size_t)t * tile_bytes;
+      if (once)
+        bulk_load_once(dst, from, bytes, &sm.full[stage], policy);
+      else
+        bulk_load(dst, from, bytes, &sm.full[stage]);
+    }
   }
   // thread 0: waits until every warp has handed the stage back, then refills it.  Without the hand-back
   // (its wait gave up) nothing is copied over a stage that may still be read.
-  __device__ __forceinline__ void refill(int t, int stage, const WaitLimit& lim, bool withhold = false) {
+  __device__ __forceinline__ void refill(int t, int stage, bool once, const WaitLimit& lim, bool withhold = false) {
     producer_wait(&sm.empty[stage], (empty_ph >> stage) & 1u, &sm.flags[0], lim);
     empty_ph ^= 1u << stage;
-    if (*(volatile int*)&sm.flags[0] == 0 && !withhold) issue(t, stage);
+    if (*(volatile int*)&sm.flags[0] == 0 && !withhold) issue(t, stage, once);
   }
   __device__ __forceinline__ bool wait_full(int stage, const WaitLimit& lim) {
     const bool ok = consumer_wait(&sm.full[stage], (full_ph >> stage) & 1u, &sm.flags[0], lim);
@@ -122,7 +130,7 @@ struct Stream {
   // thread 0, once item `done` has been read: the item that takes its stage
   __device__ __forceinline__ void refill_behind(int done, const ResidentGeom& r) {
     if (done + stages < next || next >= items()) return;
-    refill(tile_of(next), next_stage, r.g.wait, next == stages && test_at(r, kDebugNoSecondCopy));
+    refill(tile_of(next), next_stage, r.evict, r.g.wait, next == stages && test_at(r, kDebugNoSecondCopy));
     ++next;
     next_stage = next_stage == 0 ? stages - 1 : next_stage - 1;
   }
@@ -151,7 +159,7 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
     }
     sm.flags[0] = 0;
     fence_mbar_init_cluster();
-    for (int t = test_at(r, kDebugNoFirstCopy) ? 1 : 0; t < min(r.stages, st.tiles); ++t) st.issue(t, t);
+    for (int t = test_at(r, kDebugNoFirstCopy) ? 1 : 0; t < min(r.stages, st.tiles); ++t) st.issue(t, t, r.evict && t >= st.held0);
   }
   __syncwarp();
   __syncthreads();
@@ -279,7 +287,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       pin_regs(pm);
       pin_regs(pq);
       if (t + S < T_) release_stage(&sm.empty[stage], lane);
-      if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
+      if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, r.evict && t - 1 + S >= st.held0, g.wait);
       prev = stage;
       if (++stage == S) stage = 0;
     }
@@ -479,7 +487,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       pin_regs(p1);
       pin_regs(p2);
       if (t + S < T_) release_stage(&sm.empty[stage], lane);
-      if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, g.wait);
+      if (tid == 0 && t >= 1 && t - 1 + S < T_) st.refill(t - 1 + S, prev, r.evict && t - 1 + S >= st.held0, g.wait);
       prev = stage;
       if (++stage == S) stage = 0;
     }
