@@ -690,6 +690,13 @@ struct FastDiv {
   __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, mul) + (uint32_t)n) >> shr); }
 };
 
+// Layout of the reductions of gn_reduce.cuh: 2^part_shift neighbouring threads share a group's sum, the scratch has
+// rows of `stride` (odd) floats, div_W divides by the entries that a group has in such a row.
+struct ReduceGeom {
+  int part_shift, stride;
+  FastDiv div_W;
+};
+
 struct Geom {
   int N, R, C, G, D;
   int CW;            // channels per column block (multiple of VE)
@@ -705,6 +712,7 @@ struct Geom {
   // threads per group row (D / VE) are powers of two and CV <= 32.  tps_shift = log2(D / VE).
   int shuf, tps_shift;
   int red_floats;  // size of the reduction scratch `red`, set by the planner
+  ReduceGeom rd;   // its layout (forward: fused generic reductions, resident; backward: resident)
   int wsum_stride, wpart_off;  // shuffle reductions: second warp-sum buffer and (backward) per-warp channel sums in `red`, in floats
   WaitLimit wait;  // limits and give-up record of the bounded waits (set by the launcher)
   int skip_push_rank;  // -1; the exchange self-test names a cluster rank that withholds its pushes
@@ -735,13 +743,6 @@ struct WaveGeom {
   unsigned long long* trace;  // optional timeline buffer (tuning aid), else null
 };
 
-// Layout of the reductions of gn_reduce.cuh: 2^part_shift neighbouring threads share a group's sum, the scratch has
-// rows of `stride` (odd) floats, div_W divides by the entries that a group has in such a row.
-struct ReduceGeom {
-  int part_shift, stride;
-  FastDiv div_W;
-};
-
 // Geometry of the resident plan (gn_resident.cu): one CTA per SM; every sample's rows are cut into `cps`
 // contiguous row ranges, and a CTA streams its range - whole rows, hence one contiguous run of memory - in
 // tiles of BR rows through a ring of `stages` shared-memory stages.
@@ -751,7 +752,6 @@ __host__ __device__ constexpr int resident_rows(int direction) { return directio
 constexpr int kResidentPark = 8;  // tiles that tensor memory holds: 128 words a thread, 16 of them per tile
 struct ResidentGeom {
   Geom g;              // CW = C, ncb = 1, slots = G; rows_per_cta, chunks = cps
-  ReduceGeom ex;
   int cps;             // CTAs per sample
   int BR;              // rows per tile (resident_rows * TY)
   int tile_bytes;      // BR * C * sizeof(T), one tensor

@@ -19,6 +19,7 @@
 #include "gn_async.cuh"
 #include "gn_kernels.h"
 #include "gn_math.cuh"
+#include "gn_reduce.cuh"
 
 namespace gnb200 {
 
@@ -336,7 +337,7 @@ __device__ __forceinline__ void stream_apply_back(const Pack<T, VE>* __restrict_
 // CTA pushes its (mean, M2, count) into the inboxes of all CTAs of the cluster (st.async) and
 // waits on its own mbarrier for the k contributions; inboxes alternate between two copies, and a
 // copy is pushed to again only by peers that have seen this CTA's contribution to the next item.
-// dynamic smem: [tile rows_per_cta * CV packs][red][tmp slots][slot 3*slots][stat 2*slots]
+// dynamic smem: [tile rows_per_cta * CV packs][red][slot slots][stat 2*slots]
 //               [2 inboxes of k*slots entries of 4 floats][2 mbarriers][dead flag]
 // ------------------------------------------------------------------------------------------------
 // MAXT: CTA size class.  128-thread launches are compiled for six CTAs per SM (<= 80 registers).
@@ -356,9 +357,8 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 6 : 2)
 
   const size_t tile_bytes = ((size_t)g.rows_per_cta * g.CV * sizeof(P) + 15) & ~(size_t)15;
   float* red = reinterpret_cast<float*>(reinterpret_cast<char*>(smem_raw) + tile_bytes);
-  float* tmp = red + g.red_floats;
-  float* slot = tmp + g.slots;       // generic reductions: local mean | local M2 | local count
-  float* stat = slot + 3 * g.slots;  // mean[slots], rstd[slots]
+  float* slot = red + g.red_floats;  // generic reductions
+  float* stat = slot + g.slots;      // mean[slots], rstd[slots]
   // push exchange: two inboxes of k * slots entries (mean, M2, count, -), 16-byte aligned, and
   // their mbarriers
   float* inbox2 = stat + 2 * g.slots;
@@ -451,13 +451,11 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 6 : 2)
         for (unsigned q = 0; q < k; ++q) st_async_f32x4(inbox + 4 * (rank * g.slots + s), mbar, q, lm, m2loc, n_loc, 0.f);
       }
     } else {
-      cta_slot_moments<VE, UNI>(g, mean, m2, cnt, tx, ty, c0, nrows, g_lo, n_slots, red, tmp, slot);
-      __syncthreads();
-      for (int s = tid; pushing && s < g.slots; s += blockDim.x) {
-        const bool live = s < n_slots;
-        const float a = live ? slot[s] : 0.f, b = live ? slot[g.slots + s] : 0.f, c = live ? slot[2 * g.slots + s] : 0.f;
-        for (unsigned q = 0; q < k; ++q) st_async_f32x4(inbox + 4 * (rank * g.slots + s), mbar, q, a, b, c, 0.f);
-      }
+      const Crew cr = {tid, (int)blockDim.x, tid & 31, tid >> 5, (int)blockDim.x >> 5, 0};
+      crew_moments<VE, UNI>(cr, g, g.slots, mean, m2, cnt, tx, ty, nrows, red, slot, [&](int s, float mu, float q2) {
+        for (unsigned q = 0; pushing && q < k; ++q)
+          st_async_f32x4(inbox + 4 * (rank * g.slots + s), mbar, q, mu, q2, (float)nrows * (float)g.D, 0.f);
+      });
     }
     {
       // Every CTA of the cluster pushed (mean, M2, count) of each slot into every inbox.  Combine them
@@ -506,7 +504,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 6 : 2)
       tile_apply<T, VE, ACT>(stile, sstep, y + base, gstep, iters, a, b, refill,
                              x + (size_t)n2 * g.R * g.C + (refill ? cb2 * g.CW : 0) + row_off);
     }
-    // No barrier here: the next item's reductions write red / tmp / slot before their first
+    // No barrier here: the next item's reductions write red / slot before their first
     // barrier, none of which is read by the output pass, and `stat` is rewritten only after it.
   }
   // No exit barrier: nothing reaches into this CTA's shared memory after the wait of its last item.

@@ -82,12 +82,25 @@ int round_up4(int v) { return (v + 3) & ~3; }
 // warp-sum buffer of the shuffle reductions: one float per (warp, group slot)
 int wsum_stride_floats(int threads, int CV, int tps_shift) { return round_up4(((threads + 31) / 32) * (CV >> tps_shift)); }
 
+// Layout of the reductions in gn_reduce.cuh over rows of CW channels, whole groups of D, by `threads` threads; returns the floats
+// of their scratch.  Moments: a mean and an M2 per vector that lies in one group, or for each of the two parts of one that
+// straddles two; with groups narrower than a vector, and for sums, one value per channel.
+int reduce_layout(int CW, int CV, int ve, int D, int TY, int threads, bool moments, ReduceGeom* rd) {
+  const bool per_vector = moments && D % ve == 0, per_part = moments && !per_vector && D >= ve;
+  rd->stride = (per_vector ? CV : CW) | 1;
+  rd->div_W = make_fast_div(per_vector ? D / ve : per_part ? (D + 2 * ve - 2) / ve : D);
+  rd->part_shift = 0;
+  while (rd->part_shift < 5 && ((CW / D) << (rd->part_shift + 1)) <= threads) ++rd->part_shift;
+  return per_part ? 2 * TY * (2 * CV + 1) : TY * rd->stride * (per_vector ? 2 : 1);
+}
+
 size_t fwd_red_floats(int CW, int CV, int TY, int slots, int threads, bool shuf, int tps_shift) {
   if (shuf) {  // two warp-sum buffers, overlaid later by the gathered slot arrays of the peers
     const int a = 2 * wsum_stride_floats(threads, CV, tps_shift), b = 16 * 3 * slots;
     return (size_t)round_up4(a > b ? a : b);
   }
-  size_t r = (size_t)TY * CW;
+  size_t r = (size_t)TY * (CW | 1);  // one value per channel, or ...
+  if (r < (size_t)2 * TY * (2 * CV + 1)) r = (size_t)2 * TY * (2 * CV + 1);  // ... up to four per vector (reduce_layout)
   if (r < 1024) r = 1024;
   if (r < (size_t)16 * 3 * slots) r = (size_t)16 * 3 * slots;
   return r;
@@ -147,6 +160,7 @@ void fill_divisors(Geom* g, int ve, int direction, int threads, bool fused) {
   g->wpart_off = (direction == 1 && g->shuf) ? bwd_wpart_off(threads, g->CV, tps_shift, g->slots) : 0;
   g->red_floats = (int)(direction == 0 ? fwd_red_floats(g->CW, g->CV, g->TY, g->slots, threads, g->shuf != 0, tps_shift)
                                        : bwd_red_floats(g->CW, g->CV, g->TY, g->slots, threads, g->shuf != 0, tps_shift));
+  if (fused && direction == 0) (void)reduce_layout(g->CW, g->CV, ve, g->D, g->TY, threads, true, &g->rd);
   g->div_D = make_fast_div(g->D);
   g->div_CV = make_fast_div(g->CV);
   g->div_CW = make_fast_div(g->CW);
@@ -453,19 +467,6 @@ bool plan_wave(const Shape& sh, Plan* out) {
   return true;
 }
 
-// Layout of the reductions in gn_reduce.cuh for `threads` threads; returns the floats of their scratch: the row lanes' values
-// (forward where vectors lie in one group: a mean and an M2 per vector, else one value per channel), later the warps' sums
-// of a merge.
-int reduce_layout(const Shape& sh, int CV, int TY, int threads, ReduceGeom* ex) {
-  const bool per_vector = sh.direction == 0 && sh.D % sh.ve == 0;
-  ex->stride = (per_vector ? CV : sh.C) | 1;
-  ex->div_W = make_fast_div(per_vector ? sh.D / sh.ve : sh.D);
-  ex->part_shift = 0;
-  while (ex->part_shift < 5 && (sh.G << (ex->part_shift + 1)) <= threads) ++ex->part_shift;
-  const int rows = TY * ex->stride * (per_vector ? 2 : 1), merge = 2 * (threads / 32) * sh.G;
-  return rows > merge ? rows : merge;
-}
-
 // Resident plan (gn_resident.cu) in place of the multi-kernel or wave plan in *plan.  A sample's rows are cut into
 // cps = 148 / N contiguous ranges of whole rows, one CTA per SM; N * cps must be at least 85 % of the SMs.  Few rows
 // beyond 148 / N fill fewer (149 rows: 75 CTAs of two), and those calls stay here all the same: such short samples are
@@ -510,7 +511,8 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   g.CW = sh.C, g.CV = CV, g.TY = kResidentThreads / CV;
   g.ncb = 1, g.rows_per_cta = rows, g.chunks = cps, g.slots = sh.G, g.k = 1;
   g.persist = 1, g.skip_push_rank = -1;
-  g.red_floats = reduce_layout(sh, CV, g.TY, round_up(CV * g.TY, 32), &r.ex);
+  g.red_floats = reduce_layout(sh.C, CV, ve, sh.D, g.TY, round_up(CV * g.TY, 32), sh.direction == 0, &g.rd);
+  if (g.red_floats < 2 * (kResidentThreads / 32) * sh.G) g.red_floats = 2 * (kResidentThreads / 32) * sh.G;  // a merge's
   g.div_D = make_fast_div(sh.D);
   g.div_CV = make_fast_div(CV);
   g.div_CW = make_fast_div(sh.C);

@@ -3,7 +3,9 @@
 // What bounds them is latency: the tensors rest meanwhile.  So all groups are reduced at once, 2^part_shift neighbouring
 // threads to each, behind one barrier where a vector lies in one group.  Measured in gn_fwd_resident_kernel, from the
 // CTA's last rows to its sums: 1.0 us against 1.9 with a warp per group and one group after the other (256@512^2, 32
-// groups of 8 channels), 2.4 against 3.8 with groups of 4 channels (128@1024^2).
+// groups of 8 channels), 2.4 against 3.8 with groups of 4 channels (128@1024^2).  In the fused forward kernel, whose small
+// maps with groups of 10, 20 or 30 channels are a chain of dependent instructions, device us per call, before / now: 320@64^2
+// 9.1 / 7.6, 640@32^2 9.2 / 5.8, 2 x 960@76^2 34.5 / 24.9.
 #pragma once
 #include "gn_async.cuh"
 
@@ -30,19 +32,20 @@ __device__ __forceinline__ int chan_column(int c, int CV) {
   return (c & (VE - 1)) * CV + c / VE;
 }
 
-// Moments of every group over the crew's rows from the threads' (mean, M2) per lane of `cnt` rows each: the group's mean
-// first, then the squared deviations around it.  publish(s, mean, M2) is called by one thread per group s.
-//   red: TY * stride floats (UNI: twice), slot: G floats.  Rows ty, ty + TY, ... of the nrows belong to row lane ty.
+// Moments of every group of the column block (`groups`, all whole) over the crew's rows from the threads' (mean, M2) per
+// lane of `cnt` rows each: the group's mean first, then the squared deviations around it.  publish(s, mean, M2) is called by
+// one thread per group s.
+//   red: reduce_layout() floats, slot: one per group.  Rows ty, ty + TY, ... of the nrows belong to row lane ty.
 template <int VE, bool UNI, typename Publish>
-__device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, const ReduceGeom& ex, const float (&mean)[VE],
+__device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, int groups, const float (&mean)[VE],
                                              const float (&m2)[VE], float cnt, int tx, int ty, int nrows, float* red, float* slot,
                                              Publish publish) {
-  const int s = cr.tid >> ex.part_shift, part = cr.tid & ((1 << ex.part_shift) - 1), parts = 1 << ex.part_shift;
-  const int W = UNI ? g.D / VE : g.D, total = s < g.G ? g.TY * W : 0, lo = s * W;
+  const int s = cr.tid >> g.rd.part_shift, part = cr.tid & ((1 << g.rd.part_shift) - 1), parts = 1 << g.rd.part_shift;
+  const int W = UNI ? g.D / VE : g.D, total = s < groups ? g.TY * W : 0, lo = s * W;
   const float inv_n = 1.0f / ((float)nrows * (float)g.D);
   if constexpr (UNI) {
     const int rows_each = nrows / g.TY, more = nrows - rows_each * g.TY;  // row lanes below `more` have a row more
-    float* red2 = red + g.TY * ex.stride;
+    float* red2 = red + g.TY * g.rd.stride;
     if (ty < g.TY) {
       float mt = 0.f, qt = 0.f, dev = 0.f;
 #pragma unroll
@@ -54,26 +57,75 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, cons
         dev = fmaf(d, d, dev);
         qt += m2[e];
       }
-      red[ty * ex.stride + tx] = mt;
-      red2[ty * ex.stride + tx] = fmaf(cnt, dev, qt);
+      red[ty * g.rd.stride + tx] = mt;
+      red2[ty * g.rd.stride + tx] = fmaf(cnt, dev, qt);
     }
     cr.sync();
     float acc = 0.f;
     for (int i = part; i < total; i += parts) {
-      const int j = ex.div_W.div(i), c = i - j * W;
-      acc = fmaf((float)(rows_each + (j < more ? 1 : 0)), red[j * ex.stride + lo + c], acc);
+      const int j = g.rd.div_W.div(i), c = i - j * W;
+      acc = fmaf((float)(rows_each + (j < more ? 1 : 0)), red[j * g.rd.stride + lo + c], acc);
     }
-    const float mu = part_sum(acc, ex.part_shift) * (VE * inv_n);
+    const float mu = part_sum(acc, g.rd.part_shift) * (VE * inv_n);
     acc = 0.f;
     for (int i = part; i < total; i += parts) {
-      const int j = ex.div_W.div(i), c = i - j * W;
-      const float d = red[j * ex.stride + lo + c] - mu;
-      acc += fmaf((float)(VE * (rows_each + (j < more ? 1 : 0))) * d, d, red2[j * ex.stride + lo + c]);
+      const int j = g.rd.div_W.div(i), c = i - j * W;
+      const float d = red[j * g.rd.stride + lo + c] - mu;
+      acc += fmaf((float)(VE * (rows_each + (j < more ? 1 : 0))) * d, d, red2[j * g.rd.stride + lo + c]);
     }
-    acc = part_sum(acc, ex.part_shift);
-    if (part == 0 && s < g.G) publish(s, mu, acc);
+    acc = part_sum(acc, g.rd.part_shift);
+    if (part == 0 && s < groups) publish(s, mu, acc);
+  } else if (g.D >= VE) {
+    // a vector touches two groups at most: the thread's lanes of either are a part with a mean and an M2 of their own
+    const int rows_each = nrows / g.TY, more = nrows - rows_each * g.TY;
+    const int W = (g.D + 2 * VE - 2) / VE, pitch = 2 * g.CV + 1;  // vectors that a group can touch; parts per row, odd
+    float2* parts2 = reinterpret_cast<float2*>(red);
+    if (ty < g.TY) {
+      const int n0 = min(VE, (g.div_D.div(tx * VE) + 1) * g.D - tx * VE);  // lanes of the first part
+      float a0 = 0.f, a1 = 0.f, q0 = 0.f, q1 = 0.f, d0 = 0.f, d1 = 0.f;
+#pragma unroll
+      for (int e = 0; e < VE; ++e) {
+        a0 += e < n0 ? mean[e] : 0.f;
+        a1 += e < n0 ? 0.f : mean[e];
+      }
+      a0 = a0 / (float)n0;
+      a1 = n0 < VE ? a1 / (float)(VE - n0) : 0.f;
+#pragma unroll
+      for (int e = 0; e < VE; ++e) {
+        const float d = mean[e] - (e < n0 ? a0 : a1);
+        d0 = fmaf(e < n0 ? d : 0.f, d, d0);
+        d1 = fmaf(e < n0 ? 0.f : d, d, d1);
+        q0 += e < n0 ? m2[e] : 0.f;
+        q1 += e < n0 ? 0.f : m2[e];
+      }
+      parts2[ty * pitch + 2 * tx] = make_float2(a0, fmaf(cnt, d0, q0));
+      parts2[ty * pitch + 2 * tx + 1] = make_float2(a1, fmaf(cnt, d1, q1));
+    }
+    cr.sync();
+    const int c_lo = s * g.D, c_hi = c_lo + g.D, t_lo = c_lo / VE, entries = s < groups ? g.TY * W : 0;
+    auto entry = [&](int i, float& n, float2& v) {
+      const int j = g.rd.div_W.div(i), t = t_lo + i - j * W;
+      const int lanes = min((t + 1) * VE, c_hi) - max(t * VE, c_lo);
+      if (lanes <= 0) return false;
+      n = (float)(lanes * (rows_each + (j < more ? 1 : 0)));
+      v = parts2[j * pitch + 2 * t + (t * VE < c_lo ? 1 : 0)];
+      return true;
+    };
+    float acc = 0.f, n = 0.f;
+    float2 v = make_float2(0.f, 0.f);
+    for (int i = part; i < entries; i += parts)
+      if (entry(i, n, v)) acc = fmaf(n, v.x, acc);
+    const float mu = part_sum(acc, g.rd.part_shift) * inv_n;
+    acc = 0.f;
+    for (int i = part; i < entries; i += parts) {
+      if (!entry(i, n, v)) continue;
+      const float d = v.x - mu;
+      acc += fmaf(n * d, d, v.y);
+    }
+    acc = part_sum(acc, g.rd.part_shift);
+    if (part == 0 && s < groups) publish(s, mu, acc);
   } else {
-    float* mine = red + ty * ex.stride + tx;
+    float* mine = red + ty * g.rd.stride + tx;
     if (ty < g.TY) {
 #pragma unroll
       for (int e = 0; e < VE; ++e) mine[e * g.CV] = cnt * mean[e];
@@ -81,11 +133,11 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, cons
     cr.sync();
     float acc = 0.f;
     for (int i = part; i < total; i += parts) {
-      const int j = ex.div_W.div(i), c = lo + i - j * W;
-      acc += red[j * ex.stride + chan_column<VE>(c, g.CV)];
+      const int j = g.rd.div_W.div(i), c = lo + i - j * W;
+      acc += red[j * g.rd.stride + chan_column<VE>(c, g.CV)];
     }
-    const float mu = part_sum(acc, ex.part_shift) * inv_n;
-    if (part == 0 && s < g.G) slot[s] = mu;
+    const float mu = part_sum(acc, g.rd.part_shift) * inv_n;
+    if (part == 0 && s < groups) slot[s] = mu;
     cr.sync();
     if (ty < g.TY) {
 #pragma unroll
@@ -97,21 +149,21 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, cons
     cr.sync();
     acc = 0.f;
     for (int i = part; i < total; i += parts) {
-      const int j = ex.div_W.div(i), c = lo + i - j * W;
-      acc += red[j * ex.stride + chan_column<VE>(c, g.CV)];
+      const int j = g.rd.div_W.div(i), c = lo + i - j * W;
+      acc += red[j * g.rd.stride + chan_column<VE>(c, g.CV)];
     }
-    acc = part_sum(acc, ex.part_shift);
-    if (part == 0 && s < g.G) publish(s, mu, acc);
+    acc = part_sum(acc, g.rd.part_shift);
+    if (part == 0 && s < groups) publish(s, mu, acc);
   }
 }
 
 // Per-channel sums over the row lanes of one value per lane: chan[c].  red: TY * stride floats, stride > C.  On return
 // chan is not yet synchronised, and red may not be written before it is.
 template <int VE>
-__device__ __forceinline__ void crew_channel_sums(const Crew& cr, const Geom& g, const ReduceGeom& ex, const float (&v)[VE], int tx, int ty,
+__device__ __forceinline__ void crew_channel_sums(const Crew& cr, const Geom& g, const float (&v)[VE], int tx, int ty,
                                                   float* red, float* chan) {
   if (ty < g.TY) {
-    float* mine = red + ty * ex.stride + tx;
+    float* mine = red + ty * g.rd.stride + tx;
 #pragma unroll
     for (int e = 0; e < VE; ++e) mine[e * g.CV] = v[e];
   }
@@ -120,13 +172,13 @@ __device__ __forceinline__ void crew_channel_sums(const Crew& cr, const Geom& g,
     float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
     const float* q = red + k;
     int r = 0;
-    for (; r + 4 <= g.TY; r += 4, q += 4 * ex.stride) {
+    for (; r + 4 <= g.TY; r += 4, q += 4 * g.rd.stride) {
       a0 += q[0];
-      a1 += q[ex.stride];
-      a2 += q[2 * ex.stride];
-      a3 += q[3 * ex.stride];
+      a1 += q[g.rd.stride];
+      a2 += q[2 * g.rd.stride];
+      a3 += q[3 * g.rd.stride];
     }
-    for (; r < g.TY; ++r, q += ex.stride) a0 += q[0];
+    for (; r < g.TY; ++r, q += g.rd.stride) a0 += q[0];
     const int e = g.div_CV.div(k);
     chan[(k - e * g.CV) * VE + e] = (a0 + a1) + (a2 + a3);
   }
@@ -134,17 +186,17 @@ __device__ __forceinline__ void crew_channel_sums(const Crew& cr, const Geom& g,
 
 // gamma-weighted sums of every group over chan[0 .. C) and chan[C .. 2C); publish(s, w1, w2) by one thread per group
 template <typename Publish>
-__device__ __forceinline__ void crew_group_sums(const Crew& cr, const Geom& g, const ReduceGeom& ex, const float* gam, const float* chan,
+__device__ __forceinline__ void crew_group_sums(const Crew& cr, const Geom& g, const float* gam, const float* chan,
                                                 Publish publish) {
-  const int s = cr.tid >> ex.part_shift, part = cr.tid & ((1 << ex.part_shift) - 1), parts = 1 << ex.part_shift;
+  const int s = cr.tid >> g.rd.part_shift, part = cr.tid & ((1 << g.rd.part_shift) - 1), parts = 1 << g.rd.part_shift;
   float w1 = 0.f, w2 = 0.f;
   const int end = s < g.G ? (s + 1) * g.D : 0;
   for (int c = s * g.D + part; c < end; c += parts) {
     w1 = fmaf(gam[c], chan[c], w1);
     w2 = fmaf(gam[c], chan[g.C + c], w2);
   }
-  w1 = part_sum(w1, ex.part_shift);
-  w2 = part_sum(w2, ex.part_shift);
+  w1 = part_sum(w1, g.rd.part_shift);
+  w2 = part_sum(w2, g.rd.part_shift);
   if (part == 0 && s < g.G) publish(s, w1, w2);
 }
 

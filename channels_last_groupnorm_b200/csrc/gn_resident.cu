@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     merge_moments<VE>(pm, pq, pn, mean, m2, cnt);
   }
   const Crew cr = {tid, (int)blockDim.x, lane, warp, nwarps, 0};
-  crew_moments<VE, UNI>(cr, g, r.ex, mean, m2, cnt, tx, ty, nrows, red, slot,
+  crew_moments<VE, UNI>(cr, g, g.G, mean, m2, cnt, tx, ty, nrows, red, slot,
                         [&](int s, float mu, float q) { part[(size_t)blockIdx.x * g.G + s] = make_float2(mu, q); });
   uint4 ga_raw = make_uint4(0, 0, 0, 0), be_raw = ga_raw;
   if (streaming) {  // (they arrive during the wait)
@@ -499,11 +499,11 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     }
   }
   const Crew cr = {tid, (int)blockDim.x, lane, warp, nwarps, 0};
-  crew_channel_sums<VE>(cr, g, r.ex, s1, tx, ty, red, chan);
+  crew_channel_sums<VE>(cr, g, s1, tx, ty, red, chan);
   cr.sync();
-  crew_channel_sums<VE>(cr, g, r.ex, s2, tx, ty, red, chan + g.C);
+  crew_channel_sums<VE>(cr, g, s2, tx, ty, red, chan + g.C);
   cr.sync();
-  crew_group_sums(cr, g, r.ex, gam, chan,
+  crew_group_sums(cr, g, gam, chan,
                   [&](int s, float w1, float w2) { gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2); });
   for (int c = tid; c < g.C; c += blockDim.x) tpart[(size_t)blockIdx.x * g.C + c] = make_float2(chan[c], chan[g.C + c]);
   grid_barrier(count, sm.flags, r);
