@@ -173,6 +173,22 @@ int gnb200_fwd(const void* x, const void* gamma, const void* beta, int64_t N, in
   return GNB200_OK;
 }
 
+int gnb200_cast_params(const float* gamma, const float* beta, int64_t C, int dtype, void* gamma_out, void* beta_out,
+                       void* stream) {
+  if (dtype != GNB200_F16 && dtype != GNB200_BF16)
+    return fail(GNB200_ERR_INVALID_ARGUMENT, "gnb200_cast_params: dtype code %d is no 16-bit type (1=f16, 2=bf16)", dtype);
+  if (C < 1 || C > (1 << 24)) return fail(GNB200_ERR_INVALID_ARGUMENT, "gnb200_cast_params: C = %lld", (long long)C);
+  if (!gamma || !beta || !gamma_out || !beta_out)
+    return fail(GNB200_ERR_INVALID_ARGUMENT, "gnb200_cast_params: null pointer");
+  const cudaError_t err =
+      gnb200::launch_cast_params(gamma, beta, C, dtype, gamma_out, beta_out, reinterpret_cast<cudaStream_t>(stream));
+  if (err != cudaSuccess) {
+    (void)cudaGetLastError();
+    return fail(GNB200_ERR_CUDA, "gnb200_cast_params: CUDA error: %s", cudaGetErrorString(err));
+  }
+  return GNB200_OK;
+}
+
 // Fills *px from the caller's table of exchange buffers; `who` names the entry point in messages.
 static int make_peer_exchange(const void* const* peer_bufs, int rank, int world, int64_t C, bool collect, const char* who,
                               gnb200::PeerExchange* px) {

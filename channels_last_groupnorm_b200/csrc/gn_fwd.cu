@@ -718,6 +718,27 @@ static cudaError_t launch_fwd_ve(const FwdCall& c, const Plan& p, cudaStream_t s
   return p.ve == 1 ? launch_fwd_act<T, 1>(c, p, stream) : launch_fwd_act<T, VFULL>(c, p, stream);
 }
 
+// fp32 parameters of a call on 16-bit tensors, both in one launch (a launch each costs the host 4 us more than this kernel
+// takes: 8 x 256 x 64^2 training step with fp32 parameters 95 -> 84 us)
+template <typename T>
+__global__ void __launch_bounds__(256) gn_cast_params_kernel(const float* __restrict__ gamma, const float* __restrict__ beta,
+                                                             long long C, T* __restrict__ gamma_out, T* __restrict__ beta_out) {
+  const long long c = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (c >= C) return;
+  gamma_out[c] = store_param<T>(gamma[c]);
+  beta_out[c] = store_param<T>(beta[c]);
+}
+
+cudaError_t launch_cast_params(const float* gamma, const float* beta, int64_t C, int dtype, void* gamma_out, void* beta_out,
+                               cudaStream_t stream) {
+  const unsigned grid = (unsigned)((C + 255) / 256);
+  if (dtype == 1)
+    gn_cast_params_kernel<__half><<<grid, 256, 0, stream>>>(gamma, beta, C, (__half*)gamma_out, (__half*)beta_out);
+  else
+    gn_cast_params_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(gamma, beta, C, (__nv_bfloat16*)gamma_out, (__nv_bfloat16*)beta_out);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_forward(const FwdCall& c, const Plan& p, cudaStream_t stream) {
   if (p.resident) {
     const cudaError_t err = launch_forward_resident(c, p.rgeom, stream);

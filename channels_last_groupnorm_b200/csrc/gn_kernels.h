@@ -148,6 +148,10 @@ inline cudaError_t launch_chained(void (*kern)(KArgs...), unsigned grid, dim3 bl
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// gamma and beta, fp32, rounded to the 16-bit type `dtype`
+cudaError_t launch_cast_params(const float* gamma, const float* beta, int64_t C, int dtype, void* gamma_out, void* beta_out,
+                               cudaStream_t stream);
+
 cudaError_t launch_forward(const FwdCall& c, const Plan& p, cudaStream_t stream);
 cudaError_t launch_backward(const BwdCall& c, const Plan& p, cudaStream_t stream);
 

@@ -336,6 +336,25 @@ at::Tensor empty_vector(std::initializer_list<int64_t> sizes, at::ScalarType st,
   return at::detail::empty_cuda(at::IntArrayRef(sizes.begin(), sizes.size()), st, like.device(), std::nullopt);
 }
 
+// The parameters in X's dtype: themselves, or both rounded from fp32 in one launch, or as as_dtype() does it.
+void params_like(const at::Tensor& X, const Dense& d, at::Tensor& w, at::Tensor& b) {
+  const at::ScalarType st = X.scalar_type();
+  auto fp32_vector = [&](const at::Tensor& p) {
+    return p.scalar_type() == at::kFloat && p.dim() == 1 && p.size(0) == d.C && p.is_contiguous() && p.device() == X.device();
+  };
+  if (st == at::kFloat || !fp32_vector(w) || !fp32_vector(b)) {
+    w = as_dtype(w, st);
+    b = as_dtype(b, st);
+    return;
+  }
+  c10::cuda::CUDAGuard guard(X.device());
+  at::Tensor wc = empty_vector({d.C}, st, X), bc = empty_vector({d.C}, st, X);
+  check_status(gnb200_cast_params(w.const_data_ptr<float>(), b.const_data_ptr<float>(), d.C, dtype_code(X, "X"), wc.mutable_data_ptr(),
+                                  bc.mutable_data_ptr(), c10::cuda::getCurrentCUDAStream().stream()));
+  w = wc;
+  b = bc;
+}
+
 // Y; where `means` is given the statistics are results too, otherwise they share the scratch.
 at::Tensor direct_fwd(const at::Tensor& X, const Dense& d, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
                       int64_t act, at::Tensor* means, at::Tensor* rstds) {
@@ -412,15 +431,18 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
   static at::Tensor forward(AutogradContext* ctx, const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias,
                             int64_t G, double eps, int64_t act) {
     const bool cl = is_channels_last(X);
-    const at::Tensor w = as_dtype(weight, X.scalar_type()), b = as_dtype(bias, X.scalar_type());
+    at::Tensor w = weight, b = bias;
     ctx->saved_data["arg"] = std::vector<int64_t>{G, act, cl ? 1 : 0, (int64_t)weight.scalar_type(), (int64_t)bias.scalar_type()};
     Dense d;
     if (only_cuda_sees({&X, &w, &b}) && plain_tensor(X, &d)) {  // X itself is saved, in the order that flatten() would give
+      params_like(X, d, w, b);
       at::Tensor means, rstds;
       at::Tensor Y = direct_fwd(X, d, w, b, G, eps, act, &means, &rstds);
       ctx->save_for_backward({X, w, b, means, rstds});
       return Y;
     }
+    w = as_dtype(weight, X.scalar_type());
+    b = as_dtype(bias, X.scalar_type());
     const at::Tensor Xf = flatten(X, cl);
     auto [Y, means, rstds] = call_fwd(Xf, w, b, G, eps, act);
     ctx->save_for_backward({Xf, w, b, means, rstds});
@@ -480,7 +502,9 @@ at::Tensor group_norm_act_direct(const at::Tensor& X, const at::Tensor& weight, 
   if (c10::GradMode::is_enabled() && (X.requires_grad() || weight.requires_grad() || bias.requires_grad()))
     return GnFunction::apply(X, weight, bias, G, eps, act);
   at::AutoDispatchBelowADInplaceOrView guard;
-  return direct_fwd(X, d, as_dtype(weight, X.scalar_type()), as_dtype(bias, X.scalar_type()), G, eps, act, nullptr, nullptr);
+  at::Tensor w = weight, b = bias;
+  params_like(X, d, w, b);
+  return direct_fwd(X, d, w, b, G, eps, act, nullptr, nullptr);
 }
 
 // below autograd (inference mode)

@@ -88,6 +88,12 @@ int gnb200_fwd(const void* x, const void* gamma, const void* beta,
                void* y, float* mean, float* rstd,
                void* workspace, size_t workspace_bytes, void* stream);
 
+/* gamma and beta (C floats each) rounded to nearest to the 16-bit type `dtype` (GNB200_F16 or GNB200_BF16), in one launch:
+ * for callers that keep fp32 parameters beside 16-bit tensors. */
+int gnb200_cast_params(const float* gamma, const float* beta, int64_t C, int dtype, void* gamma_out, void* beta_out,
+                       void* stream);
+
+
 /*
  * Backward.  Reads dy, x, gamma, beta and the mean/rstd written by gnb200_fwd.
  * Writes dx (N*R*C) and the parameter gradients:
