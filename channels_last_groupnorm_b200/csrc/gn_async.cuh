@@ -128,7 +128,7 @@ __device__ __forceinline__ void bulk_load_once(uint32_t smem_dst, const void* sr
 
 // dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half
 // precision, dx = ag * dyh + c1 * x + c2.
-template <typename T, int ACT>
+template <typename T, int ACT, bool PAIRS = true>
 __device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw, const float (&a)[8],
                                                const float (&b)[8], const float (&ag)[8], const float (&c1)[8],
                                                const float (&c2)[8]) {
@@ -141,14 +141,24 @@ __device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw,
     float g0 = 1.f, g1 = 1.f;
     if constexpr (ACT != kActIdentity) {
       float yh0, yh1;
-      fma2(yh0, yh1, fx[2 * p], fx[2 * p + 1], a[2 * p], a[2 * p + 1], b[2 * p], b[2 * p + 1]);
+      if constexpr (PAIRS) {
+        fma2(yh0, yh1, fx[2 * p], fx[2 * p + 1], a[2 * p], a[2 * p + 1], b[2 * p], b[2 * p + 1]);
+      } else {
+        yh0 = fmaf(fx[2 * p], a[2 * p], b[2 * p]);
+        yh1 = fmaf(fx[2 * p + 1], a[2 * p + 1], b[2 * p + 1]);
+      }
       const float2 gf = __half22float2(act_grad_pair<ACT>(yh0, yh1));
       g0 = gf.x;
       g1 = gf.y;
     }
-    float t0, t1;
-    fma2(t0, t1, c1[2 * p], c1[2 * p + 1], fx[2 * p], fx[2 * p + 1], c2[2 * p], c2[2 * p + 1]);
-    fma2(o[2 * p], o[2 * p + 1], ag[2 * p], ag[2 * p + 1], fd[2 * p] * g0, fd[2 * p + 1] * g1, t0, t1);
+    if constexpr (PAIRS) {
+      float t0, t1;
+      fma2(t0, t1, c1[2 * p], c1[2 * p + 1], fx[2 * p], fx[2 * p + 1], c2[2 * p], c2[2 * p + 1]);
+      fma2(o[2 * p], o[2 * p + 1], ag[2 * p], ag[2 * p + 1], fd[2 * p] * g0, fd[2 * p + 1] * g1, t0, t1);
+    } else {
+      o[2 * p] = fmaf(ag[2 * p], fd[2 * p] * g0, fmaf(c1[2 * p], fx[2 * p], c2[2 * p]));
+      o[2 * p + 1] = fmaf(ag[2 * p + 1], fd[2 * p + 1] * g1, fmaf(c1[2 * p + 1], fx[2 * p + 1], c2[2 * p + 1]));
+    }
   }
   return pack16<T, 8>(o);
 }

@@ -266,7 +266,8 @@ __device__ __forceinline__ void bwd_row_sums(const float (&fx)[VE], float (&fd)[
 // the format it is parked in anyway - and enters the fp32 sums through mixed-precision add / fma,
 // so dy is never unpacked and dyh never packed.  act' is evaluated in f16x2; for bf16 tensors it
 // is rounded to bf16 before the product.  Returns the packed dyh.
-template <typename T, int ACT>
+// PAIRS: packed fp32 instructions, which want their operands in register pairs.
+template <typename T, int ACT, bool PAIRS = true>
 __device__ __forceinline__ uint4 bwd_row_sums_packed(const uint4& xw, const uint4& dw, const float (&a)[8],
                                                      const float (&b)[8], float (&s1)[8], float (&s2)[8]) {
   static_assert(sizeof(T) == 2, "16-bit tensors only");
@@ -279,7 +280,12 @@ __device__ __forceinline__ uint4 bwd_row_sums_packed(const uint4& xw, const uint
     uint32_t dyh = dr[p];
     if constexpr (ACT != kActIdentity) {
       float yh0, yh1;
-      fma2(yh0, yh1, mixed_add<T>(x0, -0.0f), mixed_add<T>(x1, -0.0f), a[2 * p], a[2 * p + 1], b[2 * p], b[2 * p + 1]);
+      if constexpr (PAIRS) {
+        fma2(yh0, yh1, mixed_add<T>(x0, -0.0f), mixed_add<T>(x1, -0.0f), a[2 * p], a[2 * p + 1], b[2 * p], b[2 * p + 1]);
+      } else {
+        yh0 = fmaf(mixed_add<T>(x0, -0.0f), a[2 * p], b[2 * p]);
+        yh1 = fmaf(mixed_add<T>(x1, -0.0f), a[2 * p + 1], b[2 * p + 1]);
+      }
       const __half2 g = act_grad_pair<ACT>(yh0, yh1);
       if constexpr (std::is_same<T, __half>::value) {
         const __half2 r = __hmul2(*reinterpret_cast<const __half2*>(&dr[p]), g);

@@ -537,7 +537,9 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   // 128@1024^2 143.5 / 139.1; backward 512@256^2 64.8 / 63.8, bf16 75 MB 72.0 / 71.0, but 256@512^2 119.2 / 121.0 and
   // 128@1024^2 228.7 / 234.0: with x and dy of twice L2 what is found there is what the second reads leave behind.
   r.evict = sh.direction == 0 || 2.0 * sh.N * sh.R * sh.C * s <= 192.0 * 1024 * 1024;
-  r.park = env_int("GNB200_RESIDENT_PARK", max_stages < 16 ? 0 : kResidentPark);
+  // Tensor memory, without / with: forward 512@256^2 39.1 / 35.0, 256@512^2 72.5 / 67.3, 128@1024^2 144.1 / 139.4; backward
+  // 512@256^2 66.7 / 63.8, bf16 75 MB 73.5 / 70.7, then nothing (256@512^2 118.4 / 118.3, 3 x 61 MB 160.4 / 161.6).
+  r.park = env_int("GNB200_RESIDENT_PARK", max_stages < 16 || !r.evict ? 0 : kResidentPark);
   if (r.park < 0 || r.park > kResidentPark) r.park = kResidentPark;
   r.smem_bytes = fixed + (size_t)r.stages * stage;
   r.ws_bytes = resident_workspace_bytes(r, sh.direction);

@@ -75,6 +75,7 @@ struct Stream {
   const T* src[NT];  // x (and dy): first element of the CTA's row range
   int tiles, nrows, BR, stages;
   uint32_t row_bytes, tile_bytes;
+  uint64_t policy;  // evict-first; made by thread 0 for each of its copies it cost 2 us (128@1024^2 backward 227.7 -> 225.5)
   unsigned full_ph, empty_ph, last_ph;  // last_ph: the phase of each stage's last copy
   Smem sm;
 
@@ -83,15 +84,16 @@ struct Stream {
     const uint32_t bytes = (uint32_t)min(BR, nrows - t * BR) * row_bytes;
     last_ph ^= 1u << stage;
     mbar_arrive_expect_tx(&sm.full[stage], NT * bytes);
-    const uint64_t policy = evict_first_policy();
+    const uint32_t dst = sm.stage0 + (uint32_t)(stage * NT) * tile_bytes;
+    const size_t at = (size_t)t * tile_bytes;
+    if (once) {
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
-      const uint32_t dst = sm.stage0 + (uint32_t)(stage * NT + i) * tile_bytes;
-      const char* from = reinterpret_cast<const char*>(src[i]) + (size_t)t * tile_bytes;
-      if (once)
-        bulk_load_once(dst, from, bytes, &sm.full[stage], policy);
-      else
-        bulk_load(dst, from, bytes, &sm.full[stage]);
+      for (int i = 0; i < NT; ++i)
+        bulk_load_once(dst + i * tile_bytes, reinterpret_cast<const char*>(src[i]) + at, bytes, &sm.full[stage], policy);
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+        bulk_load(dst + i * tile_bytes, reinterpret_cast<const char*>(src[i]) + at, bytes, &sm.full[stage]);
     }
   }
   // thread 0: waits until every warp has handed the stage back, then refills it.  Without the hand-back
@@ -147,6 +149,7 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
   st.tile_bytes = (uint32_t)r.tile_bytes;
   st.full_ph = st.empty_ph = 0;
   st.last_ph = ~0u;
+  st.policy = evict_first_policy();
   st.parked = max(0, min(r.park, st.tiles - r.stages));
   st.held0 = max(0, st.tiles - r.stages - st.parked);
   const int alloc_warp = 1 % (int)(blockDim.x >> 5);  // not the one that issues the copies, where there is another
@@ -404,7 +407,9 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
                            const ResidentGeom r) {
   constexpr int VE = 16 / sizeof(T);
   constexpr int KR = resident_rows(1);
-  constexpr bool kRaw = sizeof(T) == 2;  // 16-bit tensors: packed arithmetic, S2 against the raw x
+  // 16-bit tensors: packed arithmetic, S2 against the raw x.  Packed fp32 pairs only where a vector has one rstd and one mean: with
+  // eight of each the registers are short (128@1024^2: 229.0 us with them, 227.7 without)
+  constexpr bool kRaw = sizeof(T) == 2;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const Geom& g = r.g;
   const Smem sm = carve<2>(r, smem_raw);
@@ -475,7 +480,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       for (int u = 0; u < KR; ++u) {
         if (my_row + u * g.TY < here) {
           if constexpr (kRaw) {
-            bwd_row_sums_packed<T, ACT>(xw[u], dw[u], a, b, p1, p2);
+            bwd_row_sums_packed<T, ACT, UNI>(xw[u], dw[u], a, b, p1, p2);
           } else {
             float fx[VE], fd[VE];
             unpack16<T, VE>(xw[u], fx);
@@ -550,7 +555,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     for (int u = 0; u < KR; ++u) {
       if (my_row + u * g.TY < here) {
         if constexpr (kRaw) {
-          stg128_stream(o + (size_t)u * ostep, bwd_dx_packed<T, ACT>(xw[u], dw[u], a, b, a, c1, c2));
+          stg128_stream(o + (size_t)u * ostep, bwd_dx_packed<T, ACT, UNI>(xw[u], dw[u], a, b, a, c1, c2));
         } else {
           float fx[VE], fd[VE], xh[VE], yh[VE], gr[VE];
           unpack16<T, VE>(xw[u], fx);
