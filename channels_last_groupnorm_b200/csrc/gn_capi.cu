@@ -158,7 +158,7 @@ int gnb200_fwd(const void* x, const void* gamma, const void* beta, int64_t N, in
   gnb200::Plan plan;
   // the vector kernels read x, y, gamma and beta with 16-byte accesses: all four must be aligned
   const bool al = aligned16(x) && aligned16(y) && aligned16(gamma) && aligned16(beta);
-  if (!gnb200::make_plan(N, R, C, G, dtype, 0, al, &plan))
+  if (!gnb200::make_plan(N, R, C, G, dtype, 0, al, &plan, workspace && aligned16(workspace) ? workspace_bytes : 0))
     return fail(GNB200_ERR_UNSUPPORTED, "gnb200_fwd: shape N=%lld R=%lld C=%lld G=%lld is outside the supported index range",
                 (long long)N, (long long)R, (long long)C, (long long)G);
   if (plan.ws_bytes > 0 && (!workspace || workspace_bytes < plan.ws_bytes || !aligned16(workspace)))
@@ -228,7 +228,7 @@ static int bwd_impl(const char* who, const void* dy, const void* x, const void* 
     return fail(GNB200_ERR_INVALID_ARGUMENT, "%s: null tensor pointer", who);
   gnb200::Plan plan;
   const bool al = aligned16(x) && aligned16(dy) && aligned16(dx) && aligned16(gamma) && aligned16(beta);
-  if (!gnb200::make_plan(N, R, C, G, dtype, 1, al, &plan))
+  if (!gnb200::make_plan(N, R, C, G, dtype, 1, al, &plan, workspace && aligned16(workspace) ? workspace_bytes : 0))
     return fail(GNB200_ERR_UNSUPPORTED, "%s: shape N=%lld R=%lld C=%lld G=%lld is outside the supported index range", who,
                 (long long)N, (long long)R, (long long)C, (long long)G);
   if (plan.ws_bytes > 0 && (!workspace || workspace_bytes < plan.ws_bytes || !aligned16(workspace)))
@@ -487,7 +487,7 @@ int gnb200_selftest_exchange_timeout(const void* x, const void* gamma, const voi
     return fail(GNB200_ERR_INVALID_ARGUMENT, "gnb200_selftest_exchange_timeout: null tensor pointer");
   gnb200::Plan plan;
   const bool al = aligned16(x) && aligned16(y) && aligned16(gamma) && aligned16(beta);
-  if (!gnb200::make_plan(N, R, C, G, dtype, 0, al, &plan) || !plan.fused || plan.geom.k < 2)
+  if (!gnb200::make_plan(N, R, C, G, dtype, 0, al, &plan, 0) || !plan.fused || plan.geom.k < 2)
     return fail(GNB200_ERR_UNSUPPORTED,
                 "gnb200_selftest_exchange_timeout: the problem must take the fused forward plan with a cluster of at "
                 "least two CTAs");

@@ -18,6 +18,7 @@ struct Plan {
   size_t smem_bytes;  // dynamic shared memory of the first streaming kernel
   size_t ws_bytes;    // scratch bytes this plan needs
   int launches;       // kernels enqueued per call
+  bool over_fused;    // multi-pass although there is a fused plan (make_plan with less scratch gives that one)
   bool chain;         // kernels after the first are launched as programmatic dependents of their predecessor
   Geom geom;
   WaveGeom wgeom;
@@ -65,7 +66,10 @@ struct BwdCall {
 
 // direction: 0 forward, 1 backward.  `aligned16`: every tensor pointer is 16-byte aligned.
 // Returns false (and leaves *plan untouched) if the shape cannot be indexed.
-bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan);
+// `scratch`: what the caller gives; a multi-pass plan that needs more makes way for the fused one where it was only the
+// faster choice.
+bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan,
+               size_t scratch = (size_t)-1);
 
 // Largest scratch requirement over the plans the library may pick for this problem.
 size_t plan_workspace_bytes(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction);

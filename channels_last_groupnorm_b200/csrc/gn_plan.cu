@@ -284,6 +284,22 @@ bool plan_fused(const Shape& sh, Plan* out) {
   return found;
 }
 
+// Where the multi-pass plans win although the slab fits a cluster: one CTA of the cluster fills an SM, and it reads
+// row segments of at most 64 bytes out of wider rows, so the DRAM bursts are shared with column blocks that come another time.
+// Measured on B200, device us, fused / multi-pass, forward and backward:
+//   fp16  256@256^2 (16-byte segments) 55.5 / 22.7, 91.7 / 34.9    128@256^2 57.7 / 17.6, 60.5 / 26.8    512@192^2 (32 bytes) 35.6 /
+//   24.3, 63.4 / 39.0    256 x 32768 rows 22.1 / 16.3, 36.3 / 26.6    512 x 28700 rows (64 bytes) 25.0 / 22.2, 49.7 / 33.1
+//   bf16  2 x 256@200^2 38.5 / 26.0, 66.7 / 43.0    fp32  2 x 48 x 25164 rows, 9.7 MB 15.7 / 12.4, 23.5 / 23.0
+// The other sides: two CTAs per SM  3 x 256 x 11696 rows 11.5 / 16.9, 18.7 / 24.7; wide segments  4 x 2560@88^2 (160 bytes) 101 /
+// 102, 147 / 185; whole rows  12 x 12 x 25745 rows fp32 11.5 / 14.6; and below 2 MB, where the launches decide: bf16
+// 24 x 40000 rows, 1.9 MB 12.5 / 9.3, 16.0 / 16.4 (16 x 65536 rows fp16, 2.1 MB 20.2 / 9.9, 23.9 / 16.4).
+bool fused_loses(const Shape& sh, const Plan& p) {
+  const int cw = p.geom.CW;
+  return sh.ve > 1 && cw < sh.C && cw * sh.s <= 64 && p.smem_bytes > (kSmemMaxOptin - 1024) / 2 &&
+         (double)sh.N * sh.R * sh.C * sh.s >= 2e6 && env_int("GNB200_CW", 0) == 0 && env_int("GNB200_K", 0) == 0 &&
+         env_int("GNB200_THREADS", 0) == 0;
+}
+
 bool plan_two_pass(const Shape& sh, Plan* out) {
   const int ve = sh.ve, s = sh.s;
   const int target_threads = env_int("GNB200_THREADS", 256);
@@ -556,7 +572,7 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
 
 }  // namespace
 
-static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan);
+static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, bool fused_only, Plan* plan);
 static bool plan_streaming(const Shape& sh, bool twopass_only, bool wave_only, Plan* plan);
 
 // Plans a thread has made lately: a plan is a function of these seven numbers alone (no pointer, no device state),
@@ -579,10 +595,9 @@ struct PlanEntry {
 constexpr unsigned kPlanEntries = 64;
 static thread_local PlanEntry t_plans[kPlanEntries];
 
-bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan) {
-  t_overrides = overrides_present();
+static bool make_plan_any(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan) {
   if (t_overrides) {
-    if (!make_plan_inner(N, R, C, G, dtype, direction, aligned16, plan)) return false;
+    if (!make_plan_inner(N, R, C, G, dtype, direction, aligned16, false, plan)) return false;
     // GNB200_CHAIN = 0: every kernel of a call waits for the whole previous kernel (plain stream order)
     plan->chain = env_int("GNB200_CHAIN", 1) != 0;
     return true;
@@ -594,7 +609,7 @@ bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direct
   PlanEntry& entry = t_plans[h % kPlanEntries];
   if (!entry.used || !(entry.key == key)) {
     Plan made;
-    if (!make_plan_inner(N, R, C, G, dtype, direction, aligned16, &made)) return false;
+    if (!make_plan_inner(N, R, C, G, dtype, direction, aligned16, false, &made)) return false;
     made.chain = true;
     entry.plan = made;
     entry.key = key;
@@ -604,12 +619,22 @@ bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direct
   return true;
 }
 
+bool make_plan(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan, size_t scratch) {
+  t_overrides = overrides_present();
+  if (!make_plan_any(N, R, C, G, dtype, direction, aligned16, plan)) return false;
+  if (!plan->over_fused || plan->ws_bytes <= scratch) return true;
+  const bool chain = plan->chain;
+  if (!make_plan_inner(N, R, C, G, dtype, direction, aligned16, true, plan)) return false;
+  plan->chain = chain;
+  return true;
+}
+
 bool chain_enabled() {
   t_overrides = overrides_present();
   return env_int("GNB200_CHAIN", 1) != 0;
 }
 
-static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, Plan* plan) {
+static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction, bool aligned16, bool fused_only, Plan* plan) {
   if (N < 1 || R < 1 || C < 1 || G < 1 || C % G != 0) return false;
   if (N > 0x7fffffffLL || R > 0x7fffffffLL || C > (1 << 24) || (long long)N * G > 0x7fffffffLL) return false;
   if ((double)N * (double)R * (double)C > 9.0e15) return false;
@@ -628,7 +653,15 @@ static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
   const bool twopass_only = force && !strcmp(force, "twopass");
   const bool wave_only = force && !strcmp(force, "wave"), resident_only = force && !strcmp(force, "resident");
   const bool streaming_only = force && !strcmp(force, "streaming");
-  if (!twopass_only && !wave_only && !resident_only && !streaming_only && plan_fused(sh, plan)) return true;
+  if (!twopass_only && !wave_only && !resident_only && !streaming_only && plan_fused(sh, plan)) {
+    if (fused_only || (force && !strcmp(force, "fused")) || !fused_loses(sh, *plan)) return true;
+    Plan other;
+    if (!plan_streaming(sh, false, false, &other)) return true;
+    *plan = other;
+    plan_resident(sh, false, plan);
+    plan->over_fused = true;
+    return true;
+  }
   if (!plan_streaming(sh, twopass_only, wave_only, plan)) return false;
   if (!twopass_only && !wave_only) plan_resident(sh, resident_only, plan);
   return true;

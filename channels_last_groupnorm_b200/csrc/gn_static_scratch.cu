@@ -85,7 +85,7 @@ extern "C" int gnb200_bwd_static_scratch(const void* dy, const void* x, const vo
                                 "for its peers; see gnb200_wait_timeouts() / gnb200_clear_wait_timeouts()");
   gnb200::Plan plan;
   const bool al = is_aligned16(x) && is_aligned16(dy) && is_aligned16(dx) && is_aligned16(gamma) && is_aligned16(beta);
-  if (!gnb200::make_plan(N, R, C, G, dtype, 1, al, &plan))
+  if (!gnb200::make_plan(N, R, C, G, dtype, 1, al, &plan, (size_t)GNB200_STATIC_SCRATCH_BYTES))
     return gnb200::report_error(GNB200_ERR_UNSUPPORTED,
                                 "gnb200_bwd_static_scratch: shape N=%lld R=%lld C=%lld G=%lld is outside the supported "
                                 "index range",
