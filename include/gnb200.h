@@ -81,7 +81,8 @@ size_t gnb200_bwd_workspace_bytes(int64_t N, int64_t R, int64_t C, int64_t G, in
  * Forward:  y = act(gamma * (x - mean) * rstd + beta), statistics per (sample, group) over the
  * R * (C/G) elements of the slab, biased variance, rstd = 1/sqrt(var + eps).
  * Writes y (N*R*C), mean and rstd (N*G floats each).  `workspace` may be NULL when
- * gnb200_fwd_workspace_bytes() is 0.  `stream` is a cudaStream_t (NULL = default stream).
+ * gnb200_fwd_workspace_bytes() is 0, and also where a plan without scratch exists beside the faster one that the
+ * query is for: that one runs then.  `stream` is a cudaStream_t (NULL = default stream).
  */
 int gnb200_fwd(const void* x, const void* gamma, const void* beta,
                int64_t N, int64_t R, int64_t C, int64_t G, double eps, int act, int dtype,
