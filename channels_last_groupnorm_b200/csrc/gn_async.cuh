@@ -128,7 +128,7 @@ __device__ __forceinline__ void bulk_load_once(uint32_t smem_dst, const void* sr
 
 // dx of one 16-byte vector of a 16-bit tensor: dyh = dy * act'(x a + b) with act' in packed half
 // precision, dx = ag * dyh + c1 * x + c2.
-template <typename T, int ACT, bool PAIRS = true>
+template <typename T, int ACT, bool PAIRS = kPairs<T>>
 __device__ __forceinline__ uint4 bwd_dx_packed(const uint4& xw, const uint4& dw, const float (&a)[8],
                                                const float (&b)[8], const float (&ag)[8], const float (&c1)[8],
                                                const float (&c2)[8]) {

@@ -272,9 +272,16 @@ __device__ __forceinline__ void tile_bwd_dx(const T* __restrict__ gx, uint32_t r
       }
       cp_async_commit();
       if constexpr (kFold) {
-        affine<VE>(fx, c1, c2);
+        if constexpr (kPairs<T>) {
 #pragma unroll
-        for (int e = 0; e < VE; e += 2) fma2(fx[e], fx[e + 1], ag[e], ag[e + 1], fd[e], fd[e + 1], fx[e], fx[e + 1]);
+          for (int e = 0; e < VE; e += 2) {
+            fma2(fx[e], fx[e + 1], c1[e], c1[e + 1], fx[e], fx[e + 1], c2[e], c2[e + 1]);
+            fma2(fx[e], fx[e + 1], ag[e], ag[e + 1], fd[e], fd[e + 1], fx[e], fx[e + 1]);
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < VE; ++e) fx[e] = fmaf(ag[e], fd[e], fmaf(c1[e], fx[e], c2[e]));
+        }
       } else {
 #pragma unroll
         for (int e = 0; e < VE; ++e) {

@@ -341,7 +341,10 @@ __device__ __forceinline__ void stream_apply_back(const Pack<T, VE>* __restrict_
 //               [2 inboxes of k*slots entries of 4 floats][2 mbarriers][dead flag]
 // ------------------------------------------------------------------------------------------------
 // MAXT: CTA size class.  128-thread launches are compiled for six CTAs per SM (<= 80 registers).
-template <typename T, int VE, int ACT, bool UNI, int MAXT>
+// SHUF: the shuffle reductions (Geom::shuf) are compiled in instead of the generic ones.  Both in one kernel, chosen at run time, cost
+// registers; device us, before / now: 64 x 256@64^2 bf16 GELU 54.8 / 53.3, fp16 SiLU 50.9 / 48.4, 24 x 256 x 5000 rows bf16 31.9 / 29.3,
+// 11 x 512@73^2 30.4 / 27.4, 6 x 1024 x 6000 rows 35.8 / 32.5, 50 x 256@50^2 30.5 / 28.1, 10 x 512@75^2 fp16 28.3 / 25.4.
+template <typename T, int VE, int ACT, bool UNI, int MAXT, bool SHUF>
 __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 6 : 2)
     gn_fwd_fused_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
                         T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps,
@@ -430,7 +433,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 6 : 2)
     first = false;
     int g_lo, n_slots;
     cb_groups(g, c0, g_lo, n_slots);
-    if (UNI && g.shuf) {
+    if constexpr (SHUF) {
       // shuffle reductions: red doubles as the two warp-sum buffers
       float sm = 0.f;
 #pragma unroll
@@ -639,7 +642,11 @@ __global__ void __launch_bounds__(kMaxThreads)
 // ------------------------------------------------------------------------------------------------
 template <typename T, int VE, int ACT, bool UNI>
 static cudaError_t launch_fused(const FwdCall& c, const Plan& p, cudaStream_t stream) {
-  auto kern = p.threads <= 128 ? gn_fwd_fused_kernel<T, VE, ACT, UNI, 128> : gn_fwd_fused_kernel<T, VE, ACT, UNI, kMaxThreads>;
+  auto kern = p.threads <= 128 ? gn_fwd_fused_kernel<T, VE, ACT, UNI, 128, false> : gn_fwd_fused_kernel<T, VE, ACT, UNI, kMaxThreads, false>;
+  if constexpr (UNI && VE >= 4) {
+    if (p.geom.shuf)
+      kern = p.threads <= 128 ? gn_fwd_fused_kernel<T, VE, ACT, UNI, 128, true> : gn_fwd_fused_kernel<T, VE, ACT, UNI, kMaxThreads, true>;
+  }
   cudaError_t err = ensure_kernel_attributes((const void*)kern, p.smem_bytes, p.geom.k > 8);
   if (err != cudaSuccess) return err;
   cudaLaunchConfig_t cfg = {};

@@ -267,7 +267,7 @@ __device__ __forceinline__ void bwd_row_sums(const float (&fx)[VE], float (&fd)[
 // so dy is never unpacked and dyh never packed.  act' is evaluated in f16x2; for bf16 tensors it
 // is rounded to bf16 before the product.  Returns the packed dyh.
 // PAIRS: packed fp32 instructions, which want their operands in register pairs.
-template <typename T, int ACT, bool PAIRS = true>
+template <typename T, int ACT, bool PAIRS = kPairs<T>>
 __device__ __forceinline__ uint4 bwd_row_sums_packed(const uint4& xw, const uint4& dw, const float (&a)[8],
                                                      const float (&b)[8], float (&s1)[8], float (&s2)[8]) {
   static_assert(sizeof(T) == 2, "16-bit tensors only");

@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
       for (int u = 0; u < KR; ++u) {
         if (my_row + u * g.TY < here) {
           if constexpr (kRaw) {
-            bwd_row_sums_packed<T, ACT, UNI>(xw[u], dw[u], a, b, p1, p2);
+            bwd_row_sums_packed<T, ACT, UNI && kPairs<T>>(xw[u], dw[u], a, b, p1, p2);
           } else {
             float fx[VE], fd[VE];
             unpack16<T, VE>(xw[u], fx);
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     for (int u = 0; u < KR; ++u) {
       if (my_row + u * g.TY < here) {
         if constexpr (kRaw) {
-          stg128_stream(o + (size_t)u * ostep, bwd_dx_packed<T, ACT, UNI>(xw[u], dw[u], a, b, a, c1, c2));
+          stg128_stream(o + (size_t)u * ostep, bwd_dx_packed<T, ACT, UNI && kPairs<T>>(xw[u], dw[u], a, b, a, c1, c2));
         } else {
           float fx[VE], fd[VE], xh[VE], yh[VE], gr[VE];
           unpack16<T, VE>(xw[u], fx);
