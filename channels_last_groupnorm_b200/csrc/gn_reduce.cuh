@@ -41,7 +41,7 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, int 
                                              const float (&m2)[VE], float cnt, int tx, int ty, int nrows, float* red, float* slot,
                                              Publish publish) {
   const int s = cr.tid >> g.rd.part_shift, part = cr.tid & ((1 << g.rd.part_shift) - 1), parts = 1 << g.rd.part_shift;
-  const int W = UNI ? g.D / VE : g.D, total = s < groups ? g.TY * W : 0, lo = s * W;
+  const int W = UNI ? g.D / VE : g.D, total = s < groups ? g.TY * W : 0, lo = s * W;  // (no more groups than threads if D >= VE)
   const float inv_n = 1.0f / ((float)nrows * (float)g.D);
   if constexpr (UNI) {
     const int rows_each = nrows / g.TY, more = nrows - rows_each * g.TY;  // row lanes below `more` have a row more
@@ -131,13 +131,21 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, int 
       for (int e = 0; e < VE; ++e) mine[e * g.CV] = cnt * mean[e];
     }
     cr.sync();
-    float acc = 0.f;
-    for (int i = part; i < total; i += parts) {
-      const int j = g.rd.div_W.div(i), c = lo + i - j * W;
-      acc += red[j * g.rd.stride + chan_column<VE>(c, g.CV)];
+    // A CTA can have more of these groups than threads (64 samples of 25 rows x 1280 channels, one a group: 160 groups a block, 128
+    // threads), so the threads walk over them; all make the same number of rounds, since part_sum wants whole warps.
+    const int step = cr.threads >> g.rd.part_shift;
+    auto group_sum = [&](int grp) {
+      float acc = 0.f;
+      for (int i = part; i < (grp < groups ? g.TY * W : 0); i += parts) {
+        const int j = g.rd.div_W.div(i), c = grp * W + i - j * W;
+        acc += red[j * g.rd.stride + chan_column<VE>(c, g.CV)];
+      }
+      return part_sum(acc, g.rd.part_shift);
+    };
+    for (int s0 = 0; s0 < groups; s0 += step) {
+      const float mu = group_sum(s0 + s) * inv_n;
+      if (part == 0 && s0 + s < groups) slot[s0 + s] = mu;
     }
-    const float mu = part_sum(acc, g.rd.part_shift) * inv_n;
-    if (part == 0 && s < groups) slot[s] = mu;
     cr.sync();
     if (ty < g.TY) {
 #pragma unroll
@@ -147,13 +155,10 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, int 
       }
     }
     cr.sync();
-    acc = 0.f;
-    for (int i = part; i < total; i += parts) {
-      const int j = g.rd.div_W.div(i), c = lo + i - j * W;
-      acc += red[j * g.rd.stride + chan_column<VE>(c, g.CV)];
+    for (int s0 = 0; s0 < groups; s0 += step) {
+      const float q = group_sum(s0 + s);
+      if (part == 0 && s0 + s < groups) publish(s0 + s, slot[s0 + s], q);
     }
-    acc = part_sum(acc, g.rd.part_shift);
-    if (part == 0 && s < groups) publish(s, mu, acc);
   }
 }
 
