@@ -93,8 +93,8 @@ __device__ __forceinline__ void crew_moments(const Crew& cr, const Geom& g, int 
 #pragma unroll
       for (int e = 0; e < VE; ++e) {
         const float d = mean[e] - (e < n0 ? a0 : a1);
-        d0 = fmaf(e < n0 ? d : 0.f, d, d0);
-        d1 = fmaf(e < n0 ? 0.f : d, d, d1);
+        d0 = e < n0 ? fmaf(d, d, d0) : d0;  // (chosen, not multiplied by 0: the other part's d may be infinite or NaN)
+        d1 = e < n0 ? d1 : fmaf(d, d, d1);
         q0 += e < n0 ? m2[e] : 0.f;
         q1 += e < n0 ? 0.f : m2[e];
       }
