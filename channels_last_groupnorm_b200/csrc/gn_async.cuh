@@ -48,35 +48,44 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
 // between two passes: 512 columns of 128 lanes x 4 bytes.  A warp reaches the 32 lanes of its rank in its warpgroup, so
 // the warpgroups of a CTA share the columns out and a thread has kTmemColumns words of its own, i.e. 32 vectors of 16
 // bytes that nobody else touches: a store and the load that gets it back need no barrier, only wait::st.
+// All these instructions want a whole converged warp, and lane 0 of warp 0 comes back from code of its own (the copies), so
+// each begins with a __syncwarp.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTmemColumns = 128;                  // per warpgroup, hence words per thread
 constexpr uint32_t kTmemTotal = 4 * kTmemColumns;  // all of the SM's
 
 // by one whole warp; the base address is valid for the CTA's threads after their next __syncthreads
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_slot) {
+  __syncwarp();
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(smem_slot)), "r"(kTmemTotal)
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
-// by the same warp, when every thread of the CTA is done with its words
+// by the same warp, when every thread of the CTA is done with its words: its stores have been waited for too
 __device__ __forceinline__ void tmem_free(uint32_t base) {
+  __syncwarp();
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(kTmemTotal) : "memory");
 }
 // the calling thread's first word: lane in bits 31..16, column below
 __device__ __forceinline__ uint32_t tmem_own(uint32_t base, int warp) {
   return base + ((uint32_t)(warp & 3) << 21) + (uint32_t)(warp >> 2) * kTmemColumns;
 }
-// 16 words from column `col` of the thread's own on; whole converged warps
+// 16 words from column `col` of the thread's own on
 __device__ __forceinline__ void tmem_store16(uint32_t col, const uint4& a, const uint4& b, const uint4& c, const uint4& d) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(col),
       "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w),
       "r"(d.x), "r"(d.y), "r"(d.z), "r"(d.w)
       : "memory");
 }
-__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_store_wait() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 // the same 16 words back; load and wait are one statement, so that no use of them moves in between
 __device__ __forceinline__ void tmem_load16(uint32_t col, uint4& a, uint4& b, uint4& c, uint4& d) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
       "tcgen05.wait::ld.sync.aligned;"

@@ -153,7 +153,6 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
   st.parked = max(0, min(r.park, st.tiles - r.stages));
   st.held0 = max(0, st.tiles - r.stages - st.parked);
   const int alloc_warp = 1 % (int)(blockDim.x >> 5);  // not the one that issues the copies, where there is another
-  __syncwarp();
   if (st.parked && (int)(threadIdx.x >> 5) == alloc_warp) tmem_alloc(reinterpret_cast<uint32_t*>(&sm.flags[1]));
   if (threadIdx.x == 0) {
     for (int s = 0; s < r.stages; ++s) {
@@ -308,6 +307,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
     ga_raw = ldg128(gamma + tx * VE);
     be_raw = ldg128(beta + tx * VE);
   }
+  if (st.parked) tmem_store_wait();  // also where the barrier gives up and pass 2 is left out: stream_end frees the words
   grid_barrier(count, sm.flags, r);
 
   // ---- statistics of the sample: sums about the first CTA's mean, the counts known from the geometry
@@ -366,10 +366,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   int lost = ok ? -1 : T_ - 1;  // the rows of the tiles up to this one are not known
   for (int i = 0; ok; ++i) {
     if (i == S && st.parked) {  // the stages fill again meanwhile
-      tmem_store_wait();
       for (int p = st.parked - 1; p >= 0; --p) {
         uint4 w[KR];
-        __syncwarp();
         tmem_load16(st.tmem + p * 16, w[0], w[1], w[2], w[3]);
         emit(st.held0 + p, w);
         if (tid == 0) st.refill_behind(S - 1, r);
@@ -511,6 +509,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   crew_group_sums(cr, g, gam, chan,
                   [&](int s, float w1, float w2) { gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2); });
   for (int c = tid; c < g.C; c += blockDim.x) tpart[(size_t)blockIdx.x * g.C + c] = make_float2(chan[c], chan[g.C + c]);
+  if (st.parked) tmem_store_wait();  // also where the barrier gives up and pass 2 is left out: stream_end frees the words
   grid_barrier(count, sm.flags, r);
 
   // ---- A, B of the sample's groups
@@ -578,10 +577,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   int lost = ok ? -1 : T_ - 1;
   for (int i = 0; ok; ++i) {
     if (i == S && st.parked) {
-      tmem_store_wait();
       for (int p = st.parked - 1; p >= 0; --p) {
         uint4 xw[KR], dw[KR];
-        __syncwarp();
         tmem_load16(st.tmem + p * 16, xw[0], xw[1], dw[0], dw[1]);
         emit(st.held0 + p, xw, dw);
         if (tid == 0) st.refill_behind(S - 1, r);

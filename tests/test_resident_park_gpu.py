@@ -66,3 +66,45 @@ def test_reductions_over_the_cta(N, C, sp, G, dt, ctas, monkeypatch):
     assert O.rel_err(out["mean"], want["mean"]) < 1e-5
     assert O.rel_err(out["rstd"] / want["rstd"].cuda().float(), torch.ones_like(want["rstd"])) < 1e-5
     assert O.rel_err(out["dparam"][0], want["dgamma"]) <= O.TOLERANCE[DT[dt]] and O.rel_err(out["dparam"][1], want["dbeta"]) <= O.TOLERANCE[DT[dt]]
+
+
+@pytest.mark.parametrize("what", [3, 4, 5], ids=["no arrival", "no first copy", "no copy of the second pass"])
+@pytest.mark.parametrize("dt,act", [("float16", "silu"), ("float32", "relu")])
+def test_waits_that_run_out_with_tiles_in_tensor_memory(what, dt, act, monkeypatch):
+    """One CTA withholds what others, or its own threads, wait for (decided on the host, wait limit one millisecond) while tiles are
+    in tensor memory.  The call returns, what depends on it is NaN, the parked rows of a lost second pass are not, and the
+    tensor memory is given back: the next calls get it and have the bits of the first."""
+    from channels_last_groupnorm_b200 import _native as nt
+
+    from .test_parity_gpu import _flat
+
+    N, C, sp, G, code, ctas, cta, park = 2, 64, (32, 240), 8, O.ACT_CODES[act], 3, 1, 3
+    for name, value in (("FORCE_PATH", "resident"), ("RESIDENT_CTAS", ctas), ("RESIDENT_STAGES", 2), ("RESIDENT_PARK", park)):
+        monkeypatch.setenv("GNB200_" + name, str(value))
+    x, ga, be, dy = O.make_inputs(N, C, sp, DT[dt], seed=61)
+    xd, dyd, gd, bd = _flat(x.cuda()), _flat(dy.cuda()), ga.cuda(), be.cuda()
+    good = nt.fwd_raw(xd, gd, bd, G, 1e-5, code)
+    calls = (lambda: nt.fwd_raw(xd, gd, bd, G, 1e-5, code), lambda: nt.bwd_raw(dyd, xd, gd, bd, good[1], good[2], G, code))
+    for direction in (0, 1):
+        want = calls[direction]()
+        nt.check(nt.lib.gnb200_debug_next_resident(what, cta))
+        try:
+            got = calls[direction]()
+            torch.cuda.synchronize()  # the call returns and the GPU still answers
+            assert nt.wait_timeouts() > 0
+        finally:
+            nt.clear_wait_timeouts()
+        if what != 5:
+            assert all(torch.isnan(t.float()).all() for t in got)
+        else:  # two tiles were in the stages and `park` in tensor memory: those before them are missing
+            plan = dict(kv.split("=") for kv in nt.describe_plan(N, sp[0] * sp[1], C, G, DT[dt], direction).split()[2:])
+            rows, tile = int(plan["rows"]), int(plan["tile"].split("x")[1])
+            tiles = -(-rows // tile)
+            assert tiles > 2 + park
+            missing = torch.zeros(sp[0] * sp[1], dtype=torch.bool, device="cuda")
+            missing[cta * rows:cta * rows + (tiles - 2 - park) * tile] = True
+            assert torch.isnan(got[0][0, missing].float()).all()
+            assert torch.equal(got[0][0, ~missing], want[0][0, ~missing]) and torch.equal(got[0][1], want[0][1])
+        for _ in range(3):
+            assert all(torch.equal(a, b) for a, b in zip(calls[direction](), want))
+    assert nt.wait_timeouts() == 0
