@@ -20,23 +20,23 @@ DTYPE_CODES = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 
 def _load():
     try:
-        core_path, torch_path = _build.build_all()
+        core_path, torch_path, python_path = _build.build_all()
     except Exception as exc:  # pragma: no cover - depends on the toolchain of the machine
-        if not (os.path.exists(_build.CORE_LIB) and os.path.exists(_build.TORCH_LIB)):
+        core_path, torch_path, python_path = _build.CORE_LIB, _build.TORCH_LIB, _build.PYTHON_LIB
+        if not all(os.path.exists(p) for p in (core_path, torch_path, python_path)):
             raise ImportError(
                 "channels_last_groupnorm_b200: the native libraries are missing and could not be built "
                 "(run `python -m channels_last_groupnorm_b200.build`): %s" % exc) from exc
-        core_path, torch_path = _build.CORE_LIB, _build.TORCH_LIB
     core = ctypes.CDLL(core_path, mode=ctypes.RTLD_GLOBAL)
     torch.ops.load_library(torch_path)
-    # the same library is a Python module too (gn_torch.cpp: plain_call)
-    loader = importlib.machinery.ExtensionFileLoader("gnb200_torch", torch_path)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("gnb200_torch", torch_path, loader=loader))
+    # plain_call (gn_python.cpp)
+    loader = importlib.machinery.ExtensionFileLoader("gnb200_python", python_path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("gnb200_python", python_path, loader=loader))
     loader.exec_module(module)
     return core, module
 
 
-lib, torch_module = _load()
+lib, python_module = _load()
 
 lib.gnb200_version.restype = ctypes.c_int
 lib.gnb200_last_error.restype = ctypes.c_char_p

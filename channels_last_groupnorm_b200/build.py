@@ -1,8 +1,9 @@
-"""Ahead-of-time build of the two native libraries, in-tree under `lib/`.
+"""Ahead-of-time build of the native libraries, in-tree under `lib/`.
 
   lib/libgnb200.so      hand-written sm_100a CUDA kernels + planner + C ABI (include/gnb200.h);
                         depends only on the CUDA runtime (linked statically), not on torch
-  lib/gnb200_torch.so   C++ torch binding (torch.ops.gnb200.*) over that C ABI
+  lib/gnb200_torch.so   C++ torch binding (torch.ops.gnb200.*) over that C ABI; needs libtorch, not Python
+  lib/gnb200_python.so  the module's call without argument matching, a Python extension over gnb200_torch.so
 
 The reference JIT-compiles its extension on first import (src/gnnhwc/custom_gn.py:7-27); here the
 libraries are built once (`python -m channels_last_groupnorm_b200.build`) and loaded from disk.
@@ -20,6 +21,7 @@ LIB_DIR = os.path.join(PKG_DIR, "lib")
 INCLUDE_DIR = os.path.join(os.path.dirname(PKG_DIR), "include")
 CORE_LIB = os.path.join(LIB_DIR, "libgnb200.so")
 TORCH_LIB = os.path.join(LIB_DIR, "gnb200_torch.so")
+PYTHON_LIB = os.path.join(LIB_DIR, "gnb200_python.so")
 
 CUDA_SOURCES = ["gn_fwd.cu", "gn_bwd.cu", "gn_wave.cu", "gn_resident.cu", "gn_nchw.cu", "gn_f64.cu", "gn_plan.cu", "gn_capi.cu", "gn_static_scratch.cu"]
 CUDA_HEADERS = ["gn_common.cuh", "gn_math.cuh", "gn_async.cuh", "gn_reduce.cuh", "gn_peer.cuh", "gn_kernels.h", os.path.join(INCLUDE_DIR, "gnb200.h")]
@@ -65,7 +67,11 @@ def _core_digest():
 
 
 def _torch_digest():
-    return _digest(["gn_torch.cpp", os.path.join(INCLUDE_DIR, "gnb200.h")])
+    return _digest(["gn_torch.cpp", "gn_torch.h", os.path.join(INCLUDE_DIR, "gnb200.h")])
+
+
+def _python_digest():
+    return _digest(["gn_python.cpp", "gn_torch.h"])
 
 
 def core_is_stale():
@@ -74,6 +80,10 @@ def core_is_stale():
 
 def torch_is_stale():
     return not _stamp_matches(TORCH_LIB, _torch_digest())
+
+
+def python_is_stale():
+    return not _stamp_matches(PYTHON_LIB, _python_digest())
 
 
 def build_core(verbose=False, extra_flags=()):
@@ -103,7 +113,7 @@ def build_core(verbose=False, extra_flags=()):
     return CORE_LIB
 
 
-def build_torch(verbose=False):
+def _build_binding(source, lib_path, libs, verbose):
     from torch.utils import cpp_extension as ce
 
     os.makedirs(LIB_DIR, exist_ok=True)
@@ -112,24 +122,35 @@ def build_torch(verbose=False):
     for p in ce.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda_home, "include")]:
         inc += ["-isystem", p]
     torch_lib = ce.library_paths()[0]
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(CSRC, "gn_torch.cpp"), "-o", TORCH_LIB,
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(CSRC, source), "-o", lib_path,
            "-DTORCH_API_INCLUDE_EXTENSION_H"] + inc + [
-        "-L", torch_lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
-        "-L", LIB_DIR, "-lgnb200", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + torch_lib]
+        "-L", torch_lib, "-L", LIB_DIR] + libs + ["-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + torch_lib]
     if verbose:
         print("+", " ".join(cmd), flush=True)
     subprocess.check_call(cmd)
+
+
+def build_torch(verbose=False):
+    _build_binding("gn_torch.cpp", TORCH_LIB, ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-lgnb200"], verbose)
     _write_stamp(TORCH_LIB, _torch_digest())
     return TORCH_LIB
 
 
+def build_python(verbose=False):
+    _build_binding("gn_python.cpp", PYTHON_LIB, ["-lc10", "-ltorch_cpu", "-ltorch_python", "-l:gnb200_torch.so"], verbose)
+    _write_stamp(PYTHON_LIB, _python_digest())
+    return PYTHON_LIB
+
+
 def build_all(force=False, verbose=False):
-    """Builds whatever is missing or older than its sources. Returns the two library paths."""
+    """Builds whatever is missing or older than its sources. Returns the library paths."""
     if force or core_is_stale():
         build_core(verbose)
     if force or torch_is_stale():
         build_torch(verbose)
-    return CORE_LIB, TORCH_LIB
+    if force or python_is_stale():
+        build_python(verbose)
+    return CORE_LIB, TORCH_LIB, PYTHON_LIB
 
 
 if __name__ == "__main__":

@@ -14,9 +14,6 @@
 // [2, C] tensor in the statistics' dtype (the buffer a data-parallel caller all-reduces), and the ops
 // carry explicit schemas with a CUDA implementation (the reference registers catch-all functions, which
 // cannot be traced).
-#include <Python.h>
-
-#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/Tensor.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/core/dispatch/Dispatcher.h>
@@ -26,14 +23,13 @@
 #include <ATen/record_function.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
-#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
-#include <torch/csrc/autograd/python_variable.h>
 #include <torch/library.h>
 
 #include <vector>
 
 #include "../../include/gnb200.h"
+#include "gn_torch.h"
 
 namespace {
 
@@ -492,9 +488,19 @@ at::Tensor group_norm_act_autograd(const at::Tensor& X, const at::Tensor& weight
   return GnFunction::apply(X, weight, bias, G, eps, act);
 }
 
-// The module's call, if it is a plain one; an undefined tensor otherwise.
-at::Tensor group_norm_act_direct(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
-                                 int64_t act) {
+// below autograd (inference mode)
+at::Tensor group_norm_act_plain(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
+                                int64_t act) {
+  const bool cl = is_channels_last(X);
+  const at::Tensor Y = std::get<0>(call_fwd(flatten(X, cl), as_dtype(weight, X.scalar_type()), as_dtype(bias, X.scalar_type()), G,
+                                            eps, act));
+  return restore(Y, X.sizes(), cl);
+}
+
+}  // namespace
+
+at::Tensor gnb200_ops::group_norm_act_direct(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G,
+                                             double eps, int64_t act) {
   Dense d;
   if (!only_cuda_sees({&X, &weight, &bias}) || !plain_tensor(X, &d)) return at::Tensor();
   for (const at::Tensor* t : {&X, &weight, &bias})
@@ -506,17 +512,6 @@ at::Tensor group_norm_act_direct(const at::Tensor& X, const at::Tensor& weight, 
   params_like(X, d, w, b);
   return direct_fwd(X, d, w, b, G, eps, act, nullptr, nullptr);
 }
-
-// below autograd (inference mode)
-at::Tensor group_norm_act_plain(const at::Tensor& X, const at::Tensor& weight, const at::Tensor& bias, int64_t G, double eps,
-                                int64_t act) {
-  const bool cl = is_channels_last(X);
-  const at::Tensor Y = std::get<0>(call_fwd(flatten(X, cl), as_dtype(weight, X.scalar_type()), as_dtype(bias, X.scalar_type()), G,
-                                            eps, act));
-  return restore(Y, X.sizes(), cl);
-}
-
-}  // namespace
 
 // Schemas are declared apart from the implementations so that Python can attach fake-tensor
 // kernels and an autograd formula to them (channels_last_groupnorm_b200/_compile.py), which is what
@@ -548,43 +543,3 @@ TORCH_LIBRARY_IMPL(gnb200, CPU, m) {
   m.impl("bwd", &gnb200_bwd_op);
   m.impl("bwd_f32", &gnb200_bwd_f32_op);
 }
-
-// ------------------------------------------------------------------------------------------------
-// plain_call(x, weight, bias, num_groups, eps, act, num_channels) -> tensor, or None where the module's Python code has
-// to look at the call: anything but exact tensors and parameters, a torch-function mode, other argument types, a shape that it
-// refuses.  Called without torch.ops' argument matching, which took 3 us.
-// ------------------------------------------------------------------------------------------------
-namespace {
-
-const at::Tensor* exact_tensor(PyObject* o) {
-  if (Py_TYPE(o) != (PyTypeObject*)THPVariableClass && Py_TYPE(o) != (PyTypeObject*)ParameterClass) return nullptr;
-  return &THPVariable_Unpack(o);
-}
-
-PyObject* plain_call(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-  HANDLE_TH_ERRORS
-  if (nargs != 7 || !PyLong_CheckExact(args[3]) || !PyFloat_CheckExact(args[4]) || !PyLong_CheckExact(args[5]) ||
-      !PyLong_CheckExact(args[6]) || at::impl::torch_function_mode_enabled())
-    Py_RETURN_NONE;
-  const at::Tensor *x = exact_tensor(args[0]), *w = exact_tensor(args[1]), *b = exact_tensor(args[2]);
-  if (!x || !w || !b) Py_RETURN_NONE;
-  const long long G = PyLong_AsLongLong(args[3]), act = PyLong_AsLongLong(args[5]), C = PyLong_AsLongLong(args[6]);
-  if (PyErr_Occurred()) return nullptr;
-  if (!x->is_cuda() || x->dim() < 3 || x->size(1) != C) Py_RETURN_NONE;
-  const double eps = PyFloat_AS_DOUBLE(args[4]);
-  at::Tensor y;
-  {
-    pybind11::gil_scoped_release no_gil;
-    y = group_norm_act_direct(*x, *w, *b, G, eps, act);
-  }
-  if (!y.defined()) Py_RETURN_NONE;
-  return THPVariable_Wrap(std::move(y));
-  END_HANDLE_TH_ERRORS
-}
-
-PyMethodDef kMethods[] = {{"plain_call", (PyCFunction)(void (*)())plain_call, METH_FASTCALL, nullptr}, {nullptr, nullptr, 0, nullptr}};
-PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "gnb200_torch", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
-
-}  // namespace
-
-PyMODINIT_FUNC PyInit_gnb200_torch(void) { return PyModule_Create(&kModule); }

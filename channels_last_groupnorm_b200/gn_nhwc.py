@@ -133,7 +133,7 @@ def _restore_shape(flat: torch.Tensor, shape, channels_last=True) -> torch.Tenso
 
 
 _group_norm_act = torch.ops.gnb200.group_norm_act.default
-_plain_call = _native.torch_module.plain_call
+_plain_call = _native.python_module.plain_call
 _PLAIN = (torch.Tensor, nn.Parameter)
 
 

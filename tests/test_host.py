@@ -2,6 +2,7 @@
 import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 import torch
@@ -30,6 +31,21 @@ def test_core_library_does_not_link_torch():
     with open(gnbuild.CORE_LIB, "rb") as f:
         blob = f.read()
     assert b"libtorch" not in blob and b"libc10" not in blob
+
+
+def test_torch_library_loads_without_python(tmp_path):
+    # the ops are for libtorch programs too: in a process without Python every symbol of the library must resolve
+    source = tmp_path / "load.c"
+    source.write_text("""#include <dlfcn.h>
+#include <stdio.h>
+int main(int argc, char** argv) {
+  if (!dlopen(argv[1], RTLD_NOW | RTLD_GLOBAL)) return puts(dlerror()), 1;
+  if (dlsym(RTLD_DEFAULT, "Py_IsInitialized")) return puts("Python came along"), 2;
+  return 0;
+}""")
+    subprocess.check_call(["gcc", str(source), "-o", str(tmp_path / "load"), "-ldl"])
+    run = subprocess.run([str(tmp_path / "load"), gnbuild.TORCH_LIB], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stdout
 
 
 def test_activation_codes_match_reference_table():

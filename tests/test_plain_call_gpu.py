@@ -1,4 +1,4 @@
-"""The module's plain call (gn_torch.cpp: plain_call, without views or inner ops) against the general path through the
+"""The module's plain call (gn_python.cpp: plain_call, without views or inner ops) against the general path through the
 ops, which a dispatch mode forces: values, sizes, strides, gradients, and what may surround a call."""
 import pytest
 import torch
