@@ -318,9 +318,17 @@ bool plain_tensor(const at::Tensor& t, Dense* out) {
   *out = Dense{cl, cl || r == 1 ? kNHWC : kNCHW, n, c, r};
   return true;
 }
-// uninitialised, with the sizes of `like` and the strides that restore() gives
-at::Tensor empty_result(const at::Tensor& like, const Dense& d) {
-  const auto sizes = like.sizes();
+// What flatten() gives for a plain tensor: the same storage and version counter, no graph, none of its own dispatches.
+at::Tensor flat_alias(const at::Tensor& t, const Dense& d) {
+  auto* impl = t.unsafeGetTensorImpl();
+  auto flat = impl->shallow_copy_and_detach(impl->version_counter(), /*allow_tensor_metadata_change=*/true);
+  const int64_t sizes[] = {d.N, d.C, d.R};
+  const int64_t strides[] = {d.R * d.C, d.channels_last ? 1 : d.R, d.channels_last ? d.C : 1};
+  flat->set_sizes_and_strides(sizes, strides);
+  return at::Tensor(std::move(flat));
+}
+// uninitialised, with the strides that restore() gives
+at::Tensor empty_result(const at::Tensor& like, at::IntArrayRef sizes, const Dense& d) {
   at::DimVector strides(sizes.size());
   int64_t step = d.channels_last ? d.C : 1;
   for (int64_t i = (int64_t)sizes.size() - 1; i >= 2; --i) strides[i] = step, step *= sizes[i];
@@ -360,7 +368,7 @@ at::Tensor direct_fwd(const at::Tensor& X, const Dense& d, const at::Tensor& wei
   TORCH_CHECK(G >= 1 && d.C % G == 0, "gnb200: num_channels ", d.C, " is not divisible by num_groups ", G);
   TORCH_CHECK(act >= 0 && act <= 4, "gnb200: activation code ", act, " is not in 0..4");
   c10::cuda::CUDAGuard guard(X.device());
-  at::Tensor Y = empty_result(X, d);
+  at::Tensor Y = empty_result(X, X.sizes(), d);
   const size_t ws_bytes = d.layout == kNHWC ? gnb200_fwd_workspace_bytes(d.N, d.R, d.C, G, dtype)
                                             : gnb200_fwd_nchw_workspace_bytes(d.N, d.R, d.C, G, dtype);
   const size_t ws_end = (ws_bytes + 15) & ~(size_t)15, stat_bytes = (size_t)d.N * G * sizeof(float);
@@ -384,7 +392,7 @@ at::Tensor direct_fwd(const at::Tensor& X, const Dense& d, const at::Tensor& wei
   return Y;
 }
 
-// typed: dgamma, dbeta in X's dtype; otherwise the two rows of one fp32 tensor
+// X: flat.  typed: dgamma, dbeta in X's dtype; otherwise the two rows of one fp32 tensor
 void direct_bwd(const at::Tensor& dy, const at::Tensor& X, const Dense& d, const at::Tensor& weight, const at::Tensor& bias,
                 const at::Tensor& means, const at::Tensor& rstds, int64_t G, int64_t act, bool typed, at::Tensor* dx,
                 at::Tensor* dgamma, at::Tensor* dbeta) {
@@ -394,7 +402,7 @@ void direct_bwd(const at::Tensor& dy, const at::Tensor& X, const Dense& d, const
   check_stats(means, X, dtype, d.N, G, "means");
   check_stats(rstds, X, dtype, d.N, G, "rstds");
   c10::cuda::CUDAGuard guard(X.device());
-  *dx = empty_result(X, d);
+  *dx = empty_result(X, dy.sizes(), d);
   const size_t ws_bytes = d.layout == kNHWC ? gnb200_bwd_workspace_bytes(d.N, d.R, d.C, G, dtype)
                                             : gnb200_bwd_nchw_workspace_bytes(d.N, d.R, d.C, G, dtype);
   const size_t ws_end = (ws_bytes + 15) & ~(size_t)15;
@@ -428,13 +436,18 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
                             int64_t G, double eps, int64_t act) {
     const bool cl = is_channels_last(X);
     at::Tensor w = weight, b = bias;
-    ctx->saved_data["arg"] = std::vector<int64_t>{G, act, cl ? 1 : 0, (int64_t)weight.scalar_type(), (int64_t)bias.scalar_type()};
     Dense d;
-    if (only_cuda_sees({&X, &w, &b}) && plain_tensor(X, &d)) {  // X itself is saved, in the order that flatten() would give
+    const bool plain = only_cuda_sees({&X, &w, &b}) && plain_tensor(X, &d);
+    ctx->saved_data["arg"] =
+        std::vector<int64_t>{G, act, cl ? 1 : 0, (int64_t)weight.scalar_type(), (int64_t)bias.scalar_type(), plain ? 1 : 0};
+    ctx->saved_data["shape"] = X.sizes().vec();
+    // The flat tensor is saved on either path, not X: hooks and the checks of a checkpoint's recomputation, which may take the
+    // other path (a profiler started since), meet the same sizes, and X may be given other data.
+    if (plain) {
       params_like(X, d, w, b);
       at::Tensor means, rstds;
       at::Tensor Y = direct_fwd(X, d, w, b, G, eps, act, &means, &rstds);
-      ctx->save_for_backward({X, w, b, means, rstds});
+      ctx->save_for_backward({flat_alias(X, d), w, b, means, rstds});
       return Y;
     }
     w = as_dtype(weight, X.scalar_type());
@@ -442,7 +455,6 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
     const at::Tensor Xf = flatten(X, cl);
     auto [Y, means, rstds] = call_fwd(Xf, w, b, G, eps, act);
     ctx->save_for_backward({Xf, w, b, means, rstds});
-    ctx->saved_data["shape"] = X.sizes().vec();
     return restore(Y, X.sizes(), cl);
   }
 
@@ -451,26 +463,26 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
     static const auto op32 =
         c10::Dispatcher::singleton().findSchemaOrThrow("gnb200::bwd_f32", "").typed<decltype(gnb200_bwd_f32_op)>();
     const auto saved = ctx->get_saved_variables();
-    const auto arg = ctx->saved_data["arg"].toIntVector();
+    const auto shape = ctx->saved_data["shape"].toIntVector(), arg = ctx->saved_data["arg"].toIntVector();
+    const bool cl = arg[2] != 0;
     const at::ScalarType dtype = saved[0].scalar_type();
     const auto w_dtype = (at::ScalarType)arg[3], b_dtype = (at::ScalarType)arg[4];
     at::Tensor dx, dgamma, dbeta;
-    const auto flat_shape = ctx->saved_data.find("shape");
-    const bool unflattened = flat_shape == ctx->saved_data.end();
     const at::Tensor& g = grads[0];
     Dense d;
-    if (unflattened && !c10::GradMode::is_enabled() && g.defined() &&
+    if (arg[5] != 0 && !c10::GradMode::is_enabled() && g.defined() &&
         only_cuda_sees({&g, &saved[0], &saved[1], &saved[2], &saved[3], &saved[4]}) && plain_tensor(saved[0], &d) &&
-        d.channels_last == (arg[2] != 0) && g.scalar_type() == dtype && g.device() == saved[0].device() &&
-        g.sizes() == saved[0].sizes() && dense_order(g, d.channels_last)) {
+        dense_order(saved[0], cl) && g.scalar_type() == dtype && g.device() == saved[0].device() &&
+        g.sizes() == at::IntArrayRef(shape) && dense_order(g, cl)) {
+      d.channels_last = cl;  // (of the flat tensor's strides, one row or channel leaves it open)
+      d.layout = cl || d.R == 1 ? kNHWC : kNCHW;
       const bool typed = w_dtype == dtype && b_dtype == dtype;
       direct_bwd(g, saved[0], d, saved[1], saved[2], saved[3], saved[4], arg[0], arg[1], typed, &dx, &dgamma, &dbeta);
       return {dx, as_dtype(dgamma, w_dtype), as_dtype(dbeta, b_dtype), at::Tensor(), at::Tensor(), at::Tensor()};
     }
-    // (under create_graph the saved input must not bring a graph of its own along, as its flattened view does not)
-    const at::Tensor Xf = unflattened ? flatten(c10::GradMode::is_enabled() ? saved[0].detach() : saved[0], arg[2] != 0) : saved[0];
-    const auto shape = unflattened ? saved[0].sizes().vec() : flat_shape->second.toIntVector();
-    const at::Tensor dy = as_dtype(flatten(g, arg[2] != 0), dtype);
+    // (flat already; a hook may have brought it back in another storage order)
+    const at::Tensor Xf = flatten(saved[0], cl);
+    const at::Tensor dy = as_dtype(flatten(g, cl), dtype);
     if (w_dtype == dtype && b_dtype == dtype) {
       std::tie(dx, dgamma, dbeta) = op.call(dy, Xf, saved[1], saved[2], saved[3], saved[4], arg[0], arg[1]);
     } else {
@@ -479,7 +491,7 @@ struct GnFunction : torch::autograd::Function<GnFunction> {
       dgamma = dparam.select(0, 0).to(w_dtype);
       dbeta = dparam.select(0, 1).to(b_dtype);
     }
-    return {restore(dx, shape, arg[2] != 0), dgamma, dbeta, at::Tensor(), at::Tensor(), at::Tensor()};
+    return {restore(dx, shape, cl), dgamma, dbeta, at::Tensor(), at::Tensor(), at::Tensor()};
   }
 };
 
