@@ -656,7 +656,8 @@ static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
   if (!twopass_only && !wave_only && !resident_only && !streaming_only && plan_fused(sh, plan)) {
     if (fused_only || (force && !strcmp(force, "fused")) || !fused_loses(sh, *plan)) return true;
     Plan other;
-    if (!plan_streaming(sh, false, false, &other)) return true;
+    // (the multi-kernel forward of a thousand narrow groups wants more shared memory than there is: 1 x 18000 x 1024, one channel each)
+    if (!plan_streaming(sh, false, false, &other) || other.smem_bytes > kSmemMaxOptin) return true;
     *plan = other;
     plan_resident(sh, false, plan);
     plan->over_fused = true;
