@@ -289,7 +289,8 @@ bool plan_fused(const Shape& sh, Plan* out) {
 // Measured on B200, device us, fused / multi-pass, forward and backward:
 //   fp16  256@256^2 (16-byte segments) 55.5 / 22.7, 91.7 / 34.9    128@256^2 57.7 / 17.6, 60.5 / 26.8    512@192^2 (32 bytes) 35.6 /
 //   24.3, 63.4 / 39.0    256 x 32768 rows 22.1 / 16.3, 36.3 / 26.6    512 x 28700 rows (64 bytes) 25.0 / 22.2, 49.7 / 33.1
-//   bf16  2 x 256@200^2 38.5 / 26.0, 66.7 / 43.0    fp32  2 x 48 x 25164 rows, 9.7 MB 15.7 / 12.4, 23.5 / 23.0
+//   beyond L2 as well  8 x 512 x 28700 rows 130 / 126, 281 / 195    16 of them, 470 MB 257 / 253, 541 / 379    8 x 256@256^2 333 / 146, 526 / 221
+//   bf16  2 x 256@200^2 38.5 / 26.0, 66.7 / 43.0    fp32  2 x 48 x 25164 rows, 9.7 MB 17.4 / 13.1, 23.7 / 24.8
 // The other sides: two CTAs per SM  3 x 256 x 11696 rows 11.5 / 16.9, 18.7 / 24.7; wide segments  4 x 2560@88^2 (160 bytes) 101 /
 // 102, 147 / 185; whole rows  12 x 12 x 25745 rows fp32 11.5 / 14.6; and below 2 MB, where the launches decide: bf16
 // 24 x 40000 rows, 1.9 MB 12.5 / 9.3, 16.0 / 16.4 (16 x 65536 rows fp16, 2.1 MB 20.2 / 9.9, 23.9 / 16.4).
@@ -298,6 +299,34 @@ bool fused_loses(const Shape& sh, const Plan& p) {
   return sh.ve > 1 && cw < sh.C && cw * sh.s <= 64 && p.smem_bytes > (kSmemMaxOptin - 1024) / 2 &&
          (double)sh.N * sh.R * sh.C * sh.s >= 2e6 && env_int("GNB200_CW", 0) == 0 && env_int("GNB200_K", 0) == 0 &&
          env_int("GNB200_THREADS", 0) == 0;
+}
+
+// ... and where the fused plan wins all the same against `other`, the multi-pass plan that there is.  16-byte segments never do (0.4 - 0.9 of
+// its time over 100 shapes).  The lines were drawn through 560 shapes of 2 to 420 MB; fused / multi-pass, device us:
+//   backward, wave plan: where the units of a wave do not fit its team in one round, half of the team waits for the rest - bf16 77 x 64 x
+//     12838 rows 146 / 202, fp16 58 x 128 x 18448 249 / 341; groups of fewer than four channels, whose sums it takes one by one -
+//     fp16 10 x 256 x 39733, one channel each 241 / 450; and 64-byte segments in 512-thread CTAs, where the fused kernel reaches 3 TB/s -
+//     fp32 2 x 512 x 12164 46 / 72, 13 x 256 x 18857 245 / 344.  Not where that kernel runs 128 threads an SM: 4 x 512 x 26755 389 / 216.
+//   forward, more than 128 groups, or more than 64 of one or two channels in 64-byte segments: the finalize kernel's - bf16 2048 x 16441
+//     rows, 256 groups 47 / 79, 31 x 128 x 12681, 128 groups 60 / 80 (fp32 5 x 256 x 39536, 128 groups, 32 bytes 161 / 145).
+//   all clusters resident at once (14 of eight CTAs): fewer launches or no wave to wait for, while the tile is short and the grid no mere corner
+//     of the chip - bf16 3 x 128 x 17880 10.6 / 14.0, 17.4 / 21.9, fp16 3 x 48 x 29154 9.9 / 12.4, 15.0 / 18.7, fp32 3 x 64 x 13570 backward
+//     17.5 / 32.7, against 57399 rows of 32 bytes 17.7 / 13.4 and 64 x 33402 rows, 32 CTAs 15.7 / 12.6, 20.1 / 16.5; in fp32 not the forward (96 x
+//     23599 rows 17.5 / 14.1); in the backward no segments of 48 bytes (bf16 192 x 25221 24.6 / 20.7); 16-bit forward with one or two channels a group
+//     whatever the tile - 3 x 64 x 46389 17.3 / 25.2.
+bool fused_holds(const Shape& sh, const Plan& p, const Plan& other) {
+  const int seg = p.geom.CW * sh.s;
+  if (seg <= 16) return false;
+  const bool one_round = p.grid >= 48 && p.grid <= 112, short_tile = (long long)p.geom.rows_per_cta * seg <= 150000;
+  if (other.wave && !other.resident) {
+    const WaveGeom& w = other.wgeom;
+    if (p.threads <= 128) return false;
+    if (one_round && short_tile) return true;
+    return sh.D < 4 || (seg == 64 && p.threads == 512) || (long long)w.ipw * w.chunks > other.grid / w.teams;
+  }
+  if (sh.direction == 0 && (sh.G > 128 || (sh.G > 64 && sh.D <= 2 && seg == 64))) return true;
+  if (sh.s != 2 || !one_round) return false;
+  return sh.direction == 0 ? short_tile || sh.D <= 2 : short_tile && seg % 32 == 0;
 }
 
 bool plan_two_pass(const Shape& sh, Plan* out) {
@@ -658,8 +687,9 @@ static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
     Plan other;
     // (the multi-kernel forward of a thousand narrow groups wants more shared memory than there is: 1 x 18000 x 1024, one channel each)
     if (!plan_streaming(sh, false, false, &other) || other.smem_bytes > kSmemMaxOptin) return true;
+    plan_resident(sh, false, &other);
+    if (fused_holds(sh, *plan, other)) return true;
     *plan = other;
-    plan_resident(sh, false, plan);
     plan->over_fused = true;
     return true;
   }
