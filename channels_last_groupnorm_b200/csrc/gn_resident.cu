@@ -70,7 +70,8 @@ constexpr size_t kControlBytes = 2 * kMaxStages * 8 + 16;
 
 // The stage sequence of both passes, as thread 0 (which issues the copies) and all threads walk it.  Tile t
 // lives in stage t % stages in both passes; the parity of a barrier's current phase is one bit per stage.
-template <typename T, int NT>
+// HOLD: tiles are parked in tensor memory and copies carry the evict-first hint, as the geometry says; otherwise neither.
+template <typename T, int NT, bool HOLD>
 struct Stream {
   const T* src[NT];  // x (and dy): first element of the CTA's row range
   int tiles, nrows, BR, stages;
@@ -86,7 +87,7 @@ struct Stream {
     mbar_arrive_expect_tx(&sm.full[stage], NT * bytes);
     const uint32_t dst = sm.stage0 + (uint32_t)(stage * NT) * tile_bytes;
     const size_t at = (size_t)t * tile_bytes;
-    if (once) {
+    if (HOLD && once) {
 #pragma unroll
       for (int i = 0; i < NT; ++i)
         bulk_load_once(dst + i * tile_bytes, reinterpret_cast<const char*>(src[i]) + at, bytes, &sm.full[stage], policy);
@@ -138,8 +139,8 @@ struct Stream {
   }
 };
 
-template <typename T, int NT>
-__device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGeom& r, const Smem& sm, int nrows) {
+template <typename T, int NT, bool HOLD>
+__device__ __forceinline__ void stream_start(Stream<T, NT, HOLD>& st, const ResidentGeom& r, const Smem& sm, int nrows) {
   st.sm = sm;
   st.nrows = nrows;
   st.BR = r.BR;
@@ -149,11 +150,11 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
   st.tile_bytes = (uint32_t)r.tile_bytes;
   st.full_ph = st.empty_ph = 0;
   st.last_ph = ~0u;
-  st.policy = evict_first_policy();
-  st.parked = max(0, min(r.park, st.tiles - r.stages));
+  if constexpr (HOLD) st.policy = evict_first_policy();
+  st.parked = HOLD ? max(0, min(r.park, st.tiles - r.stages)) : 0;
   st.held0 = max(0, st.tiles - r.stages - st.parked);
   const int alloc_warp = 1 % (int)(blockDim.x >> 5);  // not the one that issues the copies, where there is another
-  if (st.parked && (int)(threadIdx.x >> 5) == alloc_warp) tmem_alloc(reinterpret_cast<uint32_t*>(&sm.flags[1]));
+  if (HOLD && st.parked && (int)(threadIdx.x >> 5) == alloc_warp) tmem_alloc(reinterpret_cast<uint32_t*>(&sm.flags[1]));
   if (threadIdx.x == 0) {
     for (int s = 0; s < r.stages; ++s) {
       mbar_init(&sm.full[s], 1);
@@ -167,10 +168,10 @@ __device__ __forceinline__ void stream_start(Stream<T, NT>& st, const ResidentGe
   __syncthreads();
   st.tmem = st.parked ? tmem_own(*(volatile uint32_t*)&sm.flags[1], threadIdx.x >> 5) : 0u;
 }
-template <typename T, int NT>
-__device__ __forceinline__ void stream_end(Stream<T, NT>& st, const WaitLimit& lim) {
+template <typename T, int NT, bool HOLD>
+__device__ __forceinline__ void stream_end(Stream<T, NT, HOLD>& st, const WaitLimit& lim) {
   if (threadIdx.x == 0) st.drain(lim);
-  if (!st.parked) return;
+  if (!HOLD || !st.parked) return;
   __syncwarp();
   __syncthreads();
   if ((int)(threadIdx.x >> 5) == 1 % (int)(blockDim.x >> 5)) tmem_free(*(volatile uint32_t*)&st.sm.flags[1]);
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   const bool streaming = ty < g.TY;
   const size_t row0 = (size_t)n * g.R + r0;
 
-  Stream<T, 1> st;
+  Stream<T, 1, true> st;
   st.src[0] = x + row0 * g.C;
   stream_start(st, r, sm, nrows);
   const int T_ = st.tiles, S = st.stages;
@@ -396,7 +397,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
 // backward.  scratch: tpart[cta * C + c] = (S1, S2) of channel c over the CTA's rows,
 //          gpart[cta * G + s] = gamma-weighted sums of group s over the CTA's rows.
 // ------------------------------------------------------------------------------------------------
-template <typename T, int ACT, bool UNI>
+template <typename T, int ACT, bool UNI, bool HOLD>
 __global__ void __launch_bounds__(kResidentThreads, 1)
     gn_bwd_resident_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                            const T* __restrict__ beta, const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   // what the caller gave is asked for before the ring's copies: behind 28 MB of them it would arrive 3 us later
   LaneParams<T, VE, UNI> lp;
   if (streaming) lp.load(gamma, beta, mean_in + (size_t)n * g.G, rstd_in + (size_t)n * g.G, tx * VE, g.div_D);
-  Stream<T, 2> st;
+  Stream<T, 2, HOLD> st;
   st.src[0] = x + row0 * g.C;
   st.src[1] = dy + row0 * g.C;
   stream_start(st, r, sm, nrows);
@@ -473,7 +474,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
         xw[u] = lds128(base + u * step);
         dw[u] = lds128(base + st.tile_bytes + u * step);
       }
-      if (t >= st.held0 && t < T_ - S) tmem_store16(st.tmem + (t - st.held0) * 16, xw[0], xw[1], dw[0], dw[1]);
+      if (HOLD && t >= st.held0 && t < T_ - S) tmem_store16(st.tmem + (t - st.held0) * 16, xw[0], xw[1], dw[0], dw[1]);
 #pragma unroll
       for (int u = 0; u < KR; ++u) {
         if (my_row + u * g.TY < here) {
@@ -509,7 +510,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   crew_group_sums(cr, g, gam, chan,
                   [&](int s, float w1, float w2) { gpart[(size_t)blockIdx.x * g.G + s] = make_float2(w1, w2); });
   for (int c = tid; c < g.C; c += blockDim.x) tpart[(size_t)blockIdx.x * g.C + c] = make_float2(chan[c], chan[g.C + c]);
-  if (st.parked) tmem_store_wait();  // also where the barrier gives up and pass 2 is left out: stream_end frees the words
+  if (HOLD && st.parked) tmem_store_wait();  // also where the barrier gives up and pass 2 is left out: stream_end frees the words
   grid_barrier(count, sm.flags, r);
 
   // ---- A, B of the sample's groups
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1)
   st.start_pass2(stage);
   int lost = ok ? -1 : T_ - 1;
   for (int i = 0; ok; ++i) {
-    if (i == S && st.parked) {
+    if (HOLD && i == S && st.parked) {
       for (int p = st.parked - 1; p >= 0; --p) {
         uint4 xw[KR], dw[KR];
         tmem_load16(st.tmem + p * 16, xw[0], xw[1], dw[0], dw[1]);
@@ -702,7 +703,13 @@ cudaError_t launch_u(const BwdCall& c, const ResidentGeom& r, cudaStream_t strea
   const Scratch s = scratch_of(r, 1);
   char* ws = static_cast<char*>(c.workspace);
   unsigned int* count = reinterpret_cast<unsigned int*>(ws + s.count);
-  return launch(gn_bwd_resident_kernel<T, ACT, UNI>, r, count, stream, (const T*)c.dy, (const T*)c.x, (const T*)c.gamma,
+  // HOLD is a kernel of its own.  Where nothing is parked, because x and dy are beyond what that is good for (gn_plan.cu), the code for it in the
+  // loops alone costs issue slots: device us with it / without, 16 bits: 320 x 164062 rows, 105 MB 3 % slower, 1536 x 43619 133.5 / 129.2,
+  // 1536 x 130208, 400 MB 4.5 % slower.  Full CTAs of 512 threads hide it, and beyond 165 MB they are the faster ones with it (not understood: 268 MB
+  // 256 x 523437 217.5 / 219.7, 400 MB 2.4 %; 105 MB 0.983, 165 MB 1.00, 200 MB 1.012 without / with).
+  const bool hold = r.park > 0 || (r.threads == kResidentThreads && (double)r.g.N * r.g.R * r.g.C * sizeof(T) > 165e6);
+  const auto kern = hold ? gn_bwd_resident_kernel<T, ACT, UNI, true> : gn_bwd_resident_kernel<T, ACT, UNI, false>;
+  return launch(kern, r, count, stream, (const T*)c.dy, (const T*)c.x, (const T*)c.gamma,
                 (const T*)c.beta, c.mean, c.rstd, (T*)c.dx, reinterpret_cast<float2*>(ws),
                 reinterpret_cast<float2*>(ws + s.pairs), count, c.dparam_f32, (T*)c.dgamma, (T*)c.dbeta, r);
 }
