@@ -293,6 +293,9 @@ __global__ void __launch_bounds__(kThreads)
 // instruction, and vectors that stay packed while in flight (four CTAs per SM); the kernels of the other passes likewise.  Device us,
 // before / now, forward and backward: 512@256^2 fp16 35.5 / 33.4, 68.1 / 65.9; 64 x 256@64^2 bf16 71.4 / 70.7, 129.4 / 125.1; 512@128^2
 // 11.7 / 11.6, 22.2 / 19.8; 320@96^2 8.7 / 8.7, 14.2 / 12.6; 32 x 64@56^2 fp32 18.6 / 18.3, 34.5 / 31.5.
+// Single elements (rows that are no multiple of a vector) are bound by latency instead: five CTAs and a remainder loop that is not unrolled; with
+// registers for four and the loop unrolled, short rows were 4 to 8 % slower - mean over types and activations, with 16 x 2048@7^2 1.00, 84 x
+// 2048 x 221 rows 1.00, now 0.92, 0.95; rows of 30159 and 65025 the same.
 // ------------------------------------------------------------------------------------------------
 // xh = x * rs + nmr and yh = xh * ga + be, lane by lane
 template <int VE>
@@ -312,7 +315,7 @@ __device__ __forceinline__ void normalise(const float (&fx)[VE], float rs, float
   }
 }
 template <typename T, int VE, int ACT>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, VE > 1 ? 4 : 5)
     gn_nchw_reduce_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                           const T* __restrict__ beta, const float* __restrict__ mean_in,
                           const float* __restrict__ rstd_in, float2* __restrict__ tp, long long pieces,
@@ -381,6 +384,7 @@ __global__ void __launch_bounds__(kThreads, 4)
       for (int u = 0; u < kUnroll; ++u) one(fx[u], fd[u]);
     }
   }
+#pragma unroll 1
   for (; v < v1; v += 32) {
     float fx[VE], fd[VE];
     load_vec<T, VE>(xs + v * VE, fx);
