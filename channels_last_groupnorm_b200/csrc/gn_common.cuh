@@ -302,10 +302,10 @@ __device__ __forceinline__ void mul2(float& d0, float& d1, float a0, float a1, f
       : "=f"(d0), "=f"(d1)
       : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
-// f = f * a + b, lane by lane
-template <int VE>
+// f = f * a + b, lane by lane (PAIRS: packed, where there are pairs)
+template <int VE, bool PAIRS = true>
 __device__ __forceinline__ void affine(float (&f)[VE], const float (&a)[VE], const float (&b)[VE]) {
-  if constexpr (VE % 2 == 0) {
+  if constexpr (PAIRS && VE % 2 == 0) {
 #pragma unroll
     for (int e = 0; e < VE; e += 2) fma2(f[e], f[e + 1], f[e], f[e + 1], a[e], a[e + 1], b[e], b[e + 1]);
   } else {
