@@ -262,10 +262,9 @@ __device__ __forceinline__ float mixed_fma(uint16_t a, uint16_t b, float c) {
 
 // Two fp32 operations in one instruction (PTX .f32x2, sm_100): each half rounds as the scalar one does, so results are
 // the same bits.  They save issue slots but want register pairs, so they are used where they measured faster: forward sums and affine
-// maps, the channels-first kernels, and the backward arithmetic of fp16 (kPairs).  Device us, scalar / pairs: forward 64 x 256@64^2
-// bf16 GELU 56.0 / 54.8, fp16 SiLU 54.6 / 50.9, 39 x 384@68^2 bf16 83.6 / 70.6; fp16 backward 64 x 256@64^2 95.4 / 92.6, 20 x 256 x 5000
-// rows 48.9 / 47.7, 10 x 512@75^2 46.4 / 45.7; but bf16 backward, whose halves are unpacked by shifts, 11 x 512@73^2 49.1 / 50.7, 24 x 256 x
-// 5000 rows 51.9 / 52.4, 39 x 384@68^2 124.3 / 125.0.
+// maps (but kPairsInApply), the channels-first kernels, and the backward arithmetic of fp16 (kPairs).  Device us, scalar / pairs: forward 64 x
+// 256@64^2 bf16 GELU 56.0 / 54.8, fp16 SiLU 54.6 / 50.9; fp16 backward 64 x 256@64^2 95.4 / 92.6; but bf16 backward, whose halves are unpacked
+// by shifts, 11 x 512@73^2 49.1 / 50.7, 39 x 384@68^2 124.3 / 125.0.
 template <typename T>
 constexpr bool kPairs = std::is_same<T, __half>::value;
 __device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, float b0, float b1, float c0, float c1) {

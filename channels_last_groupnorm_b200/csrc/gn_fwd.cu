@@ -347,8 +347,7 @@ __device__ __forceinline__ void stream_apply_back(const Pack<T, VE>* __restrict_
 // ------------------------------------------------------------------------------------------------
 // MAXT: CTA size class.  128-thread launches are compiled for six CTAs per SM (<= 80 registers).
 // SHUF: the shuffle reductions (Geom::shuf) are compiled in instead of the generic ones.  Both in one kernel, chosen at run time, cost
-// registers; device us, before / now: 64 x 256@64^2 bf16 GELU 54.8 / 53.3, fp16 SiLU 50.9 / 48.4, 24 x 256 x 5000 rows bf16 31.9 / 29.3,
-// 11 x 512@73^2 30.4 / 27.4, 6 x 1024 x 6000 rows 35.8 / 32.5, 50 x 256@50^2 30.5 / 28.1, 10 x 512@75^2 fp16 28.3 / 25.4.
+// registers; device us, one kernel / two: 64 x 256@64^2 bf16 GELU 54.8 / 53.3, 24 x 256 x 5000 rows 31.9 / 29.3, 10 x 512@75^2 fp16 28.3 / 25.4.
 template <typename T, int VE, int ACT, bool UNI, int MAXT, bool SHUF>
 __global__ void __launch_bounds__(MAXT, MAXT == 128 ? 6 : 2)
     gn_fwd_fused_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,

@@ -122,7 +122,6 @@ bool chain_enabled();
 // channels-first tensors (gn_nchw.cu)
 bool nchw_shape_supported(int64_t N, int64_t R, int64_t C, int64_t G);
 size_t nchw_workspace_bytes(int64_t N, int64_t R, int64_t C, int64_t G, int dtype, int direction);
-int nchw_launch_count(int direction);
 cudaError_t launch_forward_nchw(const FwdCall& c, int64_t N, int64_t R, int64_t C, int64_t G, cudaStream_t stream);
 cudaError_t launch_backward_nchw(const BwdCall& c, int64_t N, int64_t R, int64_t C, int64_t G, cudaStream_t stream);
 // double precision, either layout (gn_f64.cu); `sums` holds 2 * N * C doubles

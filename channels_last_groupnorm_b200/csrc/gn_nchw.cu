@@ -290,12 +290,11 @@ __global__ void __launch_bounds__(kThreads)
 // ------------------------------------------------------------------------------------------------
 // backward 1: one warp per piece of a channel row:  tp[(n * C + c) * ppr + j] = (S1, S2)
 // Bound by instruction issue (about 100 instructions per pair of 16-byte vectors) before it is bound by HBM: so two lanes per
-// instruction, and vectors that stay packed while in flight (four CTAs per SM); the kernels of the other passes likewise.  Device us,
-// before / now, forward and backward: 512@256^2 fp16 35.5 / 33.4, 68.1 / 65.9; 64 x 256@64^2 bf16 71.4 / 70.7, 129.4 / 125.1; 512@128^2
-// 11.7 / 11.6, 22.2 / 19.8; 320@96^2 8.7 / 8.7, 14.2 / 12.6; 32 x 64@56^2 fp32 18.6 / 18.3, 34.5 / 31.5.
-// Single elements (rows that are no multiple of a vector) are bound by latency instead: five CTAs and a remainder loop that is not unrolled; with
-// registers for four and the loop unrolled, short rows were 4 to 8 % slower - mean over types and activations, with 16 x 2048@7^2 1.00, 84 x
-// 2048 x 221 rows 1.00, now 0.92, 0.95; rows of 30159 and 65025 the same.
+// instruction, and vectors that stay packed while in flight (four CTAs per SM); the kernels of the other passes likewise.  What that gives,
+// device us of forward and backward, scalar and unpacked / so: 512@256^2 fp16 35.5 / 33.4, 68.1 / 65.9; 32 x 64@56^2 fp32 18.6 / 18.3, 34.5 / 31.5.
+// Single elements (rows that are no multiple of a vector) are bound by latency instead: five CTAs, and a remainder loop that is not unrolled, since
+// its registers would leave four: then backward calls with short rows take 1.09 (16 x 2048@7^2) and 1.05 (84 x 2048 x 221 rows) of the time, mean over
+// types and activations; rows of 30159 and 65025 elements the same.
 // ------------------------------------------------------------------------------------------------
 // xh = x * rs + nmr and yh = xh * ga + be, lane by lane
 template <int VE>
@@ -708,8 +707,6 @@ size_t nchw_workspace_bytes(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
   }
   return best;
 }
-
-int nchw_launch_count(int direction) { return direction == 0 ? 2 : 4; }  // (backward of one sample: 3)
 
 cudaError_t launch_forward_nchw(const FwdCall& c, int64_t N, int64_t R, int64_t C, int64_t G, cudaStream_t stream) {
   const bool al = aligned16(c.x) && aligned16(c.y);

@@ -5,8 +5,9 @@
 // up to 8 (16 non-portable) CTAs.
 //
 // Environment overrides (for experiments and benchmarks only):
-//   GNB200_FORCE_PATH = twopass | wave | resident | streaming: whichever of them there would be without the fused plan
-//                       (anything else: as without it)
+//   GNB200_FORCE_PATH = fused: wherever there is such a plan, faster or not
+//                     = twopass | wave | resident: these, where the shape allows it
+//                     = streaming: whichever of the three there would be without the fused plan   (anything else: as without it)
 //   GNB200_CW = channels per column block   GNB200_K = cluster size       GNB200_THREADS = target CTA size
 //   GNB200_ROWS = rows per CTA tile (multi-kernel path)                   GNB200_PERSIST = 0: one cluster per item
 //   GNB200_NO_SHUF: generic reductions      GNB200_CHAIN = 0: plain stream order between the kernels of a call
@@ -576,7 +577,6 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   const int max_stages = env_int("GNB200_RESIDENT_STAGES", 16);
   if (r.stages > max_stages) r.stages = max_stages < 2 ? 2 : max_stages;
   if (r.stages > 16) r.stages = 16;
-  // GNB200_RESIDENT_STAGES alone bounds what stays on chip
   // Rows that are on chip between the passes, and those on their second read, need no place in L2: the rows that pass 2 reads
   // again find more of it.  Device us, without / with (fp16): forward 512@256^2 37.0 / 35.0, 256@512^2 71.5 / 67.8,
   // 128@1024^2 143.5 / 139.1; backward 512@256^2 64.8 / 63.8, bf16 75 MB 72.0 / 71.0, but 256@512^2 119.2 / 121.0 and
@@ -584,6 +584,7 @@ bool plan_resident(const Shape& sh, bool forced, Plan* plan) {
   r.evict = sh.direction == 0 || 2.0 * sh.N * sh.R * sh.C * s <= 192.0 * 1024 * 1024;
   // Tensor memory, without / with: forward 512@256^2 39.1 / 35.0, 256@512^2 72.5 / 67.3, 128@1024^2 144.1 / 139.4; backward
   // 512@256^2 66.7 / 63.8, bf16 75 MB 73.5 / 70.7, then nothing (256@512^2 118.4 / 118.3, 3 x 61 MB 160.4 / 161.6).
+  // (GNB200_RESIDENT_STAGES without _PARK parks nothing: the stages alone are then what stays on chip.)
   r.park = env_int("GNB200_RESIDENT_PARK", max_stages < 16 || !r.evict ? 0 : kResidentPark);
   if (r.park < 0 || r.park > kResidentPark) r.park = kResidentPark;
   r.smem_bytes = fixed + (size_t)r.stages * stage;
@@ -677,7 +678,6 @@ static bool make_plan_inner(int64_t N, int64_t R, int64_t C, int64_t G, int dtyp
   const int vfull = 16 / sh.s;
   sh.ve = (aligned16 && C % vfull == 0) ? vfull : 1;
   sh.direction = direction;
-  // GNB200_FORCE_PATH = twopass: the multi-kernel plan; wave, resident: these plans where the shape allows it
   const char* force = env_text("GNB200_FORCE_PATH");
   const bool twopass_only = force && !strcmp(force, "twopass");
   const bool wave_only = force && !strcmp(force, "wave"), resident_only = force && !strcmp(force, "resident");

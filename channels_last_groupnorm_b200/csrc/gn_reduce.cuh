@@ -4,7 +4,7 @@
 // threads to each, behind one barrier where a vector lies in one group.  Measured in gn_fwd_resident_kernel, from the
 // CTA's last rows to its sums: 1.0 us against 1.9 with a warp per group and one group after the other (256@512^2, 32
 // groups of 8 channels), 2.4 against 3.8 with groups of 4 channels (128@1024^2).  In the fused forward kernel, whose small
-// maps with groups of 10, 20 or 30 channels are a chain of dependent instructions, device us per call, before / now: 320@64^2
+// maps with groups of 10, 20 or 30 channels are a chain of dependent instructions, device us per call, channel by channel / this way: 320@64^2
 // 9.1 / 7.6, 640@32^2 9.2 / 5.8, 2 x 960@76^2 34.5 / 24.9.
 #pragma once
 #include "gn_async.cuh"

@@ -14,9 +14,8 @@
 //            stages fill again early - and then the tiles before them in reverse order, so that what was read last (and
 //            L2 still holds) is read first; results leave with streaming (evict-first) stores
 //
-// What the tensor memory gave (fp16 SiLU, calls among others): forward 256@512^2 74.0 -> 71.7 us; reductions of all groups
-// at once and parameters asked for early: 71.7 -> 70.2, and 128@1024^2 forward + backward 368 -> 356.5.  Evict-first marks
-// (Stream::issue, the rule in gn_plan.cu): 69.9 -> 66.8.
+// Tensor memory and evict-first marks (Stream::issue) have their rules, with the figures on either side, in gn_plan.cu; the parameters
+// are asked for before the ring's first copies and all groups reduced at once because the tensors rest meanwhile (gn_reduce.cuh).
 //
 // dgamma / dbeta are added up at the end by the grid's warps, without a launch of their own.
 // Measured against the plans it replaces: see the rule in gn_plan.cu.

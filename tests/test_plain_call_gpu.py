@@ -119,3 +119,20 @@ def test_function_modes_and_subclasses_see_the_call():
         pass
 
     assert type(m(x.as_subclass(Sub))) is Sub or torch.equal(m(x.as_subclass(Sub)), y)
+
+
+def test_subclasses_are_no_plain_calls():
+    class Sub(torch.Tensor):
+        seen = []
+
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            cls.seen.append(func)
+            return super().__torch_function__(func, types, args, kwargs or {})
+
+    m = pkg.GN_NHWC(4, 32, device="cuda")
+    x = torch.randn(2, 32, 4, 4, device="cuda")
+    y = m(x)
+    assert not Sub.seen
+    z = m(x.as_subclass(Sub))
+    assert Sub.seen and torch.equal(z.as_subclass(torch.Tensor), y)
