@@ -95,22 +95,26 @@ int reduce_layout(int CW, int CV, int ve, int D, int TY, int threads, bool momen
   return per_part ? 2 * TY * (2 * CV + 1) : TY * rd->stride * (per_vector ? 2 : 1);
 }
 
-size_t fwd_red_floats(int CW, int CV, int TY, int slots, int threads, bool shuf, int tps_shift) {
+size_t fwd_red_floats(int CW, int CV, int D, int TY, int slots, int threads, bool shuf, int tps_shift) {
   if (shuf) {  // two warp-sum buffers, overlaid later by the gathered slot arrays of the peers
     const int a = 2 * wsum_stride_floats(threads, CV, tps_shift), b = 16 * 3 * slots;
     return (size_t)round_up4(a > b ? a : b);
   }
-  size_t r = (size_t)TY * (CW | 1);  // one value per channel, or ...
-  if (r < (size_t)2 * TY * (2 * CV + 1)) r = (size_t)2 * TY * (2 * CV + 1);  // ... up to four per vector (reduce_layout)
+  // one value per channel (multi-kernel plan), or what reduce_layout wants, no more: some 400 bytes can decide whether 512 threads fit (fp32 640 x
+  // 22270 rows 64.0 us, with 256 threads 70.5)
+  ReduceGeom rd;
+  size_t r = (size_t)TY * CW;
+  const size_t need = (size_t)reduce_layout(CW, CV, CW / CV, D, TY, threads, true, &rd);
+  if (r < need) r = need;
   if (r < 1024) r = 1024;
   if (r < (size_t)16 * 3 * slots) r = (size_t)16 * 3 * slots;
   return r;
 }
 // red, tmp, two slot arrays, stat, and for the push exchange two inboxes of k * slots entries of
 // four floats plus alignment slack and two mbarriers
-size_t fwd_fold_floats(int CW, int CV, int TY, int slots, int threads, bool shuf, int tps_shift, int k) {
+size_t fwd_fold_floats(int CW, int CV, int D, int TY, int slots, int threads, bool shuf, int tps_shift, int k) {
   // (+ 12: up to 3 floats of alignment slack, two 8-byte mbarriers, the dead flag and its padding)
-  return fwd_red_floats(CW, CV, TY, slots, threads, shuf, tps_shift) + (size_t)9 * slots + 8 + (size_t)2 * 4 * k * slots + 12;
+  return fwd_red_floats(CW, CV, D, TY, slots, threads, shuf, tps_shift) + (size_t)9 * slots + 8 + (size_t)2 * 4 * k * slots + 12;
 }
 // backward scratch of the CTA reductions.
 // Generic reductions: red = the per-row-lane channel sums (2 * TY * CW floats), then part and chan.
@@ -159,7 +163,7 @@ void fill_divisors(Geom* g, int ve, int direction, int threads, bool fused) {
   }
   g->wsum_stride = g->shuf ? wsum_stride_floats(threads, g->CV, tps_shift) : 0;
   g->wpart_off = (direction == 1 && g->shuf) ? bwd_wpart_off(threads, g->CV, tps_shift, g->slots) : 0;
-  g->red_floats = (int)(direction == 0 ? fwd_red_floats(g->CW, g->CV, g->TY, g->slots, threads, g->shuf != 0, tps_shift)
+  g->red_floats = (int)(direction == 0 ? fwd_red_floats(g->CW, g->CV, g->D, g->TY, g->slots, threads, g->shuf != 0, tps_shift)
                                        : bwd_red_floats(g->CW, g->CV, g->TY, g->slots, threads, g->shuf != 0, tps_shift));
   if (fused && direction == 0) (void)reduce_layout(g->CW, g->CV, ve, g->D, g->TY, threads, true, &g->rd);
   g->div_D = make_fast_div(g->D);
@@ -203,7 +207,7 @@ bool plan_fused_candidate(const Shape& sh, int cw, int k, int target_threads, Pl
   const size_t tile = (((size_t)rows * CV * ve * s + 15) & ~(size_t)15) + ring;
   int tps_shift = 0;
   const bool shuf = shuffle_geometry(sh.D, ve, CV, &tps_shift);
-  const size_t fold = (sh.direction == 0 ? fwd_fold_floats(cw, CV, TY, slots, threads, shuf, tps_shift, k)
+  const size_t fold = (sh.direction == 0 ? fwd_fold_floats(cw, CV, sh.D, TY, slots, threads, shuf, tps_shift, k)
                                          : bwd_fold_floats(cw, CV, TY, slots, threads, shuf, tps_shift, k)) * 4;
   if (tile + fold > kSmemMaxOptin - 1024) return false;
 
@@ -378,7 +382,7 @@ bool plan_two_pass(const Shape& sh, Plan* out) {
   // shared-memory rings of the streaming kernels: 4 rows x 16 bytes per thread (x; x and dy) - kRingDepth
   const size_t ring = ve > 1 ? (size_t)4 * threads * 16 : 0;
   if (sh.direction == 0) {
-    p.smem_bytes = ring + fwd_fold_floats(cw, CV, TY, slots, threads, false, 0, 1) * 4;
+    p.smem_bytes = ring + fwd_fold_floats(cw, CV, sh.D, TY, slots, threads, false, 0, 1) * 4;
     p.ws_bytes = (size_t)p.grid * slots * 3 * sizeof(float);
     p.launches = 3;
   } else {
